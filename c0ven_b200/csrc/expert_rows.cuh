@@ -14,9 +14,15 @@
 #include "cuda_rt.h"
 #include "formats.h"
 #include "iq4nl_values.h"
+#include "quant_rows.cuh"
+#include "router_topk.cuh"
 
 namespace moe {
 
+// One expert's rows start .. start + count of the expert order, at most kTileRows of them.
+struct MoeTile {
+  uint32_t expert, slot, start, count;
+};
 // Rows start .. start + n of the expert order, all of one expert (its slot among this GPU's experts), n <= 8: the
 // reference's MoeGroup (shared/moe_tile.h:20-33) with the rows named by their place in expert order.
 struct MoeGroup {
@@ -34,6 +40,35 @@ struct ActView {
   uint32_t q_stride, d_stride, bs_stride;
 };
 
+// A step that takes the short form (forward_short): at most so many rows, and assignments of rows to experts.
+constexpr uint32_t kShortRows = 8, kShortMax = 64;
+
+// Rows start .. start + count of the expert order, all of one expert; count <= kTileN.
+struct BigTile {
+  uint32_t slot, start, count;
+};
+
+// What a pack leaves: the step's assignments by expert, and the lists the experts' kernels walk.
+struct PackOut {
+  uint32_t *cnt, *base;    // NE each
+  uint32_t *chunk_off;     // [chunks][NE]: rows of the expert's run taken by earlier chunks
+  MoeTile *tiles;          // expert order, <= 64 rows each (prompt.cl:719-723)
+  MoeGroup *groups;        // <= group_max rows each: the experts with fewer than tensor_min rows
+  BigTile *big;            // <= kTileN rows each: the others, for the tensor-core kernels
+  uint32_t *counters;      // [0] tiles, [1] groups, [2] experts hit, [3] rows, [4] big tiles, [5] their rows
+};
+
+// A short step's route: exact logits in; ids, weights, gates and the lists out, those of at most kShortMax assignments by
+// comparing each with every other, where k_router_topk_pack scans all the experts through 1,024 threads.
+struct ShortRoute {
+  const float *rl;      // [T][NE + 1], exact
+  uint32_t T, NE, K;    // K experts a row
+  uint32_t group_max;   // rows a listed group holds
+  int32_t *ids;
+  float *w, *gs;
+  uint32_t *inv, *row_src;
+  PackOut o;            // chunk_off is not written
+};
 struct ExpertRowsArgs {
   const uint8_t *w0, *w1;  // slot 0's slice of the matrix (gate, up) or (down, unused), runs layout
   uint64_t slice_bytes;    // from one slot's slice to the next
@@ -48,6 +83,9 @@ struct ExpertRowsArgs {
   float *out;  // out[expert-order row][r]
   uint32_t out_stride;
   float limit;  // SwiGLU limit, 0: off
+  const float *act_f32;  // QUANT: the activation rows before quantisation, [rows][K]; act and act_row are not read
+  ShortRoute route;      // ROUTED: act_row, groups and ngroups are not read
+  QuantJob codes;        // QUANT: where the quantised rows are left too (q null: nowhere)
 };
 
 __device__ __forceinline__ uint4 ldg_stream16(const void *p) {
@@ -550,17 +588,106 @@ __host__ __device__ constexpr int rows_batch(int nmat, int nu, int m, bool heavy
   return want < cap ? want : cap;
 }
 
+// Block blk of 256 values of a row, held eight a lane, quantised into the row's place in shared memory.
+template <int QT>
+__device__ __forceinline__ QuantLane stage_quantized(const float4 &v0, const float4 &v1, uint32_t blk, uint32_t lane, uint8_t *dst, uint32_t K) {
+  constexpr bool q8k = act_is_q8k(QT);
+  const QuantLane o = quantize_lane<q8k>(v0, v1, lane);
+  *(uint2 *)(dst + 16 * act_slot<QT>(blk * 16 + lane / 2) + 8 * (lane & 1)) = o.codes;
+  if constexpr (q8k) {
+    if (lane == 0) ((float *)(dst + K))[blk] = o.d;
+    if (lane % 2 == 0) ((int16_t *)(dst + K + act_d_bytes(true, K)))[blk * 16 + lane / 2] = (int16_t)o.sum16;
+  } else {
+    if (lane % 4 == 0) ((float *)(dst + K))[blk * 8 + lane / 4] = o.d;
+  }
+  return o;
+}
+
+// The lists of a short step from its rows' experts (s_ids, kShortMax words, 0xFFFFFFFF past the last), by one CTA of 256
+// threads: what k_router_topk_pack leaves for a step whose experts all stay below the tile kernels' threshold.
+__device__ __forceinline__ void short_pack(const ShortRoute &rt, const uint32_t *s_ids) {
+  __shared__ uint32_t s_groups[kShortMax];  // an expert's groups, at its first assignment
+  const uint32_t A = rt.T * rt.K, tid = threadIdx.x;
+  for (uint32_t e = tid; e < rt.NE; e += blockDim.x) {
+    uint32_t n = 0, first = 0;
+    for (uint32_t i = 0; i < A; i++) n += s_ids[i] == e, first += s_ids[i] < e;
+    rt.o.cnt[e] = n, rt.o.base[e] = first;
+  }
+  uint32_t n = 0, first = 0, before = 0;
+  const uint32_t e = tid < A ? s_ids[tid] : 0xFFFFFFFFu;
+  const bool valid = e < rt.NE;
+  if (tid < A) {
+    for (uint32_t i = 0; i < A; i++) n += s_ids[i] == e, first += s_ids[i] < e, before += i < tid && s_ids[i] == e;
+    s_groups[tid] = valid && before == 0 ? (n + rt.group_max - 1) / rt.group_max : 0;
+    if (valid) rt.inv[tid] = first + before, rt.row_src[first + before] = tid / rt.K;
+  }
+  __syncthreads();
+  if (valid && before == 0) {
+    uint32_t tile = 0, group = 0;
+    for (uint32_t i = 0; i < A; i++)
+      if (s_ids[i] < e) tile += s_groups[i] != 0, group += s_groups[i];
+    rt.o.tiles[tile] = MoeTile{e, e, first, n};
+    for (uint32_t i = 0; i * rt.group_max < n; i++) rt.o.groups[group + i] = MoeGroup{e, first + i * rt.group_max, min(rt.group_max, n - i * rt.group_max)};
+  }
+  if (tid == 0) {
+    uint32_t hit = 0, groups = 0, rows = 0;
+    for (uint32_t i = 0; i < A; i++) hit += s_groups[i] != 0, groups += s_groups[i], rows += s_ids[i] < rt.NE;
+    rt.o.counters[0] = hit, rt.o.counters[1] = groups, rt.o.counters[2] = hit, rt.o.counters[3] = rows, rt.o.counters[4] = 0, rt.o.counters[5] = 0;
+  }
+}
+
+// The route of a short step by a CTA of 256 threads: its rows' experts into s_ids (kShortMax words); with `lists`, the
+// step's ids, weights, gates and lists written too.
+__device__ __forceinline__ void short_route(const ShortRoute &rt, uint32_t *s_ids, bool lists) {
+  if (threadIdx.x < kShortMax) s_ids[threadIdx.x] = 0xFFFFFFFFu;  // a row whose logits are not numbers may have no K experts
+  __syncthreads();
+  const uint32_t warp = threadIdx.x / 32;
+  if (warp < rt.T)
+    router_topk_row(warp, rt.rl, RouterApprox{}, nullptr, rt.NE, rt.K, lists ? rt.ids : nullptr, lists ? rt.w : nullptr, rt.gs, nullptr,
+                    (int32_t *)s_ids + warp * rt.K, nullptr);
+  __syncthreads();
+  if (lists) short_pack(rt, s_ids);
+}
+
+// The forms of k_expert_rows: the lists' groups; (gate/up, one or two rows) the top-k in the kernel; (down) rows
+// quantised in the kernel.
+enum RowsForm { ROWS_LISTED, ROWS_ROUTED, ROWS_QUANT };
+
 // NMAT 2: h[row][r] = swiglu(gate_r . x, up_r . x); NMAT 1: y[row][r] = down_r . h. One CTA of 8 warps per (row tile,
 // group); G lanes share a weight row (G = the row's units, up to 32), each taking UPL of its units (UPL 0: as many as
 // the row has, found at run time). Launch: grid (R / rows_per_cta, groups at most), 256 threads, dynamic shared memory
 // M * act_row_stride (+ 2 KB for IQ3_S's codebook).
-template <int QT, int NMAT, int M, int G, int UPL>
+//
+// ROWS_ROUTED (NMAT 2, steps of one or two rows): no top-k or list kernel runs in front. Every CTA takes the top-k of the
+// rows for itself, a warp a row (2 to 3 us, as long as it takes a kernel of its own, less that kernel's launch: 33.9 ->
+// 29.2 us for one row of Q8_0); the grid's second extent is the assignments and one more. The CTAs of an expert's first
+// assignment take all of its rows, those of its others leave; the last index's one CTA writes the lists. With more rows
+// the CTAs that find their place and leave are too many (4 rows: 55 us against 29).
+// ROWS_QUANT (NMAT 1, steps of a few rows): the rows come as f32 (act_f32) and every CTA quantises those it stages, so that no
+// quantiser runs between the two products.
+template <int QT, int NMAT, int M, int G, int UPL, int FORM>
 __global__ void __launch_bounds__(256) k_expert_rows(const ExpertRowsArgs a, const uint32_t *__restrict__ grid_global) {
   extern __shared__ __align__(16) uint8_t smem[];
   dependents_may_launch(), wait_for_predecessors();
   constexpr bool q8k = act_is_q8k(QT);
   uint32_t slot, start, n;
-  if (a.groups) {
+  constexpr bool QUANT = FORM == ROWS_QUANT, ROUTED = FORM == ROWS_ROUTED;
+  [[maybe_unused]] __shared__ uint32_t s_ids[ROUTED ? kShortMax : 1], s_act[ROUTED ? M : 1];
+  if constexpr (ROUTED) {
+    const ShortRoute &rt = a.route;
+    const uint32_t A = rt.T * rt.K, wp = threadIdx.x / 32, ln = threadIdx.x % 32;
+    const bool lists = blockIdx.y == A;
+    if (lists && blockIdx.x) return;
+    short_route(rt, s_ids, lists);
+    if (lists) return;
+    // This assignment's expert, its rows and where its run starts, by every warp alike: at most 32 assignments, one a lane.
+    const uint32_t e = s_ids[blockIdx.y], id = s_ids[ln], same = __ballot_sync(0xffffffffu, id == e);
+    start = __popc(__ballot_sync(0xffffffffu, id < e));
+    if (e >= rt.NE || blockIdx.y != (uint32_t)__ffs(same) - 1) return;
+    slot = e, n = __popc(same);
+    if (wp == 0 && id == e) s_act[__popc(same & ((1u << ln) - 1))] = ln / rt.K;
+    __syncthreads();
+  } else if (a.groups) {
     // Both loads go out together: the list is as long as the grid, so the entry can be read before the count says
     // whether it is one (a CTA's life is a chain of dependent loads; this takes one link out).
     const uint32_t ng = __ldg(a.ngroups);
@@ -611,10 +738,22 @@ __global__ void __launch_bounds__(256) k_expert_rows(const ExpertRowsArgs a, con
   if constexpr (grid_words(QT) > 0)
     for (uint32_t i = threadIdx.x; i < grid_words(QT); i += 256) grid[i] = grid_global[grid_offset(QT) + i];
   // The group's activation rows into shared memory; rows past n get zero scales, so they add nothing.
+  if constexpr (QUANT)
+    for (uint32_t i = warp; i < n * (K / 256); i += 8) {
+      const uint32_t t = i / (K / 256), blk = i % (K / 256);
+      const float4 *src = (const float4 *)(a.act_f32 + (uint64_t)(start + t) * K + blk * 256);
+      const QuantLane o = stage_quantized<QT>(src[2 * lane], src[2 * lane + 1], blk, lane, smem + t * stride, K);
+      if (blockIdx.x == 0 && a.codes.q) store_codes<q8k>(o, (uint64_t)(start + t) * (K / 256) + blk, lane, a.codes);
+    }
   for (uint32_t t = 0; t < (uint32_t)M; t++) {
     uint8_t *dst = smem + t * stride;
     if (t < n) {
-      const uint64_t row = a.act_row ? a.act_row[start + t] : start + t;
+      if constexpr (QUANT) continue;
+      uint64_t row;
+      if constexpr (ROUTED)
+        row = s_act[t];
+      else
+        row = a.act_row ? a.act_row[start + t] : start + t;
       const int4 *src = (const int4 *)(a.act.q + row * a.act.q_stride);
       const float *sd = (const float *)((const uint8_t *)a.act.d + row * a.act.d_stride);
       for (uint32_t i = threadIdx.x; i < K / 16; i += 256) ((int4 *)dst)[act_slot<QT>(i)] = src[i];
@@ -691,6 +830,116 @@ __global__ void __launch_bounds__(256) k_expert_rows(const ExpertRowsArgs a, con
       }
       finish(acc, r);
     }
+  }
+}
+
+// The down product of a step of one or two rows with everything after it: out[t][r] = sum over k, in rank order, of w[t][k] *
+// (down_r of the row's k-th expert . h), + gs[t] * s[t][r], + res[t][r]. In place of a quantiser, k_expert_rows and
+// k_combine, whose launches such a step spends its time on: a warp takes an output row r for every assignment of the step
+// (an expert that two rows share is read again out of the caches), so a CTA holds all of the inner rows, which it
+// quantises itself (at most 32 rows; the same 2 KB of f32 a row by every CTA, out of L2: what makes it the slower form for more rows). The codes are left in q, d, bs
+// too, in expert order, by the CTAs in turn. G lanes a weight row, UPL units of it a lane.
+// Launch: grid by rows_per_warp * 8 output rows, 256 threads, dynamic shared memory A * act_row_stride + the codebook.
+struct DownCombineArgs {
+  const uint8_t *w;
+  uint64_t slice_bytes;
+  uint32_t K, R;               // values per weight row; weight rows
+  uint32_t rows_per_warp;
+  uint32_t T, used, NE;
+  const float *h;              // [expert-order row][K]
+  const int32_t *ids;
+  const float *wk;
+  const uint32_t *inv;
+  const float *gs, *s, *res;   // s, res: null, not wanted
+  float *out;                  // [T][R]
+  QuantJob codes;
+};
+constexpr uint32_t kDownCombineMaxSmem = 100 * 1024;  // two CTAs an SM
+__host__ __device__ constexpr uint32_t down_combine_smem(uint32_t qt, uint32_t rows, uint32_t K) {
+  return rows * act_row_stride(act_is_q8k(qt), K) + 4 * grid_words(qt);
+}
+// Whether the kernel takes a step of `rows` assignments: its rows fit a CTA, and a weight row has at most 128 units.
+__host__ __device__ constexpr bool down_combine_takes(uint32_t qt, uint32_t rows, uint32_t K) {
+  const uint32_t unit = qt == QT_Q8_0 ? 16 : qt == QT_IQ3_S || qt == QT_IQ3_XXS || qt == QT_IQ2_S || qt == QT_Q2_0 ? 64 : 32;
+  return K / unit <= 128 && down_combine_smem(qt, rows, K) <= kDownCombineMaxSmem;
+}
+template <int QT, int G, int UPL>
+__global__ void __launch_bounds__(256) k_down_combine(const DownCombineArgs a, const uint32_t *__restrict__ grid_global) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ uint32_t s_ids[kShortMax], s_row[kShortMax];
+  __shared__ float s_w[kShortMax], s_y[8][kShortMax];
+  dependents_may_launch();
+  constexpr bool q8k = act_is_q8k(QT);
+  static_assert(down_combine_takes(QT, 1, 128 * Unit<QT>::kValues) == (down_combine_smem(QT, 1, 128 * Unit<QT>::kValues) <= kDownCombineMaxSmem) &&
+                    !down_combine_takes(QT, 0, 129 * Unit<QT>::kValues),
+                "the type's unit, as the host's rule has it");
+  constexpr uint32_t RPP = 32 / G;
+  constexpr int RB = rows_batch(1, UPL, 1, grid_words(QT) > 0);
+  using Raw = typename Unit<QT>::Raw;
+  const uint32_t A = a.T * a.used, K = a.K, stride = act_row_stride(q8k, K), upr = K / Unit<QT>::kValues;
+  const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, li = lane % G, sub = lane / G;
+  const uint64_t nblk = (uint64_t)a.R * (K / block_values(QT));
+  uint32_t *grid = (uint32_t *)(smem + A * stride);
+  if constexpr (grid_words(QT) > 0)
+    for (uint32_t i = threadIdx.x; i < grid_words(QT); i += 256) grid[i] = grid_global[grid_offset(QT) + i];
+  wait_for_predecessors();
+  if (threadIdx.x < A) {
+    s_ids[threadIdx.x] = (uint32_t)a.ids[threadIdx.x], s_row[threadIdx.x] = a.inv[threadIdx.x], s_w[threadIdx.x] = a.wk[threadIdx.x];
+    // An assignment without an expert (a row whose logits are not numbers) adds nothing.
+    if (s_ids[threadIdx.x] >= a.NE || s_row[threadIdx.x] >= A) s_ids[threadIdx.x] = 0xFFFFFFFFu;
+  }
+  __syncthreads();
+  Raw raw[RB][UPL];
+  auto fetch = [&](uint32_t r, uint32_t a0) {
+#pragma unroll
+    for (int b = 0; b < RB; b++) {
+      const uint32_t i = a0 + b * RPP + sub;
+      if (r < a.R && i < A && s_ids[i] != 0xFFFFFFFFu) {
+        const uint8_t *w = a.w + (uint64_t)s_ids[i] * a.slice_bytes;
+#pragma unroll
+        for (int j = 0; j < UPL; j++)
+          if (li + G * j < upr) raw[b][j] = Unit<QT>::fetch(w, nblk, K, r, li + G * j, nullptr);
+      }
+    }
+  };
+  // The first weights are on their way while the inner rows are quantised.
+  const uint32_t r0 = (blockIdx.x * 8 + warp) * a.rows_per_warp;
+  fetch(r0, 0);
+  for (uint32_t i = warp; i < A * (K / 256); i += 8) {
+    const uint32_t p = i / (K / 256), blk = i % (K / 256);
+    const float4 *src = (const float4 *)(a.h + (uint64_t)p * K + blk * 256);
+    const QuantLane o = stage_quantized<QT>(src[2 * lane], src[2 * lane + 1], blk, lane, smem + p * stride, K);
+    if (p % gridDim.x == blockIdx.x) store_codes<q8k>(o, (uint64_t)p * (K / 256) + blk, lane, a.codes);
+  }
+  __syncthreads();
+  for (uint32_t rr = 0; rr < a.rows_per_warp && r0 + rr < a.R; rr++) {
+    const uint32_t r = r0 + rr;
+    for (uint32_t a0 = 0; a0 < A; a0 += RPP * RB) {
+      if (rr | a0) fetch(r, a0);
+#pragma unroll
+      for (int b = 0; b < RB; b++) {
+        const uint32_t i = a0 + b * RPP + sub;
+        float acc = 0.0f;
+        if (i < A && s_ids[i] != 0xFFFFFFFFu) {
+#pragma unroll
+          for (int j = 0; j < UPL; j++)
+            if (li + G * j < upr) unit_dot<QT, 1>(raw[b][j], K, li + G * j, smem + s_row[i] * stride, stride, &acc, 1, grid);
+        }
+#pragma unroll
+        for (int off = G / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+        if (li == 0 && i < A) s_y[warp][i] = acc;
+      }
+    }
+    __syncwarp();
+    if (lane < a.T) {
+      float acc = 0.0f;
+      for (uint32_t k = 0; k < a.used; k++) acc = fmaf(s_w[lane * a.used + k], s_y[warp][lane * a.used + k], acc);
+      const uint64_t at = (uint64_t)lane * a.R + r;
+      if (a.s) acc = fmaf(a.gs[lane], a.s[at], acc);
+      if (a.res) acc += a.res[at];
+      a.out[at] = acc;
+    }
+    __syncwarp();
   }
 }
 

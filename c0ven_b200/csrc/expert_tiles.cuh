@@ -26,10 +26,6 @@
 
 namespace moe {
 
-// Rows start .. start + count of the expert order, all of one expert; count <= kTileN.
-struct BigTile {
-  uint32_t slot, start, count;
-};
 constexpr uint32_t kTileM = 128;   // weight rows a CTA takes
 constexpr uint32_t kTileN = 256;   // activation rows at most
 constexpr uint32_t kTileK = 64;    // values of the contraction a stage holds

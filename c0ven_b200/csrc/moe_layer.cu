@@ -51,6 +51,24 @@ static cudaError_t launch_rows(uint32_t qt, int nmat, const ExpertRowsArgs &a, i
 #undef ROWS_CASE
 }
 
+template <int QT>
+cudaError_t launch_down_combine(const DownCombineArgs &a, const uint32_t *grid_global, const LaunchCtx &ctx, cudaStream_t st);
+
+static cudaError_t launch_down_combine_type(uint32_t qt, const DownCombineArgs &a, const uint32_t *grid, const LaunchCtx &ctx, cudaStream_t st) {
+  switch (qt) {
+    case QT_Q8_0: return launch_down_combine<QT_Q8_0>(a, grid, ctx, st);
+    case QT_Q4_K: return launch_down_combine<QT_Q4_K>(a, grid, ctx, st);
+    case QT_Q6_K: return launch_down_combine<QT_Q6_K>(a, grid, ctx, st);
+    case QT_IQ3_S: return launch_down_combine<QT_IQ3_S>(a, grid, ctx, st);
+    case QT_IQ4_NL: return launch_down_combine<QT_IQ4_NL>(a, grid, ctx, st);
+    case QT_IQ4_XS: return launch_down_combine<QT_IQ4_XS>(a, grid, ctx, st);
+    case QT_IQ3_XXS: return launch_down_combine<QT_IQ3_XXS>(a, grid, ctx, st);
+    case QT_IQ2_S: return launch_down_combine<QT_IQ2_S>(a, grid, ctx, st);
+    case QT_Q2_0: return launch_down_combine<QT_Q2_0>(a, grid, ctx, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 static cudaError_t launch_tiles(uint32_t qt, int nmat, const ExpertTilesArgs &a, const CUtensorMap &map, uint32_t max_tiles, const uint32_t *grid,
                                 const LaunchCtx &ctx, cudaStream_t st) {
 #define TILES_CASE(T)                                                                                  \
@@ -93,6 +111,7 @@ struct ActBuffers {
       h_row_map = make_rows_map(h.get(), hr, K, 1);
     }
   }
+  QuantJob job() const { return QuantJob{q.get(), d.get(), bs.get(), h.get(), q8k}; }
   ActView view(uint64_t row0 = 0) const {
     const uint32_t dn = q8k ? K / 256 : K / 32;
     return ActView{q.get() + row0 * K, d.get() + row0 * dn, q8k ? bs.get() + row0 * (K / 16) : nullptr, K, dn * 4, K / 8};
@@ -439,16 +458,10 @@ void quantize_rows(moe_layer *l, const float *src, uint64_t rows, uint32_t Kv, c
                    const float *gate = nullptr, float *gate_parts = nullptr, RouterSplit rs = RouterSplit{}) {
   const uint64_t nblk = rows * (Kv / 256);
   if (nblk == 0) return;
-  const ActView v = dst.view();
   const unsigned grid = (unsigned)((nblk + 7) / 8);
-  if (dst.q8k)
-    launched(l, launch_kernel(l->ctx.pdl, k_quant_q8_K, dim3(grid), dim3(256), 0, st, src, nblk, (int8_t *)v.q, (float *)v.d, (int16_t *)v.bs, dst.h.get(),
-                              gate, Kv / 256, gate_parts, rs),
-             "quantize");
-  else
-    launched(l, launch_kernel(l->ctx.pdl, k_quant_q8_0, dim3(grid), dim3(256), 0, st, src, nblk, (int8_t *)v.q, (float *)v.d, dst.h.get(), gate, Kv / 256,
-                              gate_parts, rs),
-             "quantize");
+  launched(l, launch_kernel(l->ctx.pdl, dst.q8k ? k_quant<true> : k_quant<false>, dim3(grid), dim3(256), 0, st, src, nblk, dst.job(), gate, Kv / 256,
+                            gate_parts, rs),
+           "quantize");
 }
 
 // Whether a call of R expert rows keeps its experts' results in f16: when every expert takes the tile kernels, whose
@@ -480,9 +493,40 @@ uint32_t tensor_budget_for(const moe_layer *l, uint64_t R) {
   return l->can_tensor && !l->cfg.tensor_min_rows && R >= 64 && R < 1280 ? l->sms / 2 : 0;
 }
 
+// The exact fp32 router product of a step's rows, its x quantised by the same launch.
+void launch_router_rows(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
+  const uint32_t E = l->E, NE = l->NE, N = l->N;
+  // Rows a CTA takes: the fewer, the more CTAs share the step's multiply-adds and the shorter a lane's chain of them, for
+  // one more reading of the router's 4 MB out of L2 a pass. Up to 16 rows 2 (or the one), above 4, while the passes are
+  // few; 8 in the long steps of a layer kept off the tensor cores, where the readings would be what counts.
+  const uint32_t tm = T == 1 ? 1 : T <= 16 ? 2 : T <= kRouterExactRows ? 4 : 8, warps = T <= 4 ? 1 : tm <= 4 ? 4 : 8;
+  const size_t smem = (size_t)tm * kRouterPieces * (E / kRouterPieces + 4) * sizeof(float);
+  if (!l->rows_attr_set) {
+    const size_t row = (size_t)kRouterPieces * (E / kRouterPieces + 4) * sizeof(float);
+    auto allow = [&](auto kernel, size_t rows) {
+      if (rows * row > 48 * 1024) CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(rows * row)));
+    };
+    allow(k_router_logits_rows<1>, 1), allow(k_router_logits_rows<1, 16>, 1), allow(k_router_logits_rows<2>, 2), allow(k_router_logits_rows<2, 16>, 2);
+    allow(k_router_logits_rows<4>, 4), allow(k_router_logits_rows<8>, 8);
+    l->rows_attr_set = true;
+  }
+  const uint32_t passes = (T + tm - 1) / tm;
+  StepQuant sq{};
+  sq.job[0] = l->xq_routed.job();
+  if (l->has_shared && !l->shared_x_same) sq.job[1] = l->xq_shared.job();
+  sq.nblk = (uint64_t)T * (E / 256);
+  sq.ctas = (uint32_t)((sq.nblk + (uint64_t)warps * passes - 1) / (warps * passes));
+  const dim3 grid(sq.ctas + (N + 4 * warps - 1) / (4 * warps), passes);
+  const bool deep = (E / kRouterPieces) % 64 == 0;  // sixteen loads in flight a lane: a step of one row is all latency
+  auto kernel = tm == 1 ? (deep ? k_router_logits_rows<1, 16> : k_router_logits_rows<1>)
+                        : tm == 2 ? (deep ? k_router_logits_rows<2, 16> : k_router_logits_rows<2>) : tm == 4 ? k_router_logits_rows<4> : k_router_logits_rows<8>;
+  launched(l, launch_kernel(l->ctx.pdl, kernel, grid, dim3(32 * warps), smem, st, x, T, E, l->router.get(), N, l->bias.get(), NE, l->rl.get(), sq),
+           "router logits");
+}
+
 // Quantise x, the router's logits and top-k, and the pack of the step's T * K assignments over every expert.
 void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
-  const uint32_t E = l->E, NE = l->NE, K = l->K, N = l->N;
+  const uint32_t E = l->E, NE = l->NE, K = l->K;
   const uint64_t A = (uint64_t)T * K;
   // Steps of up to kRouterExactRows rows (and every step of a layer kept off the tensor cores) take the exact fp32
   // product; longer ones the tensor-core product, whose logits the top-k kernel treats as approximate.
@@ -491,32 +535,10 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
   if (approx)
     quantize_rows(l, x, T, E, l->xq_routed, st, l->router.get() + (size_t)NE * E, l->gate_parts.get(),
                   RouterSplit{l->rx_hi.get(), l->rx_lo.get(), l->norm2_parts.get()});
-  else
-    quantize_rows(l, x, T, E, l->xq_routed, st);
-  if (l->has_shared && !l->shared_x_same) quantize_rows(l, x, T, E, l->xq_shared, st);
+  if (approx && l->has_shared && !l->shared_x_same) quantize_rows(l, x, T, E, l->xq_shared, st);
   mark(l, ST_ROUTER, st);
   if (!approx) {
-    // Steps of up to 2 rows stage only those (8 KB a row); longer ones 8 rows a pass.
-    const uint32_t tm = T <= 2 ? T : 8;
-    const size_t smem = (size_t)tm * kRouterPieces * (E / kRouterPieces + 4) * sizeof(float);
-    if (!l->rows_attr_set) {
-      const int most = (int)((size_t)8 * kRouterPieces * (E / kRouterPieces + 4) * sizeof(float));
-      CUDA_OK(cudaFuncSetAttribute(k_router_logits_rows<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-      l->rows_attr_set = true;
-    }
-    const uint32_t warps = tm <= 2 ? 1 : 8;
-    const dim3 grid((N + 4 * warps - 1) / (4 * warps), (T + tm - 1) / tm);
-    const bool deep = (E / kRouterPieces) % 64 == 0;  // sixteen loads in flight a lane: a step of one row is all latency
-    if (tm == 1 && deep)
-      k_router_logits_rows<1, 16><<<grid, 32, smem, st>>>(x, T, E, l->router.get(), N, l->bias.get(), NE, l->rl.get());
-    else if (tm == 1)
-      k_router_logits_rows<1><<<grid, 32, smem, st>>>(x, T, E, l->router.get(), N, l->bias.get(), NE, l->rl.get());
-    else if (tm == 2 && deep)
-      k_router_logits_rows<2, 16><<<grid, 32, smem, st>>>(x, T, E, l->router.get(), N, l->bias.get(), NE, l->rl.get());
-    else if (tm == 2)
-      k_router_logits_rows<2><<<grid, 32, smem, st>>>(x, T, E, l->router.get(), N, l->bias.get(), NE, l->rl.get());
-    else
-      k_router_logits_rows<8><<<grid, 256, smem, st>>>(x, T, E, l->router.get(), N, l->bias.get(), NE, l->rl.get());
+    launch_router_rows(l, x, T, st);
   } else {
     if (!l->router_attr_set) {
       CUDA_OK(cudaFuncSetAttribute(k_router_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRouterSmemBytes));
@@ -529,8 +551,8 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
     const RouterMmaArgs ra{T, E, NE, ne_tile, l->rw_unscale.get(), l->approx.get(), l->error.get()};
     const uint32_t items = row_tiles * ((NE + ne_tile - 1) / ne_tile);
     k_router_mma<<<std::min(items, l->sms), kRouterThreads, kRouterSmemBytes, st>>>(ra, l->rx_hi_map, l->rx_lo_map, l->rw_hi_map, l->rw_lo_map);
+    launched(l, cudaGetLastError(), "router logits");
   }
-  launched(l, cudaGetLastError(), "router logits");
   const uint32_t nchunks = (T + kChunkTokens - 1) / kChunkTokens;
   // On one GPU the pack also lists the groups and big tiles of the experts' kernels; expert parallel, it only sorts.
   const uint32_t tm = l->local == NE ? tensor_min_for(l, A) : 0, budget = l->local == NE ? tensor_budget_for(l, A) : 0;
@@ -675,10 +697,15 @@ void stage_shared(moe_layer *l, uint32_t T, cudaStream_t st) {
   a.w0 = l->sg.get(), a.w1 = l->su.get(), a.K = E, a.R = F, a.rows_per_cta = 32;
   a.act = xs.view(), a.dense_rows = T, a.out = hs, a.out_stride = F, a.limit = c.swiglu_limit;
   launched(l, launch_rows(c.shexp_gate_type, 2, a, M, dense_groups, l->grid.get(), l->ctx, st), "shared gate/up");
-  quantize_rows(l, hs, T, F, l->hq_shared, st);
   ExpertRowsArgs b{};
   b.w0 = l->sd.get(), b.K = F, b.R = E, b.rows_per_cta = 128;
-  b.act = l->hq_shared.view(), b.dense_rows = T, b.out = l->s.get(), b.out_stride = E;
+  b.dense_rows = T, b.out = l->s.get(), b.out_stride = E;
+  // In a step of few rows the down kernel quantises its rows as it stages them; in a longer one (a layer kept off the tile
+  // kernels), where each of its many CTAs would do so for every group of rows, a kernel of its own does it once.
+  if (T <= kShortRows)
+    b.act_f32 = hs;
+  else
+    quantize_rows(l, hs, T, F, l->hq_shared, st), b.act = l->hq_shared.view();
   launched(l, launch_rows(c.shexp_down_type, 1, b, M, dense_groups, l->grid.get(), l->ctx, st), "shared down");
 }
 
@@ -689,6 +716,61 @@ void stage_combine(moe_layer *l, const Y *y, uint32_t T, float *out, cudaStream_
                             (const float *)l->gs.get(), (const float *)(l->has_shared ? l->s.get() : nullptr), l->K, l->E, out, l->residual),
            "combine");
   mark(l, ST_COPIES, st);
+}
+
+// Whether a step of T rows takes the short form (forward_short): every expert stays on the integer-dot kernels whatever
+// the routing, and one CTA can compare each of the step's assignments with every other.
+bool takes_short_form(const moe_layer *l, uint32_t T) {
+  const uint64_t A = (uint64_t)T * l->K;
+  const uint32_t tm = tensor_min_for(l, A);
+  return !l->profile && T <= kShortRows && A <= kShortMax && (tm == 0 || T < tm) && tensor_budget_for(l, A) == 0;
+}
+
+// A step of a few rows, in as few launches as its kernels can be put together into, for launches are what its time goes
+// into: the router with x quantised, the top-k with the lists, gate/up, the down product, which quantises its rows, and
+// the combine; with one or two rows the top-k is in the gate/up kernel and the combine in the down one. Beside the
+// routed experts', the shared expert's two. Stage by stage (forward_device) such a step is eleven launches, eight of them
+// one after another.
+void forward_short(moe_layer *l, const float *x, uint32_t T, float *out, cudaStream_t st) {
+  const uint32_t E = l->E, F = l->F, NE = l->NE, K = l->K, A = T * K;
+  const moe_layer_config &c = l->cfg;
+  PackBuffers &pk = l->pack;
+  launch_router_rows(l, x, T, st);
+  if (l->has_shared) {
+    l->fork_ev->record(st);
+    CUDA_OK(cudaStreamWaitEvent(l->aux->get(), l->fork_ev->get(), 0));
+    stage_shared(l, T, l->aux->get());
+    l->join_ev->record(l->aux->get());
+  }
+  const uint32_t gmax = group_cap(A, NE);
+  const ShortRoute rt{l->rl.get(), T, NE, K, gmax, l->ids.get(), l->w.get(), l->gs.get(), pk.inv.get(), pk.row_src.get(), pk.out()};
+  const bool routed = T <= 2;  // the top-k in the gate/up kernel
+  if (!routed) launched(l, launch_kernel(l->ctx.pdl, k_short_route, dim3(1), dim3(32 * kShortRows), 0, st, rt), "router top-k and lists");
+  l->last_T = T, l->last_pack = &pk, l->last_tensor_min = tensor_min_for(l, A);
+  const int M = routed ? (int)T : group_rows(std::min(gmax, T));
+  ExpertRowsArgs a{};
+  a.w0 = l->wg.get(), a.w1 = l->wu.get(), a.slice_bytes = l->gate_slice, a.K = E, a.R = F, a.rows_per_cta = 32;
+  a.act = l->xq_routed.view(), a.act_row = pk.row_src.get(), a.groups = pk.groups.get(), a.ngroups = pk.counters.get() + 1;
+  a.out = l->h.get(), a.out_stride = F, a.limit = c.swiglu_limit;
+  if (routed) a.route = rt;
+  launched(l, launch_rows(c.gate_type, 2, a, M, routed ? A + 1 : A, l->grid.get(), l->ctx, st), "experts gate/up");
+  if (T <= 2 && down_combine_takes(c.down_type, A, F)) {
+    if (l->has_shared) CUDA_OK(cudaStreamWaitEvent(st, l->join_ev->get(), 0));
+    DownCombineArgs d{};
+    d.w = l->wd.get(), d.slice_bytes = l->down_slice, d.K = F, d.R = E, d.T = T, d.used = K, d.NE = NE;
+    d.h = l->h.get(), d.ids = l->ids.get(), d.wk = l->w.get(), d.inv = pk.inv.get();
+    d.gs = l->gs.get(), d.s = l->has_shared ? l->s.get() : nullptr, d.res = l->residual, d.out = out, d.codes = l->hq_routed.job();
+    launched(l, launch_down_combine_type(c.down_type, d, l->grid.get(), l->ctx, st), "experts down and combine");
+  } else {
+    ExpertRowsArgs b{};
+    b.w0 = l->wd.get(), b.slice_bytes = l->down_slice, b.K = F, b.R = E, b.rows_per_cta = 128;
+    b.act_f32 = l->h.get(), b.codes = l->hq_routed.job(), b.groups = pk.groups.get(), b.ngroups = pk.counters.get() + 1;
+    b.out = l->y.get(), b.out_stride = E;
+    launched(l, launch_rows(c.down_type, 1, b, M, A, l->grid.get(), l->ctx, st), "experts down");
+    if (l->has_shared) CUDA_OK(cudaStreamWaitEvent(st, l->join_ev->get(), 0));
+    stage_combine<float>(l, l->y.get(), T, out, st);
+  }
+  l->stats.calls++, l->stats.rows += T, l->stats.assignments += A;
 }
 
 constexpr uint32_t kGraphMaxRows = 64;
@@ -705,6 +787,7 @@ void forward_device(moe_layer *l, const float *x, uint32_t T, float *out, cudaSt
     LaunchCtx &c;
     ~PdlOff() { c.pdl = false; }
   } pdl_off{l->ctx};
+  if (takes_short_form(l, T)) return forward_short(l, x, T, out, st);
   // The shared expert needs only the quantised rows: it runs on a second stream beside the routed experts and joins
   // before the combine. With per-stage timing on, it runs in line instead, so that its stage can be timed.
   // In long steps it runs in line after all: the routed kernels then fill the GPU for many rounds of items dealt to

@@ -1,0 +1,71 @@
+"""On a B200: steps of a few rows, which run in three launches (the router with the quantisers; gate/up with the top-k in
+every CTA; the down product with the combine), against the CPU oracle and against the same layer stage by stage (a
+profiled layer takes its steps that way). Around the edges of the rule: 8 rows, 64 assignments, 128 units a weight row."""
+import numpy as np
+import pytest
+
+from c0ven_b200 import MoELayer, synth
+from oracle import oracle as O
+from test_gpu_parity import INT_PATH_REL, TYPES, check
+
+pytestmark = pytest.mark.gpu
+
+
+def compare(layer, rows, seed=0, shared=True):
+    on_gpu = layer if shared else dict(layer, gate_shexp=None)
+    short, staged = MoELayer(on_gpu, max_tokens=64, no_tensor=True), MoELayer(on_gpu, max_tokens=64, no_tensor=True, profile=True)
+    for T in rows:
+        x = synth.make_input(T, layer["n_embd"], seed=seed + T)
+        out = check(layer, short, x, INT_PATH_REL).copy()
+        check(layer, staged, x, INT_PATH_REL)
+        assert np.array_equal(short.groups(), staged.groups()), T
+        for inner in (False, True):
+            (q, d, bs), (q2, d2, bs2) = short.quantized(T, inner=inner), staged.quantized(T, inner=inner)
+            if not inner:
+                assert np.array_equal(q, q2) and np.array_equal(d, d2)
+            # Inner rows: sums whose last bit may differ, so now and then a code that rounds the other way.
+            assert np.abs(q.astype(np.int32) - q2).max() <= 1 and np.mean(q != q2) <= 1e-2
+            assert np.allclose(d, d2, rtol=1e-3)
+            if bs is not None and len(bs):
+                assert np.array_equal(bs.reshape(-1), q.reshape(-1, 16).astype(np.int32).sum(1).astype(np.int16).reshape(-1))
+        assert np.array_equal(short.forward(x), out)  # seen before: recorded; and once more from the recording
+        assert np.array_equal(short.forward(x), out)
+    short.close(), staged.close()
+
+
+@pytest.mark.parametrize("t", TYPES)
+def test_every_type(t):
+    layer = synth.make_layer(n_embd=512, n_ff=512, n_experts=32, n_used=4, gate_type=t, seed=t)
+    compare(layer, (1, 2, 3, 5, 8, 9))
+
+
+@pytest.mark.parametrize("t", TYPES)
+def test_every_type_in_lengths_nothing_is_specialised_for(t):
+    layer = synth.make_layer(n_embd=768, n_ff=1280, n_experts=32, n_used=7, gate_type=t, shexp_gate_type=synth.Q8_0, shexp_down_type=t, seed=t)
+    compare(layer, (1, 4, 8))
+
+
+@pytest.mark.parametrize("n_used,rows", [(1, (1, 8)), (8, (7, 8)), (9, (7, 8)), (16, (4, 5))])
+def test_assignments_around_the_limit_with_shared_experts(n_used, rows):
+    layer = synth.make_layer(n_embd=512, n_ff=256, n_experts=32, n_used=n_used, gate_type=synth.Q4_K, down_type=synth.Q6_K,
+                             shexp_gate_type=synth.Q8_0, shexp_down_type=synth.Q8_0, zipf_s=1.1, seed=n_used)
+    compare(layer, rows)
+
+
+@pytest.mark.parametrize("n_ff", [2048, 2304, 4096])
+def test_weight_rows_around_the_longest(n_ff):
+    layer = synth.make_layer(n_embd=256, n_ff=n_ff, n_experts=32, n_used=4, gate_type=synth.Q4_K, down_type=synth.Q8_0, seed=n_ff)
+    compare(layer, (1, 8))
+
+
+def test_without_a_shared_expert_and_equal_logits():
+    layer = synth.make_layer(n_embd=512, n_ff=256, n_experts=32, n_used=4, gate_type=synth.Q8_0, seed=33)
+    for k in ("gate_shexp", "up_shexp", "down_shexp"):
+        layer[k] = np.zeros_like(layer[k])  # the oracle always has one: with scales of 0 it adds nothing
+    layer["router"][5] = layer["router"][2]
+    compare(layer, (1, 3, 8), shared=False)
+    gpu = MoELayer(dict(layer, gate_shexp=None), max_tokens=8)
+    x = np.zeros((2, 512), dtype=np.float32)
+    assert np.all(gpu.forward(x) == 0)
+    assert np.array_equal(gpu.route(2)[0], O.moe_forward(layer, x)[1])
+    gpu.close()
