@@ -271,86 +271,125 @@ __host__ __device__ inline bool n_is_tensor(uint32_t n, uint32_t tensor_min) { r
 // two rows, whose tiles would be all decode and no product: the threshold moves only if the experts that then change
 // kernels hold at least half of the step's rows.
 // The scan itself, for every thread of a CTA of 512 threads or more (the threads past 511 only keep the barriers):
-// thread e < NE brings its expert's row count `run`; returns the first row of the expert's run.
+// thread e < NE brings its expert's row count `run`; returns the first row of the expert's run. One CTA works while the
+// step waits, so what counts is its chain of barriers and dependent reads: prefix sums by shuffles with one barrier
+// between the warps' part and the block's, and the short tiles ranked by a counting sort over their lengths (every
+// thread reading all 512 lengths to find its rank took longer than all the rest).
 __device__ __forceinline__ uint32_t pack_scan_block(uint32_t e, uint32_t run, uint32_t NE, uint32_t first_expert, uint32_t tensor_min,
                                                     uint32_t tensor_budget, uint32_t group_max, const PackOut &o) {
-  __shared__ uint32_t s_rows[512], s_tiles[512], s_groups[512], s_hit[512], s_big[512], s_bigrows[512], s_hit2[512];
-  __shared__ uint32_t s_rows_ge[3], s_total;
+  constexpr uint32_t kWarps = 16, kSums = 7;
+  __shared__ uint32_t s_sum[kSums][kWarps], s_ge[4][kWarps], s_rows_ge[4][kWarps];
+  __shared__ uint16_t s_len[kWarps][kTileN];  // short tiles of a length in a warp; then how many of that length come before the warp's
+  __shared__ uint32_t s_bin[kTileN / 32];
   const bool in = e < 512;
+  const uint32_t lane = e % 32, warp = e / 32;
   if (!in || e >= NE) run = 0;
+  // A value over the 16 warps' entries of a row: the sum before this warp's, and the sum of all.
+  auto before_and_all = [&](const uint32_t *row, uint32_t &all) {
+    uint32_t v = lane < kWarps ? row[lane] : 0;
+    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? v : 0);
+    all = __reduce_add_sync(0xffffffffu, v);
+    return before;
+  };
   if (tensor_budget) {
     // Lower only if the experts that would move hold at least half of the step's rows: moving a few rows costs two
     // more kernels for nothing.
-    if (e < 3) s_rows_ge[e] = 0;
-    if (e == 3) s_total = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t least = 1u << j, c = __popc(__ballot_sync(0xffffffffu, run >= least));
+      const uint32_t r = __reduce_add_sync(0xffffffffu, run >= least ? run : 0);
+      if (in && lane == 0) s_ge[j][warp] = c, s_rows_ge[j][warp] = r;
+    }
     __syncthreads();
-    if (run >= 2) atomicAdd(&s_rows_ge[0], run);
-    if (run >= 4) atomicAdd(&s_rows_ge[1], run);
-    if (run >= 8) atomicAdd(&s_rows_ge[2], run);
-    if (run) atomicAdd(&s_total, run);
-    const uint32_t ge1 = __syncthreads_count(run >= 1), ge2 = __syncthreads_count(run >= 2), ge4 = __syncthreads_count(run >= 4),
-                   ge8 = __syncthreads_count(run >= 8);
-    if (ge1 <= tensor_budget) {
+    uint32_t ge[4], rows_ge[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) before_and_all(s_ge[j], ge[j]), before_and_all(s_rows_ge[j], rows_ge[j]);
+    if (ge[0] <= tensor_budget) {
       tensor_min = 1;  // few experts in all: every one to the tile kernels
     } else {
-      const int pick = ge2 <= tensor_budget ? 0 : ge4 <= tensor_budget ? 1 : ge8 <= tensor_budget ? 2 : -1;
-      if (pick >= 0 && 2 * s_rows_ge[pick] >= s_total) tensor_min = min(tensor_min, 2u << pick);
+      const int pick = ge[1] <= tensor_budget ? 1 : ge[2] <= tensor_budget ? 2 : ge[3] <= tensor_budget ? 3 : 0;
+      if (pick > 0 && 2 * (pick == 1 ? rows_ge[1] : pick == 2 ? rows_ge[2] : rows_ge[3]) >= rows_ge[0]) tensor_min = min(tensor_min, 1u << pick);
     }
   }
   const bool tensor = n_is_tensor(run, tensor_min);
   const uint32_t n = run, nt = (n + kTileRows - 1) / kTileRows, ng = tensor ? 0 : (n + group_max - 1) / group_max;
   const uint32_t nb = tensor ? (n + kTileN - 1) / kTileN : 0;
-  if (in) s_rows[e] = n, s_tiles[e] = nt, s_groups[e] = ng, s_hit[e] = n > 0, s_big[e] = nb, s_bigrows[e] = tensor ? n : 0;
-  __syncthreads();
-  for (uint32_t off = 1; off < 512; off <<= 1) {
-    const bool take = in && e >= off;
-    const uint32_t a = take ? s_rows[e - off] : 0, b = take ? s_tiles[e - off] : 0;
-    const uint32_t c = take ? s_groups[e - off] : 0, d = take ? s_hit[e - off] : 0;
-    const uint32_t f = take ? s_big[e - off] : 0, g = take ? s_bigrows[e - off] : 0;
-    __syncthreads();
-    if (in) s_rows[e] += a, s_tiles[e] += b, s_groups[e] += c, s_hit[e] += d, s_big[e] += f, s_bigrows[e] += g;
-    __syncthreads();
-  }
-  const uint32_t first = in ? s_rows[e] - n : 0;
-  if (e < NE) {
-    o.cnt[e] = n;
-    o.base[e] = first;
-    const uint32_t tile0 = s_tiles[e] - nt, group0 = s_groups[e] - ng;
-    for (uint32_t i = 0; i < nt; i++)
-      o.tiles[tile0 + i] = MoeTile{first_expert + e, e, first + i * kTileRows, min(kTileRows, n - i * kTileRows)};
-    for (uint32_t i = 0; i < ng; i++)
-      o.groups[group0 + i] = MoeGroup{e, first + i * group_max, min(group_max, n - i * group_max)};
-  }
   // Big tiles, in the order the tile kernels deal them to their CTAs round by round. First the experts that have at
   // least one full tile of kTileN rows, in expert order, each one's tiles side by side, its last, shorter one too: the
   // CTAs that take them run at the same time, so an expert's weights come from HBM once and from L2 after that (with
   // the short tiles all at the end, as this list once had them, every expert's weights were read from HBM again for
   // its short tile: 3.5 GB of traffic a 32,768-row gate/up launch against 2.6 GB the algorithm needs). Then the experts
   // with one short tile only, by falling row count (ties in expert order), so that the last rounds hold the
-  // shortest items. s_bigrows is free to reuse: the scan's total is read first.
-  const uint32_t total_rows_big = s_bigrows[511], nfull = tensor ? n / kTileN : 0, rem = tensor ? n % kTileN : 0;
-  const uint32_t mine = nfull ? nfull + (rem != 0) : 0;
-  __syncthreads();
-  if (in) s_hit2[e] = mine, s_bigrows[e] = nfull ? 0 : rem;
-  __syncthreads();
-  for (uint32_t off = 1; off < 512; off <<= 1) {
-    const uint32_t a = in && e >= off ? s_hit2[e - off] : 0;
-    __syncthreads();
-    if (in) s_hit2[e] += a;
-    __syncthreads();
-  }
-  if (e < NE) {
-    const uint32_t tile0 = s_hit2[e] - mine, all_long = s_hit2[511];
-    for (uint32_t i = 0; i < mine; i++) o.big[tile0 + i] = BigTile{e, first + i * kTileN, i < nfull ? kTileN : rem};
-    if (!nfull && rem) {
-      uint32_t rank = 0;
-      for (uint32_t j = 0; j < 512; j++) rank += s_bigrows[j] > rem || (s_bigrows[j] == rem && j < e);
-      o.big[all_long + rank] = BigTile{e, first, rem};
+  // shortest items.
+  const uint32_t nfull = tensor ? n / kTileN : 0, rem = tensor ? n % kTileN : 0;
+  const uint32_t mine = nfull ? nfull + (rem != 0) : 0, len = nfull ? 0 : rem;  // len: the expert's short tile, 0 without one
+  // Inclusive sums within the warp of what the lists are laid out by; plain sums of the rest.
+  uint32_t v[4] = {n, nt, ng, mine};
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (uint32_t off = 1; off < 32; off <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, v[j], off);
+      if (lane >= off) v[j] += u;
     }
+  const uint32_t hit = __popc(__ballot_sync(0xffffffffu, n > 0)), big = __reduce_add_sync(0xffffffffu, nb),
+                 bigrows = __reduce_add_sync(0xffffffffu, tensor ? n : 0);
+  if (in) {
+    for (uint32_t i = lane; i < kTileN / 2; i += 32) ((uint32_t *)s_len[warp])[i] = 0;
+    if (lane == 31) s_sum[0][warp] = v[0], s_sum[1][warp] = v[1], s_sum[2][warp] = v[2], s_sum[3][warp] = v[3];
+    if (lane == 0) s_sum[4][warp] = hit, s_sum[5][warp] = big, s_sum[6][warp] = bigrows;
+    __syncwarp();
+  }
+  const uint32_t same = __match_any_sync(0xffffffffu, len);
+  if (in && len && (uint32_t)__ffs(same) - 1 == lane) s_len[warp][len] = (uint16_t)__popc(same);
+  __syncthreads();
+  // Thread e < 256 has the tiles of length e: how many come before each warp's, and (below) before all of that length.
+  uint32_t longer = 0;
+  if (e < kTileN) {
+    uint32_t sum = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kWarps; w++) {
+      const uint32_t c = s_len[w][e];
+      s_len[w][e] = (uint16_t)sum;
+      sum += c;
+    }
+    longer = sum;
+#pragma unroll
+    for (uint32_t off = 1; off < 32; off <<= 1) {
+      const uint32_t u = __shfl_down_sync(0xffffffffu, longer, off);
+      if (lane + off < 32) longer += u;
+    }
+    if (lane == 0) s_bin[warp] = longer;
+    longer -= sum;  // within the warp's 32 lengths
+  }
+  __syncthreads();
+  if (e < kTileN) {
+    for (uint32_t w = warp + 1; w < kTileN / 32; w++) longer += s_bin[w];
+#pragma unroll
+    for (uint32_t w = 0; w < kWarps; w++) s_len[w][e] = (uint16_t)(s_len[w][e] + longer);
+  }
+  __syncthreads();
+  uint32_t all[kSums], before[4];
+#pragma unroll
+  for (int j = 0; j < (int)kSums; j++) {
+    const uint32_t b = before_and_all(s_sum[j], all[j]);
+    if (j < 4) before[j] = b + v[j];
+  }
+  const uint32_t first = in ? before[0] - n : 0;
+  if (e < NE) {
+    o.cnt[e] = n;
+    o.base[e] = first;
+    const uint32_t tile0 = before[1] - nt, group0 = before[2] - ng, big0 = before[3] - mine;
+    for (uint32_t i = 0; i < nt; i++)
+      o.tiles[tile0 + i] = MoeTile{first_expert + e, e, first + i * kTileRows, min(kTileRows, n - i * kTileRows)};
+    for (uint32_t i = 0; i < ng; i++)
+      o.groups[group0 + i] = MoeGroup{e, first + i * group_max, min(group_max, n - i * group_max)};
+    for (uint32_t i = 0; i < mine; i++) o.big[big0 + i] = BigTile{e, first + i * kTileN, i < nfull ? kTileN : rem};
+    if (len) o.big[all[3] + s_len[warp][len] + __popc(same & ((1u << lane) - 1))] = BigTile{e, first, rem};
   }
   if (e == 511) {
-    o.counters[0] = s_tiles[e], o.counters[1] = s_groups[e], o.counters[2] = s_hit[e], o.counters[3] = s_rows[e];
-    o.counters[4] = s_big[e], o.counters[5] = total_rows_big;
+    o.counters[0] = all[1], o.counters[1] = all[2], o.counters[2] = all[4], o.counters[3] = all[0];
+    o.counters[4] = all[5], o.counters[5] = all[6];
   }
   return first;
 }
