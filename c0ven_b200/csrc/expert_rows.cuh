@@ -79,6 +79,7 @@ struct ExpertRowsArgs {
   const MoeGroup *groups;   // null: dense_rows rows of slot 0, taken M at a time
   const uint32_t *ngroups;
   uint32_t dense_rows;
+  uint32_t halves;          // CTAs, along the grid's third extent, that share a group M rows each (0 or 1: one takes it whole)
   uint32_t slabs;           // row slabs a CTA takes one after another (0 or 1: one); only with the row length known at compile time
   float *out;  // out[expert-order row][r]
   uint32_t out_stride;
@@ -92,6 +93,10 @@ __device__ __forceinline__ uint4 ldg_stream16(const void *p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
+}
+// `bytes` from p on (both multiples of 16) asked for in the L2.
+__device__ __forceinline__ void prefetch_l2_bulk(const void *p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ int dot4x4(const uint4 &w, const int4 &a) {
   int s = __dp4a((int)w.x, a.x, 0);
@@ -603,6 +608,19 @@ __device__ __forceinline__ QuantLane stage_quantized(const float4 &v0, const flo
   return o;
 }
 
+// Weight rows r0 .. r1 of the slice w, every run's part of them rounded out to 16 bytes, asked for in the L2. (The last
+// run's may reach up to 15 bytes past the slice: a matrix is followed by 16 bytes of its allocation.)
+template <int QT>
+__device__ __forceinline__ void prefetch_weight_rows(const uint8_t *w, uint64_t nblk, uint32_t K, uint32_t r0, uint32_t r1) {
+  const uint32_t bpr = K / block_values(QT);
+#pragma unroll
+  for (uint32_t f = 0; f < nfields(QT); f++) {
+    const uint32_t row = bpr * field(QT, f).size;
+    const uint64_t run = run_offset(QT, f, nblk), at = (run + (uint64_t)r0 * row) & ~(uint64_t)15, end = (run + (uint64_t)r1 * row + 15) & ~(uint64_t)15;
+    prefetch_l2_bulk(w + at, (uint32_t)(end - at));
+  }
+}
+
 // The lists of a short step from its rows' experts (s_ids, kShortMax words, 0xFFFFFFFF past the last), by one CTA of 256
 // threads: what k_router_topk_pack leaves for a step whose experts all stay below the tile kernels' threshold.
 __device__ __forceinline__ void short_pack(const ShortRoute &rt, const uint32_t *s_ids) {
@@ -693,7 +711,8 @@ __global__ void __launch_bounds__(256) k_expert_rows(const ExpertRowsArgs a, con
     const uint32_t ng = __ldg(a.ngroups);
     const MoeGroup g = a.groups[blockIdx.y];
     if (blockIdx.y >= ng) return;
-    slot = g.slot, start = g.start, n = g.n;
+    if (blockIdx.z * M >= g.n) return;
+    slot = g.slot, start = g.start + blockIdx.z * M, n = min((uint32_t)M, g.n - blockIdx.z * M);
   } else {
     start = blockIdx.y * M;
     if (start >= a.dense_rows) return;
@@ -733,6 +752,15 @@ __global__ void __launch_bounds__(256) k_expert_rows(const ExpertRowsArgs a, con
     }
   };
   if constexpr (UPL > 0) fetch_slab(r_begin);
+  // What the CTA's warps will come to later is asked for in the L2 now, by one thread: a warp loads a slab, computes it and
+  // only then loads the next, so without this HBM's latency stands in front of every slab.
+  if (threadIdx.x == 0) {
+    const uint32_t end = min(a.R, (blockIdx.x + 1) * slabs * slab_rows), from = min(end, blockIdx.x * slabs * slab_rows + (UPL > 0 ? slab_rows : 0));
+    if (from < end) {
+      prefetch_weight_rows<QT>(w0, nblk, K, from, end);
+      if constexpr (NMAT == 2) prefetch_weight_rows<QT>(w1, nblk, K, from, end);
+    }
+  }
 
   uint32_t *grid = (uint32_t *)(smem + M * stride);
   if constexpr (grid_words(QT) > 0)
@@ -772,11 +800,13 @@ __global__ void __launch_bounds__(256) k_expert_rows(const ExpertRowsArgs a, con
 
   auto finish = [&](float (&acc)[NMAT][M], uint32_t r) {
 #pragma unroll
-    for (int m = 0; m < NMAT; m++)
+    for (int t = 0; t < M; t++) {
+      if ((uint32_t)t >= n) break;  // the same for the whole CTA
 #pragma unroll
-      for (int t = 0; t < M; t++)
+      for (int m = 0; m < NMAT; m++)
 #pragma unroll
         for (int off = G / 2; off > 0; off >>= 1) acc[m][t] += __shfl_xor_sync(0xffffffffu, acc[m][t], off);
+    }
     if (li == 0 && r < a.R) {
 #pragma unroll
       for (int t = 0; t < M; t++)

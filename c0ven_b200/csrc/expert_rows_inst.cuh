@@ -39,7 +39,7 @@ static cudaError_t launch_one(ExpertRowsArgs a, uint32_t max_groups, const uint3
     if (FORM == ROWS_ROUTED) slabs = (uint32_t)std::min<uint64_t>(8, (ctas + 3 * ctx.sms - 1) / (3 * ctx.sms));
   }
   a.slabs = slabs;
-  const dim3 grid((a.R + a.rows_per_cta * slabs - 1) / (a.rows_per_cta * slabs), max_groups);
+  const dim3 grid((a.R + a.rows_per_cta * slabs - 1) / (a.rows_per_cta * slabs), max_groups, std::max(1u, a.halves));
   return launch_kernel(ctx.pdl, kernel, grid, dim3(256), smem, st, a, grid_global);
 }
 

@@ -600,7 +600,11 @@ void stage_experts(moe_layer *l, const ActSource &src, const PackBuffers &pk, ui
   // The most groups and big tiles the rows can make: an expert below tm rows has (tm - 2) / 8 + 1 groups at most, and one
   // at or above it a tile per 256 rows and one more.
   const uint32_t gmax = group_cap(R, nexp);
-  const int M = group_rows(std::min<uint64_t>(std::min<uint64_t>(gmax, most), tm ? std::min<uint64_t>(R, tm - 1) : R));
+  int M = group_rows(std::min<uint64_t>(std::min<uint64_t>(gmax, most), tm ? std::min<uint64_t>(R, tm - 1) : R));
+  // Groups of up to eight rows where an expert has two or three on average: the kernel for four, whose accumulators leave
+  // room for three CTAs on an SM, takes nearly all of them whole, and the odd longer one in two halves.
+  const uint32_t halves = M == 8 && R <= 3ull * nexp ? 2 : 1;
+  M /= halves;
   const uint32_t max_groups =
       tm ? (tm > 1 ? (uint32_t)std::min<uint64_t>(R, (uint64_t)nexp * ((tm - 2) / gmax + 1)) : 0) : (uint32_t)std::min<uint64_t>(R, R / gmax + nexp);
   // The pack may have lowered the threshold to 1 (tensor_budget_for): the tile launches are sized for that.
@@ -642,7 +646,7 @@ void stage_experts(moe_layer *l, const ActSource &src, const PackBuffers &pk, ui
     a.w0 = l->wg.get(), a.w1 = l->wu.get(), a.slice_bytes = l->gate_slice, a.K = E, a.R = F, a.rows_per_cta = 32;
     a.act = src.view, a.act_row = src.act_row;
     a.groups = pk.groups.get(), a.ngroups = pk.counters.get() + 1;
-    a.out = l->h.get(), a.out_stride = F, a.limit = c.swiglu_limit;
+    a.out = l->h.get(), a.out_stride = F, a.limit = c.swiglu_limit, a.halves = halves;
     launched(l, launch_rows(c.gate_type, 2, a, M, max_groups, l->grid.get(), l->ctx, st), "experts gate/up");
   }
   mark(l, ST_DOWN, st);  // the down stage starts with its input's quantiser
@@ -661,7 +665,7 @@ void stage_experts(moe_layer *l, const ActSource &src, const PackBuffers &pk, ui
     a.act = l->hq_routed.view(), a.act_row = nullptr;
     a.groups = pk.groups.get(), a.ngroups = pk.counters.get() + 1;
     if (y16) throw std::logic_error("f16 results with experts on the integer-dot kernels");
-    a.out = (float *)y, a.out_stride = E;
+    a.out = (float *)y, a.out_stride = E, a.halves = halves;
     launched(l, launch_rows(c.down_type, 1, a, M, max_groups, l->grid.get(), l->ctx, st), "experts down");
   }
 }
