@@ -405,7 +405,8 @@ void create(moe_layer *l, const moe_layer_config &c, const moe_layer_weights &w)
 // The bound. An approximate logit differs from the fp32 sum in the exact order by (a) the dropped lo * lo products and
 // the rounding of the lo parts, at most 2^-20 of sum |x_i w_i|; (b) the roundings of the accumulations, each taken as
 // at most 2^-23 of the running sum, one per MMA of 16 values and three MMAs a step: 3 E / 16 of them; (c) the exact
-// order's own roundings: chains of E / 8 fused multiply-adds at 2^-24 of the running sum each, then eight additions.
+// order's own roundings: chains of E / 8 fused multiply-adds at 2^-24 of the running sum each, then eight additions, and
+// the up to three that put a split product's pieces together.
 // sum |x_i w_i| <= |x| |w_e| (Cauchy-Schwarz), so eps = eps_rel |x| max_e |w_e| with eps_rel = (3 E / 16 + E / 8 + 16) 2^-23
 // (2^-13.6 at E = 2048) covers all three in the worst case, where every rounding falls the same way; measured errors
 // are some hundred times smaller, and the GPU tests hold them under a quarter of the bound. The bias adds one rounding
@@ -445,7 +446,9 @@ void setup_router_tensor(moe_layer *l, const float *router, const float *bias, c
   l->rx_hi.alloc(xrows * E), l->rx_lo.alloc(xrows * E);
   CUDA_OK(cudaMemsetAsync(l->rx_hi.get(), 0, xrows * E * sizeof(__half), st));
   CUDA_OK(cudaMemsetAsync(l->rx_lo.get(), 0, xrows * E * sizeof(__half), st));
-  l->approx.alloc((size_t)T * NE), l->norm2_parts.alloc((size_t)T * (E / 256));
+  // In a short step a logit comes in up to four pieces (stage_route), as long as there are no more items than SMs.
+  const uint64_t split_rows = (uint64_t)kRouterTileRows * l->sms / ((NE + 127) / 128);
+  l->approx.alloc(std::max<uint64_t>(T, std::min<uint64_t>(4ull * T, split_rows)) * NE), l->norm2_parts.alloc((size_t)T * (E / 256));
   l->rw_hi_map = make_rows_map(l->rw_hi.get(), wrows, E, 128);  // 128 experts a box: an item takes one or two
   l->rw_lo_map = make_rows_map(l->rw_lo.get(), wrows, E, 128);
   l->rx_hi_map = make_rows_map(l->rx_hi.get(), xrows, E, kRouterTileRows);
@@ -537,6 +540,7 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
                   RouterSplit{l->rx_hi.get(), l->rx_lo.get(), l->norm2_parts.get()});
   if (approx && l->has_shared && !l->shared_x_same) quantize_rows(l, x, T, E, l->xq_shared, st);
   mark(l, ST_ROUTER, st);
+  uint32_t router_parts = 1;
   if (!approx) {
     launch_router_rows(l, x, T, st);
   } else {
@@ -548,8 +552,10 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
     // they still all run at once (8,192 rows: 128 items of 256 experts took 50 us, 256 items of 128 took 62).
     const uint32_t row_tiles = (T + kRouterTileRows - 1) / kRouterTileRows;
     const uint32_t ne_tile = 2 * row_tiles * ((NE + kRouterTileExperts - 1) / kRouterTileExperts) <= l->sms ? 128 : kRouterTileExperts;
-    const RouterMmaArgs ra{T, E, NE, ne_tile, l->rw_unscale.get(), l->approx.get(), l->error.get()};
-    const uint32_t items = row_tiles * ((NE + ne_tile - 1) / ne_tile);
+    const uint32_t tiles = row_tiles * ((NE + ne_tile - 1) / ne_tile);
+    router_parts = 4 * tiles <= l->sms ? 4 : 2 * tiles <= l->sms ? 2 : 1;
+    const RouterMmaArgs ra{T, E, NE, ne_tile, l->rw_unscale.get(), router_parts, l->approx.get(), l->error.get()};
+    const uint32_t items = tiles * router_parts;
     k_router_mma<<<std::min(items, l->sms), kRouterThreads, kRouterSmemBytes, st>>>(ra, l->rx_hi_map, l->rx_lo_map, l->rw_hi_map, l->rw_lo_map);
     launched(l, cudaGetLastError(), "router logits");
   }
@@ -567,7 +573,7 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
     mark(l, ST_PACK, st);
   } else {
     if (approx) {
-      const RouterApprox ap{l->approx.get(), x, l->router.get(), l->norm2_parts.get(), l->gate_parts.get(), E, E / 256,
+      const RouterApprox ap{l->approx.get(), x, l->router.get(), l->norm2_parts.get(), l->gate_parts.get(), E, E / 256, router_parts, (uint64_t)T * NE,
                             l->router_eps_rel, l->router_eps_abs};
       k_router_topk_rows<<<(T + kTopkRowsPerCta - 1) / kTopkRowsPerCta, 32 * kTopkRowsPerCta, 0, st>>>(ap, l->bias.get(), T, NE, K, l->ids.get(),
                                                                                                   l->w.get(), l->gs.get());

@@ -7,7 +7,9 @@
 // as three f16 MMAs into one f32 accumulator. The router's rows are scaled by a power of two per expert so that their
 // lo parts are normal f16 numbers; the scale is taken out again, exactly, when the accumulators are read.
 //
-// A work item is 128 rows of x by 256 experts (128 in steps too short to give every SM an item of 256); persistent CTAs of six warps take items in turn: one thread issues the
+// A work item is 128 rows of x by 256 experts (128 in steps too short to give every SM an item of 256, and then, where that
+// still leaves SMs idle, a half or a quarter of the row: an item is a chain of stages at the pace of one SM's copies,
+// 32 of them and some 33 us at 2,048 values a row, however few items there are); persistent CTAs of six warps take items in turn: one thread issues the
 // bulk-tensor copies (x hi and lo: 64 values x 128 rows; the router's hi and lo: 64 values x 256 experts, all in the
 // 128-byte-swizzled K-major layout), one issues the MMAs (M 128, N 256, K 16; twelve a stage), four warps read the
 // accumulators back and store the logits. Tensor memory holds two accumulators of 256 columns, so the MMAs of item
@@ -29,7 +31,8 @@ struct RouterMmaArgs {
   uint32_t T, E, NE;
   uint32_t ne_tile;        // experts an item takes: 256, or 128 when items of 256 would leave SMs without one
   const float *w_unscale;  // [NE]: what an accumulator is multiplied by (the inverse of the expert's power-of-two scale)
-  float *logits;           // [T][NE]
+  uint32_t parts;          // pieces of the row an item's product is cut into (each a whole number of stages): 1, 2 or 4
+  float *logits;           // [parts][T][NE]: each piece's sums; the top-k kernel adds them
   uint32_t *error;         // set non-zero when a wait ran out
 };
 
@@ -41,8 +44,8 @@ static __global__ void __launch_bounds__(kRouterThreads, 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const uint32_t KT = a.E / kRouterTileK, ne_tile = a.ne_tile, col_tiles = (a.NE + ne_tile - 1) / ne_tile;
-  const uint32_t nitems = ((a.T + kRouterTileRows - 1) / kRouterTileRows) * col_tiles;
+  const uint32_t KT = a.E / kRouterTileK / a.parts, ne_tile = a.ne_tile, col_tiles = (a.NE + ne_tile - 1) / ne_tile;
+  const uint32_t tiles = ((a.T + kRouterTileRows - 1) / kRouterTileRows) * col_tiles, nitems = tiles * a.parts;
   if (blockIdx.x >= nitems) return;
   uint64_t *bars = (uint64_t *)(smem + S * kRouterStageBytes);
   const uint32_t bar0 = smem_u32(bars);
@@ -70,12 +73,12 @@ static __global__ void __launch_bounds__(kRouterThreads, 1)
     if (lane == 0) {
       uint32_t li = 0;
       for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x, li++) {
-        const uint32_t row0 = (item / col_tiles) * kRouterTileRows, e0 = (item % col_tiles) * ne_tile;
+        const uint32_t tile = item % tiles, row0 = (tile / col_tiles) * kRouterTileRows, e0 = (tile % col_tiles) * ne_tile;
         for (uint32_t it = 0; it < KT && ok; it++) {
           const uint32_t g = li * KT + it, s = g % S, use_s = g / S;
           if (use_s > 0) ok = mbar_wait(empty_bar(s), (use_s - 1) & 1, abort, a.error);
           if (!ok) break;
-          const uint32_t st = smem_u32(smem + s * kRouterStageBytes), k0 = it * kRouterTileK;
+          const uint32_t st = smem_u32(smem + s * kRouterStageBytes), k0 = (item / tiles * KT + it) * kRouterTileK;
           // The router's maps copy 128 experts' rows a box: one or two boxes for each half.
           mbar_arrive_expect(full_bar(s), 2 * kRouterABytes + 2 * ne_tile * kRouterTileK * 2);
           tma_load_rows(st, &x_hi, k0, row0, full_bar(s));
@@ -126,13 +129,13 @@ static __global__ void __launch_bounds__(kRouterThreads, 1)
     const uint32_t q = warp % 4;
     uint32_t li = 0;
     for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x, li++) {
-      const uint32_t row0 = (item / col_tiles) * kRouterTileRows, e0 = (item % col_tiles) * ne_tile;
+      const uint32_t tile = item % tiles, row0 = (tile / col_tiles) * kRouterTileRows, e0 = (tile % col_tiles) * ne_tile;
       const uint32_t b = li & 1, use_b = li / 2;
       ok = mbar_wait(acc_full(b), use_b & 1, abort, a.error);
       if (!ok) break;
       tc_fence_after();
       const uint32_t t = row0 + 32 * q + lane;
-      float *out = a.logits + (uint64_t)t * a.NE + e0;
+      float *out = a.logits + ((uint64_t)(item / tiles) * a.T + t) * a.NE + e0;
       for (uint32_t c = 0; c < ne_tile / 16; c++) {
         if (e0 + 16 * c >= a.NE) break;
         uint32_t v[16];

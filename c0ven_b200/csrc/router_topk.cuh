@@ -31,12 +31,14 @@ constexpr int kMaxPerLane = 16;  // experts a lane holds at most: 512 / 32
 // with |x_t|^2 summed from norm2_parts. The top-k below then recomputes, in the exact order, only what that bound
 // cannot decide.
 struct RouterApprox {
-  const float *logits;       // [T][NE]; null: the logits are exact rows rl[t][NE + 1]
+  float *logits;             // [parts][T][NE], to be added up (the sum is left in part 0); null: the logits are exact rows rl[t][NE + 1]
   const float *x;            // [T][E]
   const float *W;            // [NE][E]
   const float *norm2_parts;  // [T][nparts]
   const float *gate_parts;   // [T][nparts]: the parts of the shared expert's gate logit
   uint32_t E, nparts;
+  uint32_t parts;
+  uint64_t part_stride;      // T * NE
   float eps_rel, eps_abs;
 };
 
@@ -167,7 +169,12 @@ __device__ __forceinline__ void router_topk_row(uint32_t t, const float *__restr
       const uint32_t e = lane + 32 * j;
       float f;
       if (ap.logits) {
-        f = ap.logits[(uint64_t)t * NE + e];
+        float *at = ap.logits + (uint64_t)t * NE + e;
+        f = *at;
+        if (ap.parts > 1) {
+          for (uint32_t p = 1; p < ap.parts; p++) f += at[p * ap.part_stride];
+          *at = f;
+        }
         if (bias) f = __fadd_rn(f, bias[e]);
         finite = finite && isfinite(f);
       } else {
