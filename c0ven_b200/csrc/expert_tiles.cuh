@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "expert_rows.cuh"
 #include "formats.h"
@@ -285,45 +286,51 @@ __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefe
 __device__ __forceinline__ __half2 small_h2(uint32_t v) { return __hsub2(as_h2(0x64006400u | v | (v << 16)), as_h2(0x64006400u)); }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Decoders. A stage is 64 values of every one of the tile's 128 weight rows; a thread takes one half of a row's stage,
-// 32 values: it fetches the half's quants and scales into registers (Raw), a stage ahead, and later writes them as f16
-// into the operand tile, chunks 4 h .. 4 h + 3 of row m. All arithmetic is in f16 pairs; integers reach f16 through
-// the exponent trick above, never through a conversion instruction.
+// Decoders. A stage is 64 values of every one of the tile's 128 weight rows, and a thread turns a whole row of it into f16,
+// as two halves of 32 values: chunks 4 h .. 4 h + 3 of row m of the operand tile. All arithmetic is in f16 pairs;
+// integers reach f16 through the exponent trick above, never through a conversion instruction.
+//
+// A type whose quants come by the threads' own loads is fetched in units of kUnitStages stages of a row, into registers,
+// a unit ahead of the decode. A load whose lanes each read a row of their own costs the load pipe a wavefront a lane,
+// whatever its width, so a unit is as much of a row as one round of wide loads brings: half a block of 256 values (two
+// stages), whose codes, signs, high bits and scales are then 3 to 8 loads. (Fetched a stage at a time, in halves of 32,
+// the same 128 values were 8 to 28 loads: 28 for Q6_K, 20 for IQ2_S and IQ3_S.) The unit of Q8_0, IQ4_NL and IQ4_XS is
+// one stage: two units of two in flight spill registers there, which cost more than the loads (IQ4_XS and IQ4_NL, 4,352
+// rows of the benchmark's layer: 1.01 ms against 0.97).
 template <int QT>
 struct Decoder;
 
 // Q8_0: w = d * q. A half is one block.
 template <>
 struct Decoder<QT_Q8_0> {
-  static constexpr uint32_t kStageBytes = 64;  // bytes of a row's main quants run a 64-value stage reads
-  struct Hdr {};
-  __device__ static __forceinline__ Hdr fetch_hdr(const uint8_t *, uint64_t, uint32_t, uint32_t, uint32_t) { return Hdr{}; }
+  static constexpr uint32_t kUnitStages = 1;
+  static constexpr uint32_t kUnitBytes = 64;  // of the main quants run
+  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint32_t K, uint32_t r, uint32_t u) { return s + (uint64_t)r * K + 64 * u; }
   struct Raw {
-    uint4 q0, q1;
-    __half d;
+    uint4 q[4];
+    __half2 d;
   };
-  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint64_t, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    return s + (uint64_t)r * K + k0 + 32 * h;
-  }
-  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
+  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t u) {
     Raw x;
-    const uint8_t *q = s + (uint64_t)r * K + k0 + 32 * h;
-    x.q0 = ldg16(q), x.q1 = ldg16(q + 16);
-    x.d = __ldg((const __half *)(s + 32 * nblk) + (uint64_t)r * (K / 32) + k0 / 32 + h);
+    const uint8_t *q = quants_at(s, K, r, u);
+#pragma unroll
+    for (int i = 0; i < 4; i++) x.q[i] = ldg16(q + 16 * i);
+    x.d = __ldg((const __half2 *)((const __half *)(s + 32 * nblk) + (uint64_t)r * (K / 32) + 2 * u));
     return x;
   }
-  __device__ static __forceinline__ void store(const Hdr &, const Raw &x, uint8_t *tile, uint32_t m, uint32_t h, uint32_t, const uint32_t *) {
-    const __half2 d2 = __half2half2(x.d), off = as_h2(0x64806480u);  // 1152 = 1024 + 128
-    const uint32_t w[8] = {x.q0.x, x.q0.y, x.q0.z, x.q0.w, x.q1.x, x.q1.y, x.q1.z, x.q1.w};
-    uint32_t o[16];
+  template <int S>
+  __device__ static __forceinline__ void store(const Raw &x, uint8_t *tile, uint32_t m, const uint32_t *) {
+    const __half2 off = as_h2(0x64806480u);  // 1152 = 1024 + 128
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-      const uint32_t u = w[j] ^ 0x80808080u;  // int8 + 128
-      o[2 * j] = as_u32(__hmul2(__hsub2(as_h2(bias_h2(u, 0x4140)), off), d2));
-      o[2 * j + 1] = as_u32(__hmul2(__hsub2(as_h2(bias_h2(u, 0x4342)), off), d2));
+    for (int c = 0; c < 8; c++) {  // a chunk of eight values
+      const __half2 d2 = c < 4 ? __low2half2(x.d) : __high2half2(x.d);
+      const uint4 &q = x.q[c / 2];
+      const uint32_t u0 = (c & 1 ? q.z : q.x) ^ 0x80808080u, u1 = (c & 1 ? q.w : q.y) ^ 0x80808080u;  // int8 + 128
+      uint4 o;
+      o.x = as_u32(__hmul2(__hsub2(as_h2(bias_h2(u0, 0x4140)), off), d2)), o.y = as_u32(__hmul2(__hsub2(as_h2(bias_h2(u0, 0x4342)), off), d2));
+      o.z = as_u32(__hmul2(__hsub2(as_h2(bias_h2(u1, 0x4140)), off), d2)), o.w = as_u32(__hmul2(__hsub2(as_h2(bias_h2(u1, 0x4342)), off), d2));
+      store_chunk(tile, m, c, o);
     }
-#pragma unroll
-    for (int c = 0; c < 4; c++) store_chunk(tile, m, 4 * h + c, make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]));
   }
 };
 
@@ -333,7 +340,7 @@ struct Decoder<QT_Q8_0> {
 // block's d, dmin and scales are one 16-byte piece, loaded once for its four stages.
 template <>
 struct Decoder<QT_Q4_K> {
-  static constexpr uint32_t kStageBytes = 32;  // bytes of a row's main quants run a 64-value stage reads
+  static constexpr uint32_t kUnitStages = 1;
   struct Hdr {
     uint4 v;  // d, dmin; then the 12 bytes of packed scales and minimums
   };
@@ -342,12 +349,6 @@ struct Decoder<QT_Q4_K> {
   };
   __device__ static __forceinline__ Hdr fetch_hdr(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t k0) {
     return Hdr{__ldg((const uint4 *)(s + 128 * nblk + 16 * ((uint64_t)r * (K / 256) + k0 / 256)))};
-  }
-  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint64_t, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    return s + (uint64_t)r * (K / 2) + (k0 / 64) * 32 + 16 * h;
-  }
-  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    return Raw{ldg16(quants_at(s, nblk, K, r, k0, h))};
   }
   // The 6-bit scale and minimum of sub-blocks 2 c and 2 c + 1 (QUANT_FORMATS.md:386-392), each pair as two bytes of a word.
   __device__ static __forceinline__ void scales_of(const Hdr &x, uint32_t c, uint32_t &sc, uint32_t &mn) {
@@ -360,122 +361,140 @@ struct Decoder<QT_Q4_K> {
       sc = (p & 0x0F0Fu) | ((a >> 2) & 0x3030u), mn = ((p >> 4) & 0x0F0Fu) | ((b >> 2) & 0x3030u);
     }
   }
-  __device__ static __forceinline__ void store(const Hdr &hd, const Raw &x, uint8_t *tile, uint32_t m, uint32_t h, uint32_t k0, const uint32_t *) {
+  // The stage's 32 bytes of a row, both nibbles. A byte beside the exponent byte 0x64 is the f16 value 1024 + byte: 1024 + q
+  // for a low nibble, 1024 + 16 q for a high nibble left in place. q comes out exactly (v - 1024, or v / 16 - 64 in one
+  // fused step); then w = a * q + c with a = d * sc and c = -dmin * m, each a product of two f16 numbers rounded once,
+  // taken for both sub-blocks by one instruction and once for the stage.
+  __device__ static __forceinline__ void store(const Hdr &hd, const Raw (&x)[2], uint8_t *tile, uint32_t m, uint32_t k0) {
     uint32_t sc, mn;
     scales_of(hd, (k0 % 256) / 64, sc, mn);
-    // A byte beside the exponent byte 0x64 is the f16 value 1024 + byte: 1024 + q for a low nibble, 1024 + 16 q for a
-    // high nibble left in place. q comes out exactly (v - 1024, or v / 16 - 64 in one fused step); then w = a * q + c
-    // with a = d * sc and c = -dmin * m, rounded once.
-    const __half2 dm = as_h2(hd.v.x);
-    const float d = __low2float(dm), dmin = __high2float(dm);
-    const __half2 A0 = __float2half2_rn(d * (float)(sc & 0xFF)), A1 = __float2half2_rn(d * (float)(sc >> 8));
-    const __half2 C0 = __float2half2_rn(-dmin * (float)(mn & 0xFF)), C1 = __float2half2_rn(-dmin * (float)(mn >> 8));
-    const __half2 k1024 = as_h2(0x64006400u), k16th = as_h2(0x2C002C00u), km64 = as_h2(0xD400D400u);  // 1024, 1/16, -64
-    const uint32_t w[4] = {x.q.x, x.q.y, x.q.z, x.q.w};
-    uint32_t lo[8], hi[8];
+    const __half2 dm = as_h2(hd.v.x), k1024 = as_h2(0x64006400u), k16th = as_h2(0x2C002C00u), km64 = as_h2(0xD400D400u);  // 1024, 1/16, -64
+    const __half2 A = __hmul2(__low2half2(dm), __hsub2(as_h2(bias_h2(sc, 0x4140)), k1024));
+    const __half2 C = __hmul2(__high2half2(dm), __hsub2(k1024, as_h2(bias_h2(mn, 0x4140))));
+    const __half2 A0 = __low2half2(A), A1 = __high2half2(A), C0 = __low2half2(C), C1 = __high2half2(C);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const uint32_t l = w[i] & 0x0F0F0F0Fu, g = w[i] & 0xF0F0F0F0u;
-      lo[2 * i] = as_u32(__hfma2(__hsub2(as_h2(bias_h2(l, 0x4140)), k1024), A0, C0));
-      lo[2 * i + 1] = as_u32(__hfma2(__hsub2(as_h2(bias_h2(l, 0x4342)), k1024), A0, C0));
-      hi[2 * i] = as_u32(__hfma2(__hfma2(as_h2(bias_h2(g, 0x4140)), k16th, km64), A1, C1));
-      hi[2 * i + 1] = as_u32(__hfma2(__hfma2(as_h2(bias_h2(g, 0x4342)), k16th, km64), A1, C1));
+    for (int h = 0; h < 2; h++) {
+      const uint32_t w[4] = {x[h].q.x, x[h].q.y, x[h].q.z, x[h].q.w};
+      uint32_t lo[8], hi[8];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const uint32_t l = w[i] & 0x0F0F0F0Fu, g = w[i] & 0xF0F0F0F0u;
+        lo[2 * i] = as_u32(__hfma2(__hsub2(as_h2(bias_h2(l, 0x4140)), k1024), A0, C0));
+        lo[2 * i + 1] = as_u32(__hfma2(__hsub2(as_h2(bias_h2(l, 0x4342)), k1024), A0, C0));
+        hi[2 * i] = as_u32(__hfma2(__hfma2(as_h2(bias_h2(g, 0x4140)), k16th, km64), A1, C1));
+        hi[2 * i + 1] = as_u32(__hfma2(__hfma2(as_h2(bias_h2(g, 0x4342)), k16th, km64), A1, C1));
+      }
+      store_chunk(tile, m, 2 * h, make_uint4(lo[0], lo[1], lo[2], lo[3]));
+      store_chunk(tile, m, 2 * h + 1, make_uint4(lo[4], lo[5], lo[6], lo[7]));
+      store_chunk(tile, m, 4 + 2 * h, make_uint4(hi[0], hi[1], hi[2], hi[3]));
+      store_chunk(tile, m, 5 + 2 * h, make_uint4(hi[4], hi[5], hi[6], hi[7]));
     }
-    store_chunk(tile, m, 2 * h, make_uint4(lo[0], lo[1], lo[2], lo[3]));
-    store_chunk(tile, m, 2 * h + 1, make_uint4(lo[4], lo[5], lo[6], lo[7]));
-    store_chunk(tile, m, 4 + 2 * h, make_uint4(hi[0], hi[1], hi[2], hi[3]));
-    store_chunk(tile, m, 5 + 2 * h, make_uint4(hi[4], hi[5], hi[6], hi[7]));
   }
 };
 
-// Q6_K: w = d * scales[v / 16] * (q - 32). A stage is a quarter of a block: one nibble of 64 bytes of ql and two bits
-// of 32 bytes of qh; a half is 32 bytes of ql with all 32 of qh, two groups of 16 with a scale each.
+// Q6_K: w = d * scales[v / 16] * (q - 32). A unit is half a block: 64 bytes of ql, whose low nibbles are the first stage's
+// values and whose high ones the second's, 32 bytes of qh (bits 0, 1 and 2, 3 of them the first stage's halves, 4, 5 and
+// 6, 7 the second's) and eight scales, two a half.
 template <>
 struct Decoder<QT_Q6_K> {
-  static constexpr uint32_t kStageBytes = 32;  // bytes of a row's main quants run a 64-value stage reads
-  struct Hdr {};
-  __device__ static __forceinline__ Hdr fetch_hdr(const uint8_t *, uint64_t, uint32_t, uint32_t, uint32_t) { return Hdr{}; }
+  static constexpr uint32_t kUnitStages = 2;
+  static constexpr uint32_t kUnitBytes = 64;  // of the main quants run
+  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint32_t K, uint32_t r, uint32_t u) { return s + (uint64_t)r * (K / 2) + 64 * u; }
   struct Raw {
-    uint4 l0, l1, h0, h1;
-    int sc0, sc1;
+    uint4 l[4], h[2];
+    uint2 sc;
     __half d;
   };
-  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint64_t, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    return s + 128 * ((uint64_t)r * (K / 256) + k0 / 256) + 64 * ((k0 % 256) / 128) + 32 * h;
-  }
-  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    const uint32_t v0 = k0 % 256, hh = v0 / 128;  // the stage starts at value v0 of its block: 0, 64, 128 or 192
-    const uint64_t blk = (uint64_t)r * (K / 256) + k0 / 256;
+  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t u) {
+    const uint64_t blk = (uint64_t)r * (K / 256) + u / 2;
+    const uint32_t hh = u % 2;
     Raw x;
-    const uint8_t *ql = s + 128 * blk + 64 * hh + 32 * h, *qh = s + 128 * nblk + 64 * blk + 32 * hh;
-    x.l0 = ldg16(ql), x.l1 = ldg16(ql + 16), x.h0 = ldg16(qh), x.h1 = ldg16(qh + 16);
-    const int8_t *sc = (const int8_t *)(s + 192 * nblk + 16 * blk) + v0 / 16 + 2 * h;
-    x.sc0 = __ldg(sc), x.sc1 = __ldg(sc + 1);
+    const uint8_t *ql = quants_at(s, K, r, u), *qh = s + 128 * nblk + 64 * blk + 32 * hh;
+#pragma unroll
+    for (int i = 0; i < 4; i++) x.l[i] = ldg16(ql + 16 * i);
+    x.h[0] = ldg16(qh), x.h[1] = ldg16(qh + 16);
+    x.sc = __ldg((const uint2 *)(s + 192 * nblk + 16 * blk + 8 * hh));
     x.d = __ldg((const __half *)(s + 208 * nblk) + blk);
     return x;
   }
-  __device__ static __forceinline__ void store(const Hdr &, const Raw &x, uint8_t *tile, uint32_t m, uint32_t h, uint32_t k0, const uint32_t *) {
-    const bool high = (k0 % 128) >= 64;  // values 64 .. 127 of the block's half: the high nibbles, qh's bits 4 .. 7
-    const uint32_t sh = (high ? 4 : 0) + (h ? 2 : 0), nsh = high ? 4 : 0;
+  template <int S>
+  __device__ static __forceinline__ void store(const Raw &x, uint8_t *tile, uint32_t m, const uint32_t *) {
     const __half2 d2 = __half2half2(x.d), off = as_h2(0x64206420u), o128 = as_h2(0x64806480u);  // 1056 = 1024 + 32; 1152
-    const __half2 ds0 = __hmul2(d2, __hsub2(as_h2(0x64006400u | (uint32_t)(x.sc0 + 128) * 0x10001u), o128));
-    const __half2 ds1 = __hmul2(d2, __hsub2(as_h2(0x64006400u | (uint32_t)(x.sc1 + 128) * 0x10001u), o128));
-    const uint32_t l[8] = {x.l0.x, x.l0.y, x.l0.z, x.l0.w, x.l1.x, x.l1.y, x.l1.z, x.l1.w};
-    const uint32_t b[8] = {x.h0.x, x.h0.y, x.h0.z, x.h0.w, x.h1.x, x.h1.y, x.h1.z, x.h1.w};
-    uint32_t o[16];
+    const uint32_t b[8] = {x.h[0].x, x.h[0].y, x.h[0].z, x.h[0].w, x.h[1].x, x.h[1].y, x.h[1].z, x.h[1].w};
+    const uint32_t scu = (S ? x.sc.y : x.sc.x) ^ 0x80808080u;  // int8 + 128
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const uint32_t q = ((l[i] >> nsh) & 0x0F0F0F0Fu) | (((b[i] >> sh) & 0x03030303u) << 4);
-      const __half2 ds = i < 4 ? ds0 : ds1;
-      o[2 * i] = as_u32(__hmul2(__hsub2(as_h2(bias_h2(q, 0x4140)), off), ds));
-      o[2 * i + 1] = as_u32(__hmul2(__hsub2(as_h2(bias_h2(q, 0x4342)), off), ds));
+    for (int h = 0; h < 2; h++) {
+      const uint32_t l[8] = {x.l[2 * h].x, x.l[2 * h].y, x.l[2 * h].z, x.l[2 * h].w, x.l[2 * h + 1].x, x.l[2 * h + 1].y, x.l[2 * h + 1].z, x.l[2 * h + 1].w};
+      const __half2 ds0 = __hmul2(d2, __hsub2(as_h2(bias_h2(scu, h ? 0x4242 : 0x4040)), o128));
+      const __half2 ds1 = __hmul2(d2, __hsub2(as_h2(bias_h2(scu, h ? 0x4343 : 0x4141)), o128));
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        uint4 o;
+        uint32_t *p = &o.x;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          const int i = 2 * c + k;
+          const uint32_t q = ((l[i] >> (4 * S)) & 0x0F0F0F0Fu) | (((b[i] >> (4 * S + 2 * h)) & 0x03030303u) << 4);
+          const __half2 ds = i < 4 ? ds0 : ds1;
+          p[2 * k] = as_u32(__hmul2(__hsub2(as_h2(bias_h2(q, 0x4140)), off), ds));
+          p[2 * k + 1] = as_u32(__hmul2(__hsub2(as_h2(bias_h2(q, 0x4342)), off), ds));
+        }
+        store_chunk(tile, m, 4 * h + c, o);
+      }
     }
-#pragma unroll
-    for (int c = 0; c < 4; c++) store_chunk(tile, m, 4 * h + c, make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]));
   }
 };
 
 // IQ3_S: w = d * (1 + 2 s) * grid[index][i] * sign. A half is one sub-block of 32: 8 bytes of qs, a byte of qh, 4 of
-// signs, a nibble of scale. The codebook is in shared memory.
+// signs, a nibble of scale; a unit is four of them. The codebook is in shared memory.
 template <>
 struct Decoder<QT_IQ3_S> {
-  static constexpr uint32_t kStageBytes = 16;  // bytes of a row's main quants run a 64-value stage reads
-  struct Hdr {};
-  __device__ static __forceinline__ Hdr fetch_hdr(const uint8_t *, uint64_t, uint32_t, uint32_t, uint32_t) { return Hdr{}; }
+  static constexpr uint32_t kUnitStages = 2;
+  static constexpr uint32_t kUnitBytes = 32;  // of the main quants run
+  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint32_t K, uint32_t r, uint32_t u) { return s + (uint64_t)r * (K / 4) + 32 * u; }
   struct Raw {
-    uint2 qs;
-    uint32_t sg, qh, sc;
+    uint4 qs[2], sg;
+    uint32_t qh;
+    uint16_t sc;
     __half d;
   };
-  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint64_t, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    return s + 64 * ((uint64_t)r * (K / 256) + k0 / 256) + 8 * ((k0 % 256) / 32 + h);
-  }
-  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    const uint32_t sb = (k0 % 256) / 32 + h;  // the sub-block within its block
-    const uint64_t blk = (uint64_t)r * (K / 256) + k0 / 256;
+  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t u) {
+    const uint64_t blk = (uint64_t)r * (K / 256) + u / 2;
+    const uint32_t hh = u % 2;
     Raw x;
-    x.qs = __ldg((const uint2 *)(s + 64 * blk + 8 * sb));
-    x.sg = __ldg((const uint32_t *)(s + 64 * nblk + 32 * blk + 4 * sb));
-    x.qh = __ldg(s + 96 * nblk + 8 * blk + sb);
-    x.sc = (__ldg(s + 104 * nblk + 4 * blk + sb / 2) >> (4 * (sb & 1))) & 0xF;
+    const uint8_t *qs = quants_at(s, K, r, u);
+    x.qs[0] = ldg16(qs), x.qs[1] = ldg16(qs + 16);
+    x.sg = ldg16(s + 64 * nblk + 32 * blk + 16 * hh);
+    x.qh = __ldg((const uint32_t *)(s + 96 * nblk + 8 * blk + 4 * hh));
+    x.sc = __ldg((const uint16_t *)(s + 104 * nblk + 4 * blk + 2 * hh));
     x.d = __ldg((const __half *)(s + 108 * nblk) + blk);
     return x;
   }
-  __device__ static __forceinline__ void store(const Hdr &, const Raw &x, uint8_t *tile, uint32_t m, uint32_t h, uint32_t, const uint32_t *grid) {
-    const __half2 ls = small_h2(2 * x.sc + 1), d2 = __half2half2(x.d), off = as_h2(0x64006400u);
-    uint32_t o[16];
+  template <int S>
+  __device__ static __forceinline__ void store(const Raw &x, uint8_t *tile, uint32_t m, const uint32_t *grid) {
+    const __half2 d2 = __half2half2(x.d), off = as_h2(0x64006400u);
+    const uint32_t qs[4] = {x.qs[S].x, x.qs[S].y, x.qs[S].z, x.qs[S].w};
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const uint32_t word = k < 4 ? x.qs.x : x.qs.y;
-      const uint32_t g = grid[((word >> (8 * (k & 3))) & 0xFF) | (((x.qh >> k) & 1u) << 8)];
-      const uint32_t nib = (x.sg >> (4 * k)) & 0xF;
-      // The sign bit of each f16: values 4k, 4k + 1 from the nibble's bits 0, 1; 4k + 2, 4k + 3 from bits 2, 3.
-      const uint32_t s01 = ((nib & 1u) << 15) | ((nib & 2u) << 30), s23 = ((nib & 4u) << 13) | ((nib & 8u) << 28);
-      o[2 * k] = as_u32(__hmul2(__hmul2(__hsub2(as_h2(bias_h2(g, 0x4140)), off), ls), d2)) ^ s01;
-      o[2 * k + 1] = as_u32(__hmul2(__hmul2(__hsub2(as_h2(bias_h2(g, 0x4342)), off), ls), d2)) ^ s23;
+    for (int h = 0; h < 2; h++) {
+      const __half2 ls = small_h2(2 * (((uint32_t)x.sc >> (8 * S + 4 * h)) & 0xF) + 1);
+      const uint32_t qh = x.qh >> (16 * S + 8 * h), sg = S ? (h ? x.sg.w : x.sg.z) : (h ? x.sg.y : x.sg.x);
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        uint4 o;
+        uint32_t *p = &o.x;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          const int k = 2 * c + j;
+          const uint32_t g = grid[((qs[2 * h + k / 4] >> (8 * (k & 3))) & 0xFF) | (((qh >> k) & 1u) << 8)];
+          const uint32_t nib = (sg >> (4 * k)) & 0xF;
+          // The sign bit of each f16: values 4k, 4k + 1 from the nibble's bits 0, 1; 4k + 2, 4k + 3 from bits 2, 3.
+          const uint32_t s01 = ((nib & 1u) << 15) | ((nib & 2u) << 30), s23 = ((nib & 4u) << 13) | ((nib & 8u) << 28);
+          p[2 * j] = as_u32(__hmul2(__hmul2(__hsub2(as_h2(bias_h2(g, 0x4140)), off), ls), d2)) ^ s01;
+          p[2 * j + 1] = as_u32(__hmul2(__hmul2(__hsub2(as_h2(bias_h2(g, 0x4342)), off), ls), d2)) ^ s23;
+        }
+        store_chunk(tile, m, 4 * h + c, o);
+      }
     }
-#pragma unroll
-    for (int c = 0; c < 4; c++) store_chunk(tile, m, 4 * h + c, make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]));
   }
 };
 
@@ -489,80 +508,87 @@ __device__ __forceinline__ void grid_word_to_f16(uint32_t g, uint32_t nib, __hal
 }
 
 // IQ3_XXS: w = d * (0.5 + s) / 2 * grid[index][i] * sign. A half is one sub-block of 32: 8 bytes of indices and its
-// word of four 7-bit sign indices and the scale. The codebook is in shared memory.
+// word of four 7-bit sign indices and the scale; a unit is four of them. The codebook is in shared memory.
 template <>
 struct Decoder<QT_IQ3_XXS> {
-  static constexpr uint32_t kStageBytes = 16;  // bytes of a row's main quants run a 64-value stage reads
-  struct Hdr {};
-  __device__ static __forceinline__ Hdr fetch_hdr(const uint8_t *, uint64_t, uint32_t, uint32_t, uint32_t) { return Hdr{}; }
+  static constexpr uint32_t kUnitStages = 2;
+  static constexpr uint32_t kUnitBytes = 32;  // of the main quants run
+  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint32_t K, uint32_t r, uint32_t u) { return s + (uint64_t)r * (K / 4) + 32 * u; }
   struct Raw {
-    uint2 qs;
-    uint32_t w32;
+    uint4 qs[2], w32;
     __half d;
   };
-  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint64_t, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    return s + 64 * ((uint64_t)r * (K / 256) + k0 / 256) + 8 * ((k0 % 256) / 32 + h);
-  }
-  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    const uint32_t sb = (k0 % 256) / 32 + h;  // the sub-block within its block
-    const uint64_t blk = (uint64_t)r * (K / 256) + k0 / 256;
+  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t u) {
+    const uint64_t blk = (uint64_t)r * (K / 256) + u / 2;
+    const uint32_t hh = u % 2;
     Raw x;
-    x.qs = __ldg((const uint2 *)(s + 64 * blk + 8 * sb));
-    x.w32 = __ldg((const uint32_t *)(s + 64 * nblk + 32 * blk + 4 * sb));
+    const uint8_t *qs = quants_at(s, K, r, u);
+    x.qs[0] = ldg16(qs), x.qs[1] = ldg16(qs + 16);
+    x.w32 = ldg16(s + 64 * nblk + 32 * blk + 16 * hh);
     x.d = __ldg((const __half *)(s + 96 * nblk) + blk);
     return x;
   }
-  __device__ static __forceinline__ void store(const Hdr &, const Raw &x, uint8_t *tile, uint32_t m, uint32_t h, uint32_t, const uint32_t *grid) {
-    // d * (2 s + 1) / 4, rounded to f16 once.
-    const __half2 sc = __float2half2_rn(__half2float(x.d) * (float)(2 * (x.w32 >> 28) + 1) * 0.25f);
-    uint32_t o[16];
+  template <int S>
+  __device__ static __forceinline__ void store(const Raw &x, uint8_t *tile, uint32_t m, const uint32_t *grid) {
+    const uint32_t qs[4] = {x.qs[S].x, x.qs[S].y, x.qs[S].z, x.qs[S].w};
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const uint32_t word = k < 4 ? x.qs.x : x.qs.y;
-      const uint32_t k7 = (x.w32 >> (7 * (k >> 1))) & 127u, sbyte = k7 | ((__popc(k7) & 1u) << 7);
-      grid_word_to_f16(grid[(word >> (8 * (k & 3))) & 0xFF], (sbyte >> (4 * (k & 1))) & 0xF, sc, o + 2 * k);
+    for (int h = 0; h < 2; h++) {
+      const uint32_t w32 = S ? (h ? x.w32.w : x.w32.z) : (h ? x.w32.y : x.w32.x);
+      // d * (2 s + 1) / 4, rounded to f16 once.
+      const __half2 sc = __float2half2_rn(__half2float(x.d) * (float)(2 * (w32 >> 28) + 1) * 0.25f);
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const uint32_t k7 = (w32 >> (7 * c)) & 127u, sbyte = k7 | ((__popc(k7) & 1u) << 7);
+        const uint32_t word = qs[2 * h + c / 2] >> (16 * (c & 1));
+        uint32_t o[4];
+        grid_word_to_f16(grid[word & 0xFF], sbyte & 0xF, sc, o), grid_word_to_f16(grid[(word >> 8) & 0xFF], sbyte >> 4, sc, o + 2);
+        store_chunk(tile, m, 4 * h + c, make_uint4(o[0], o[1], o[2], o[3]));
+      }
     }
-#pragma unroll
-    for (int c = 0; c < 4; c++) store_chunk(tile, m, 4 * h + c, make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]));
   }
 };
 
 // IQ2_S: w = d * (0.5 + s) / 4 * grid[index][i] * sign. A half is one sub-block of 32: four groups of 8 values, each a
 // 10-bit index (a byte of qs, two bits of the sub-block's qh byte) and a byte of signs; a scale nibble per two groups.
+// A unit is four sub-blocks.
 template <>
 struct Decoder<QT_IQ2_S> {
-  static constexpr uint32_t kStageBytes = 8;  // bytes of a row's main quants run a 64-value stage reads
-  struct Hdr {};
-  __device__ static __forceinline__ Hdr fetch_hdr(const uint8_t *, uint64_t, uint32_t, uint32_t, uint32_t) { return Hdr{}; }
+  static constexpr uint32_t kUnitStages = 2;
+  static constexpr uint32_t kUnitBytes = 16;  // of the main quants run
+  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint32_t K, uint32_t r, uint32_t u) { return s + (uint64_t)r * (K / 8) + 16 * u; }
   struct Raw {
-    uint32_t qs, sg, qh, sc;
+    uint4 qs, sg;
+    uint32_t qh, sc;
     __half d;
   };
-  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint64_t, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    return s + 32 * ((uint64_t)r * (K / 256) + k0 / 256) + 4 * ((k0 % 256) / 32 + h);
-  }
-  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    const uint32_t sb = (k0 % 256) / 32 + h;
-    const uint64_t blk = (uint64_t)r * (K / 256) + k0 / 256;
+  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t u) {
+    const uint64_t blk = (uint64_t)r * (K / 256) + u / 2;
+    const uint32_t hh = u % 2;
     Raw x;
-    x.qs = __ldg((const uint32_t *)(s + 32 * blk + 4 * sb));
-    x.sg = __ldg((const uint32_t *)(s + 32 * nblk + 32 * blk + 4 * sb));
-    x.qh = __ldg(s + 64 * nblk + 8 * blk + sb);
-    x.sc = __ldg(s + 72 * nblk + 8 * blk + sb);
+    x.qs = ldg16(quants_at(s, K, r, u));
+    x.sg = ldg16(s + 32 * nblk + 32 * blk + 16 * hh);
+    x.qh = __ldg((const uint32_t *)(s + 64 * nblk + 8 * blk + 4 * hh));
+    x.sc = __ldg((const uint32_t *)(s + 72 * nblk + 8 * blk + 4 * hh));
     x.d = __ldg((const __half *)(s + 80 * nblk) + blk);
     return x;
   }
-  __device__ static __forceinline__ void store(const Hdr &, const Raw &x, uint8_t *tile, uint32_t m, uint32_t h, uint32_t, const uint32_t *grid) {
+  template <int S>
+  __device__ static __forceinline__ void store(const Raw &x, uint8_t *tile, uint32_t m, const uint32_t *grid) {
     const float d8 = __half2float(x.d) * 0.125f;  // d * (2 s + 1) / 8
-    const __half2 sc_lo = __float2half2_rn(d8 * (float)(2 * (x.sc & 0xF) + 1)), sc_hi = __float2half2_rn(d8 * (float)(2 * (x.sc >> 4) + 1));
     const uint2 *grid2 = (const uint2 *)grid;
 #pragma unroll
-    for (int g = 0; g < 4; g++) {
-      const uint2 e = grid2[((x.qs >> (8 * g)) & 0xFF) | (((x.qh >> (2 * g)) & 3u) << 8)];
-      const uint32_t sb = (x.sg >> (8 * g)) & 0xFF;
-      uint32_t o[4];
-      grid_word_to_f16(e.x, sb & 0xF, g < 2 ? sc_lo : sc_hi, o), grid_word_to_f16(e.y, sb >> 4, g < 2 ? sc_lo : sc_hi, o + 2);
-      store_chunk(tile, m, 4 * h + g, make_uint4(o[0], o[1], o[2], o[3]));
+    for (int h = 0; h < 2; h++) {
+      const uint32_t sc = x.sc >> (16 * S + 8 * h), qh = x.qh >> (16 * S + 8 * h);
+      const uint32_t qs = S ? (h ? x.qs.w : x.qs.z) : (h ? x.qs.y : x.qs.x), sg = S ? (h ? x.sg.w : x.sg.z) : (h ? x.sg.y : x.sg.x);
+      const __half2 sc_lo = __float2half2_rn(d8 * (float)(2 * (sc & 0xF) + 1)), sc_hi = __float2half2_rn(d8 * (float)(2 * ((sc >> 4) & 0xF) + 1));
+#pragma unroll
+      for (int g = 0; g < 4; g++) {
+        const uint2 e = grid2[((qs >> (8 * g)) & 0xFF) | (((qh >> (2 * g)) & 3u) << 8)];
+        const uint32_t sb = (sg >> (8 * g)) & 0xFF;
+        uint32_t o[4];
+        grid_word_to_f16(e.x, sb & 0xF, g < 2 ? sc_lo : sc_hi, o), grid_word_to_f16(e.y, sb >> 4, g < 2 ? sc_lo : sc_hi, o + 2);
+        store_chunk(tile, m, 4 * h + g, make_uint4(o[0], o[1], o[2], o[3]));
+      }
     }
   }
 };
@@ -587,87 +613,90 @@ __device__ __forceinline__ void iq4_store32(const uint4 &q, __half2 d2, uint8_t 
   for (int c = 0; c < 4; c++) store_chunk(tile, m, 4 * h + c, make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]));
 }
 
-// Q2_0: w = (q - 1) * d. A stage is one block of 64; a half is 8 of its 16 bytes.
+// Q2_0: w = (q - 1) * d. A stage is one block of 64, 16 bytes.
 template <>
 struct Decoder<QT_Q2_0> {
-  static constexpr uint32_t kStageBytes = 16;  // bytes of a row's main quants run a 64-value stage reads
-  struct Hdr {};
-  __device__ static __forceinline__ Hdr fetch_hdr(const uint8_t *, uint64_t, uint32_t, uint32_t, uint32_t) { return Hdr{}; }
+  static constexpr uint32_t kUnitStages = 2;
+  static constexpr uint32_t kUnitBytes = 32;  // of the main quants run
+  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint32_t K, uint32_t r, uint32_t u) { return s + (uint64_t)r * (K / 4) + 32 * u; }
   struct Raw {
-    uint2 q;
-    __half d;
+    uint4 q[2];
+    __half2 d;
   };
-  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint64_t, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    return s + (uint64_t)r * (K / 4) + k0 / 4 + 8 * h;
-  }
-  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
+  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t u) {
     Raw x;
-    x.q = __ldg((const uint2 *)quants_at(s, nblk, K, r, k0, h));
-    x.d = __ldg((const __half *)(s + 16 * nblk) + (uint64_t)r * (K / 64) + k0 / 64);
+    const uint8_t *q = quants_at(s, K, r, u);
+    x.q[0] = ldg16(q), x.q[1] = ldg16(q + 16);
+    x.d = __ldg((const __half2 *)((const __half *)(s + 16 * nblk) + (uint64_t)r * (K / 64) + 2 * u));
     return x;
   }
-  __device__ static __forceinline__ void store(const Hdr &, const Raw &x, uint8_t *tile, uint32_t m, uint32_t h, uint32_t, const uint32_t *) {
-    uint32_t w[8], o[16];
+  template <int S>
+  __device__ static __forceinline__ void store(const Raw &x, uint8_t *tile, uint32_t m, const uint32_t *) {
+    const __half2 d2 = S ? __high2half2(x.d) : __low2half2(x.d);
+    const uint32_t q[4] = {x.q[S].x, x.q[S].y, x.q[S].z, x.q[S].w};
 #pragma unroll
-    for (int i = 0; i < 8; i++) w[i] = q2_bytes(((i < 4 ? x.q.x : x.q.y) >> (8 * (i & 3))) & 0xFF);
-    const __half2 d2 = __half2half2(x.d);
-    int8x16_to_f16(*(const uint32_t(*)[4])&w[0], d2, o), int8x16_to_f16(*(const uint32_t(*)[4])&w[4], d2, o + 8);
+    for (int i = 0; i < 4; i++) {  // 16 values a word
+      uint32_t w[4], o[8];
 #pragma unroll
-    for (int c = 0; c < 4; c++) store_chunk(tile, m, 4 * h + c, make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]));
+      for (int j = 0; j < 4; j++) w[j] = q2_bytes((q[i] >> (8 * j)) & 0xFF);
+      int8x16_to_f16(w, d2, o);
+      store_chunk(tile, m, 2 * i, make_uint4(o[0], o[1], o[2], o[3])), store_chunk(tile, m, 2 * i + 1, make_uint4(o[4], o[5], o[6], o[7]));
+    }
   }
 };
 
 // IQ4_NL: w = d * table[q]. A half is one block of 32.
 template <>
 struct Decoder<QT_IQ4_NL> {
-  static constexpr uint32_t kStageBytes = 32;  // bytes of a row's main quants run a 64-value stage reads
-  struct Hdr {};
-  __device__ static __forceinline__ Hdr fetch_hdr(const uint8_t *, uint64_t, uint32_t, uint32_t, uint32_t) { return Hdr{}; }
+  static constexpr uint32_t kUnitStages = 1;
+  static constexpr uint32_t kUnitBytes = 32;  // of the main quants run
+  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint32_t K, uint32_t r, uint32_t u) { return s + (uint64_t)r * (K / 2) + 32 * u; }
   struct Raw {
-    uint4 q;
-    __half d;
+    uint4 q[2];
+    __half2 d;
   };
-  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint64_t, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    return s + (uint64_t)r * (K / 2) + k0 / 2 + 16 * h;
-  }
-  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
+  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t u) {
     Raw x;
-    x.q = ldg16(quants_at(s, nblk, K, r, k0, h));
-    x.d = __ldg((const __half *)(s + 16 * nblk) + (uint64_t)r * (K / 32) + k0 / 32 + h);
+    const uint8_t *q = quants_at(s, K, r, u);
+    x.q[0] = ldg16(q), x.q[1] = ldg16(q + 16);
+    x.d = __ldg((const __half2 *)((const __half *)(s + 16 * nblk) + (uint64_t)r * (K / 32) + 2 * u));
     return x;
   }
-  __device__ static __forceinline__ void store(const Hdr &, const Raw &x, uint8_t *tile, uint32_t m, uint32_t h, uint32_t, const uint32_t *) {
-    iq4_store32(x.q, __half2half2(x.d), tile, m, h);
+  template <int S>
+  __device__ static __forceinline__ void store(const Raw &x, uint8_t *tile, uint32_t m, const uint32_t *) {
+    iq4_store32(x.q[0], __low2half2(x.d), tile, m, 0), iq4_store32(x.q[1], __high2half2(x.d), tile, m, 1);
   }
 };
 
 // IQ4_XS: w = d * (ls - 32) * table[q]. A half is one sub-block of 32 with its 6-bit ls.
 template <>
 struct Decoder<QT_IQ4_XS> {
-  static constexpr uint32_t kStageBytes = 32;  // bytes of a row's main quants run a 64-value stage reads
-  struct Hdr {};
-  __device__ static __forceinline__ Hdr fetch_hdr(const uint8_t *, uint64_t, uint32_t, uint32_t, uint32_t) { return Hdr{}; }
+  static constexpr uint32_t kUnitStages = 1;
+  static constexpr uint32_t kUnitBytes = 32;  // of the main quants run
+  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint32_t K, uint32_t r, uint32_t u) { return s + (uint64_t)r * (K / 2) + 32 * u; }
   struct Raw {
-    uint4 q;
-    uint32_t ls;
+    uint4 q[2];
+    uint32_t sl, sh;  // the two sub-blocks' low nibbles; their high pairs of bits, at bit 4 (u % 2)
     __half d;
   };
-  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint64_t, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    return s + (uint64_t)r * (K / 2) + k0 / 2 + 16 * h;
-  }
-  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t k0, uint32_t h) {
-    const uint32_t ib = (k0 % 256) / 32 + h;  // the sub-block within its block
-    const uint64_t blk = (uint64_t)r * (K / 256) + k0 / 256;
+  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t u) {
+    const uint64_t blk = (uint64_t)r * (K / 256) + u / 4;
     Raw x;
-    x.q = ldg16(quants_at(s, nblk, K, r, k0, h));
-    const uint32_t sl = __ldg((const uint32_t *)(s + 128 * nblk) + blk), sh = __ldg((const uint16_t *)(s + 132 * nblk) + blk);
-    x.ls = ((sl >> (4 * ib)) & 0xF) | (((sh >> (2 * ib)) & 3) << 4);
+    const uint8_t *q = quants_at(s, K, r, u);
+    x.q[0] = ldg16(q), x.q[1] = ldg16(q + 16);
+    x.sl = __ldg(s + 128 * nblk + 4 * blk + u % 4);
+    x.sh = (uint32_t)__ldg(s + 132 * nblk + 2 * blk + u % 4 / 2) >> (4 * (u % 2));
     x.d = __ldg((const __half *)(s + 134 * nblk) + blk);
     return x;
   }
-  __device__ static __forceinline__ void store(const Hdr &, const Raw &x, uint8_t *tile, uint32_t m, uint32_t h, uint32_t, const uint32_t *) {
+  template <int S>
+  __device__ static __forceinline__ void store(const Raw &x, uint8_t *tile, uint32_t m, const uint32_t *) {
     // d * (ls - 32) rounded to f16 once; ls - 32 is in -32 .. 31, exact in f16.
-    iq4_store32(x.q, __float2half2_rn(__half2float(x.d) * (float)((int)x.ls - 32)), tile, m, h);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const uint32_t ls = ((x.sl >> (4 * h)) & 0xF) | (((x.sh >> (2 * h)) & 3) << 4);
+      iq4_store32(x.q[h], __float2half2_rn(__half2float(x.d) * (float)((int)ls - 32)), tile, m, h);
+    }
   }
 };
 
@@ -679,6 +708,32 @@ struct Decoder<QT_IQ4_XS> {
 // instruction). Q4_K, the benchmark's type: its quants are one run of K / 2 bytes a row, which a 3-D map (bytes of the
 // row, rows, expert slots) covers.
 __host__ __device__ constexpr bool quants_by_copy(uint32_t qt) { return qt == QT_Q4_K; }
+
+// What a decode thread loads of a block beside the quants the ring brings.
+template <int QT, bool = quants_by_copy(QT)>
+struct HeaderOf {
+  using type = typename tc::Decoder<QT>::Hdr;
+};
+template <int QT>
+struct HeaderOf<QT, false> {
+  struct type {};
+};
+
+// The values a stage holds. The stages of an item follow one another through the decode groups, stage it going to group
+// it % groups; where a group's unit is two stages, they are the units of `groups` groups at a time, first stages first, so
+// that a thread finds both stages of a unit in the registers it filled with one round of loads. A row whose units the
+// groups do not divide ends with half a round: as many stages as there are groups, taken in the row's order, one each.
+// No group so goes more than `groups` stages without one of its own: its wait on a stage's empty barrier tells the
+// phases apart only if its last stage lies no further back than the ring is long.
+template <int QT, uint32_t GROUPS>
+struct StageMap {
+  static constexpr uint32_t kUnit = tc::Decoder<QT>::kUnitStages, kRound = GROUPS * kUnit;
+  __device__ static __forceinline__ uint32_t first_value(uint32_t it, uint32_t KT) {
+    if constexpr (kUnit == 1) return it * kTileK;
+    const uint32_t r0 = it / kRound * kRound, i = it - r0;
+    return (KT - r0 >= kRound ? r0 + i % GROUPS * kUnit + i / GROUPS : it) * kTileK;
+  }
+};
 
 // Shared memory of a CTA: the stages (NMAT weight tiles of 16 KB and a row tile of 32 KB each), then (for types whose
 // quants come by copy) a ring of two quant slots, then the barriers, then a codebook type's codebook.
@@ -756,6 +811,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
   // stage's NMAT * 128 rows are one group of threads; the 512 decode threads form 2 groups (two matrices) or 4 (one),
   // and group g takes stages g, g + groups, ...
   constexpr uint32_t kGroupThreads = NMAT * kTileM, kDecGroups = kTileDecoders / kGroupThreads;
+  static_assert(kDecGroups <= S, "a decode group waits on the phase before the last of a stage it may not have seen (StageMap)");
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
 
@@ -927,7 +983,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
     // For types whose quants come by copy, the one thing a decode thread still loads itself is a block's header, and it
     // asks for it a block ahead (across items too), so that no stage begins by waiting for it: hdr_ahead holds the
     // header of the next block the thread will decode.
-    typename Dec::Hdr hdr_ahead;
+    [[maybe_unused]] typename HeaderOf<QT>::type hdr_ahead;
     if constexpr (quants_by_copy(QT)) {
       const uint32_t i0 = item_at(0);
       if (i0 != kNoItem && first < KT) {
@@ -944,20 +1000,28 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
       const uint32_t item_after = quants_by_copy(QT) ? item_at(rnd + 1) : kNoItem;
       ItemTile t_after{0, 0, 0};
       if (item_after != kNoItem) t_after = item_tile(a, item_after / RTU);
-      // Quants come from HBM the first time an expert is touched; a request for the L2 goes out kAhead stages before
-      // the load into registers, which itself goes a stage of this thread's before the decode.
-      constexpr uint32_t kLineStages = 128 / Dec::kStageBytes;
-      constexpr uint32_t kAhead = kLineStages > 6 ? kLineStages : 6 / kLineStages * kLineStages;  // a whole number of lines, about 6 stages
-      Raw raw[2][2];  // [buffer][half]
-      // The block's scales travel with the stage's quants: loaded when a stage is the thread's first in its block, kept
-      // for its later stages there.
-      typename Dec::Hdr hdr[2], hdr_last;
-      uint32_t blk_fetched = 0xFFFFFFFFu;
-      auto fetch = [&](uint32_t b, uint32_t it) {
-        const uint32_t k0 = it * kTileK;
-        if constexpr (quants_by_copy(QT)) {
+      auto stage_begin = [&](uint32_t it, uint32_t &s) {
+        const uint32_t g = li * KT + it, use_s = g / S;
+        s = g % S;
+        if (use_s > 0) ok = mbar_wait(empty_bar(s), (use_s - 1) & 1, abort, a.error);
+        if (ok) tc_fence_after();
+        return ok;
+      };
+      auto stage_end = [&](uint32_t s) {
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) arrive_lead(full_lead(s), full_bar(s));
+      };
+      auto tile_of = [&](uint32_t s) { return smem + s * SM::kStageBytes + mat * SM::kWBytes; };
+      if constexpr (quants_by_copy(QT)) {
+        // This thread's stages: first, first + kDecGroups, ...; the quants wait in shared memory, so nothing is loaded ahead but
+        // a block's scales, kept for the thread's later stages there.
+        uint32_t blk_fetched = 0xFFFFFFFFu;
+        typename Dec::Hdr hdr;
+        for (uint32_t it = first; it < KT && ok; it += kDecGroups) {
+          const uint32_t k0 = it * kTileK;
           // The header asked for a block ago is this block's; the one after it is asked for now.
-          if (it == first || k0 / 256 != blk_fetched) hdr_last = hdr_ahead, blk_fetched = k0 / 256;
+          if (it == first || k0 / 256 != blk_fetched) hdr = hdr_ahead, blk_fetched = k0 / 256;
           const uint32_t it2 = it + kDecGroups;
           if (it2 < KT) {
             if (it2 * kTileK / 256 != blk_fetched) hdr_ahead = Dec::fetch_hdr(wm, nblk, K, r0 + m, (it2 * kTileK) & ~255u);
@@ -965,74 +1029,78 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
             hdr_ahead = Dec::fetch_hdr((mat == 0 ? a.w0 : a.w1) + (uint64_t)t_after.slot * a.slice_bytes, nblk, K,
                                        item_rows0(item_after) + m, (first * kTileK) & ~255u);
           }
-        } else {
-          if (k0 / 256 != blk_fetched) hdr_last = Dec::fetch_hdr(wm, nblk, K, r0 + m, k0 & ~255u), blk_fetched = k0 / 256;
-        }
-        hdr[b] = hdr_last;
-        if constexpr (quants_by_copy(QT)) {
           // The stage's 32 bytes of this row from the quant ring: slot qn holds one stage per group, this group's at
           // bytes 32 * first of the row, its 16-byte pieces swizzled by the row as the copy laid them.
           const uint32_t qn = li * (KT / kDecGroups) + it / kDecGroups, qb = qn % SM::kQSlots;
-          if (!mbar_wait(q_full(qb), (qn / SM::kQSlots) & 1, abort, a.error)) {
-            ok = false;
-            return;
-          }
+          ok = mbar_wait(q_full(qb), (qn / SM::kQSlots) & 1, abort, a.error);
+          if (!ok) break;
           const uint8_t *row = smem + SM::kQuants + qb * SM::kQSlotBytes + mat * SM::kQMatBytes + m * SM::kQRowBytes;
           const uint32_t sw = SM::kQRowBytes == 64 ? (m >> 1) & 3 : m & 7;
-          raw[b][0].q = *(const uint4 *)(row + 16 * ((2 * first) ^ sw));
-          raw[b][1].q = *(const uint4 *)(row + 16 * ((2 * first + 1) ^ sw));
+          Raw raw[2];
+          raw[0].q = *(const uint4 *)(row + 16 * ((2 * first) ^ sw));
+          raw[1].q = *(const uint4 *)(row + 16 * ((2 * first + 1) ^ sw));
           // These reads are the generic proxy's and the copy that refills the slot is the async proxy's: without the
           // fence the copy was seen to overtake them (a few 128-byte lines of a slot read as the next stage's quants,
           // run to run different). The fence orders the reads before whatever the arrival below lets loose.
           fence_async_smem();
           __syncwarp();
           if (lane == 0) mbar_arrive(q_empty(qb));
-        } else {
-          raw[b][0] = Dec::fetch(wm, nblk, K, r0 + m, k0, 0);
-          raw[b][1] = Dec::fetch(wm, nblk, K, r0 + m, k0, 1);
-          // One request a 128-byte line, which holds kLineStages stages of the row.
-          if (it % kLineStages == 0 && k0 + kAhead * kTileK < K) prefetch_l2(Dec::quants_at(wm, nblk, K, r0 + m, k0 + kAhead * kTileK, 0));
-        }
-      };
-      auto stage_step = [&](uint32_t b, uint32_t it) {
-        const uint32_t g = li * KT + it, s = g % S, use_s = g / S, k0 = it * kTileK;
-        if (use_s > 0) ok = mbar_wait(empty_bar(s), (use_s - 1) & 1, abort, a.error);
-        if (!ok) return;
-        tc_fence_after();
-        uint8_t *tile = smem + s * SM::kStageBytes + mat * SM::kWBytes;
-        Dec::store(hdr[b], raw[b][0], tile, m, 0, k0, grid);
-        Dec::store(hdr[b], raw[b][1], tile, m, 1, k0, grid);
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) arrive_lead(full_lead(s), full_bar(s));
-      };
-      // The first lines of a row's quants are asked for an item ahead (below), so that an item does not begin by
-      // waiting for HBM; the CTA's first item asks for its own.
-      auto ask_ahead = [&](const uint8_t *w, uint32_t row) {
-        for (uint32_t p = 0; p < kAhead && p < KT; p += kLineStages) prefetch_l2(Dec::quants_at(w, nblk, K, row, p * kTileK, 0));
-      };
-      if (!quants_by_copy(QT) && first == 0 && li == 0) ask_ahead(wm, r0 + m);
-      const uint32_t item_next = quants_by_copy(QT) ? kNoItem : item_at(rnd + 1);
-      // This thread's stages: first, first + kDecGroups, ...; the quants of one are loaded while the one before decodes.
-      if constexpr (quants_by_copy(QT)) {
-        // The quants wait in shared memory: nothing to load ahead; a stage is read and decoded in one go.
-        for (uint32_t it = first; it < KT && ok; it += kDecGroups) {
-          fetch(0, it);
-          if (ok) stage_step(0, it);
+          uint32_t s;
+          if (!stage_begin(it, s)) break;
+          Dec::store(hdr, raw, tile_of(s), m, k0);
+          stage_end(s);
         }
       } else {
-      if (first < KT) fetch(0, first);
-      for (uint32_t it = first; it < KT && ok; it += 2 * kDecGroups) {
-        if (it + kDecGroups < KT) fetch(1, it + kDecGroups);
-        stage_step(0, it);
-        if (it == 0 && item_next != kNoItem) {  // group 0, after its first stage: the next item's first lines
+        // This thread's units: first, first + kDecGroups, ...; one is loaded while the one before it decodes. In a round cut
+        // short (half of one: StageMap) the thread takes one stage of the unit its stage falls into.
+        constexpr uint32_t U = Dec::kUnitStages;
+        const uint32_t units = KT / U, whole = units / kDecGroups * kDecGroups, last = whole + first / U;
+        Raw raw[2];
+        auto one_stage = [&](auto half, const Raw &x, uint32_t it) {
+          uint32_t s;
+          if (!stage_begin(it, s)) return;
+          Dec::template store<decltype(half)::value>(x, tile_of(s), m, grid);
+          stage_end(s);
+        };
+        auto fetch = [&](Raw &x, uint32_t u) {
+          const uint32_t v = u < whole ? u : last;
+          if (v >= units) return;
+          x = Dec::fetch(wm, nblk, K, r0 + m, v);
+          // The main run's lines come from HBM the first time an expert is touched: one request a 128-byte line for the L2,
+          // a whole number of lines and at least three units of every group's ahead.
+          constexpr uint32_t kLine = 128 / Dec::kUnitBytes, kAhead = (3 * kDecGroups + kLine - 1) / kLine * kLine;
+          if (v % kLine == 0 && v + kAhead < units) prefetch_l2(Dec::quants_at(wm, K, r0 + m, v + kAhead));
+        };
+        auto unit_step = [&](const Raw &x, uint32_t u) {
+          if (u < whole) {
+            one_stage(std::integral_constant<int, 0>{}, x, (u - first) * U + first);
+            if constexpr (U == 2)
+              if (ok) one_stage(std::integral_constant<int, 1>{}, x, (u - first) * U + kDecGroups + first);
+          } else if constexpr (U == 2) {
+            const uint32_t it = whole * U + first;
+            if (it >= KT) return;
+            if (first % 2)
+              one_stage(std::integral_constant<int, 1>{}, x, it);
+            else
+              one_stage(std::integral_constant<int, 0>{}, x, it);
+          }
+        };
+        // The first lines of a row's quants are asked for an item ahead, so that an item does not begin by waiting for HBM.
+        const uint32_t item_next = item_at(rnd + 1);
+        if (first == 0 && item_next != kNoItem) {
           const ItemTile tn = item_tile(a, item_next / RTU);
-          ask_ahead((mat == 0 ? a.w0 : a.w1) + (uint64_t)tn.slot * a.slice_bytes, item_rows0(item_next) + m);
+          const uint8_t *wn = (mat == 0 ? a.w0 : a.w1) + (uint64_t)tn.slot * a.slice_bytes;
+          for (uint32_t u = 0; u < units && u < 3 * kDecGroups; u += 128 / Dec::kUnitBytes) prefetch_l2(Dec::quants_at(wn, K, item_rows0(item_next) + m, u));
         }
-        if (!ok || it + kDecGroups >= KT) break;
-        if (it + 2 * kDecGroups < KT) fetch(0, it + 2 * kDecGroups);
-        stage_step(1, it + kDecGroups);
-      }
+        const uint32_t rounds = (units + kDecGroups - 1) / kDecGroups;
+        fetch(raw[0], first);
+        for (uint32_t j = 0; j < rounds && ok; j += 2) {
+          if (j + 1 < rounds) fetch(raw[1], first + (j + 1) * kDecGroups);
+          unit_step(raw[0], first + j * kDecGroups);
+          if (!ok || j + 1 >= rounds) break;
+          if (j + 2 < rounds) fetch(raw[0], first + (j + 2) * kDecGroups);
+          unit_step(raw[1], first + (j + 1) * kDecGroups);
+        }
       }
       if (is_wide(t.count)) {
         // Both buffers: the next item's MMAs wait for this epilogue, so these warps take four fifths of it.
@@ -1111,15 +1179,15 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
           }
           ok = __shfl_sync(0xffffffffu, ok, 0);
           if (!ok) break;
-          const uint32_t xt = smem_u32(smem + s * SM::kStageBytes) + NMAT * SM::kWBytes;
+          const uint32_t xt = smem_u32(smem + s * SM::kStageBytes) + NMAT * SM::kWBytes, x0 = StageMap<QT, kDecGroups>::first_value(it, KT);
 #pragma unroll
           for (uint32_t c = 0; c < kPerLane; c++) {
             const uint32_t copy = lane + 32 * c;
             if (copy < ncopies) {
               if constexpr (PAIR)
-                tma_gather4_rows_pair(xt + copy * 4 * kTileK * 2, &act_map, it * kTileK, idx[4 * c], idx[4 * c + 1], idx[4 * c + 2], idx[4 * c + 3], bar);
+                tma_gather4_rows_pair(xt + copy * 4 * kTileK * 2, &act_map, x0, idx[4 * c], idx[4 * c + 1], idx[4 * c + 2], idx[4 * c + 3], bar);
               else
-                tma_gather4_rows(xt + copy * 4 * kTileK * 2, &act_map, it * kTileK, idx[4 * c], idx[4 * c + 1], idx[4 * c + 2], idx[4 * c + 3], bar);
+                tma_gather4_rows(xt + copy * 4 * kTileK * 2, &act_map, x0, idx[4 * c], idx[4 * c + 1], idx[4 * c + 2], idx[4 * c + 3], bar);
             }
           }
         }
@@ -1145,15 +1213,15 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
           const uint32_t g = li * KT + it, s = g % S, use_s = g / S;
           if (use_s > 0) ok = mbar_wait(empty_bar(s), (use_s - 1) & 1, abort, a.error);
           if (!ok) break;
-          const uint32_t xt = smem_u32(smem + s * SM::kStageBytes) + NMAT * SM::kWBytes;
+          const uint32_t xt = smem_u32(smem + s * SM::kStageBytes) + NMAT * SM::kWBytes, x0 = StageMap<QT, kDecGroups>::first_value(it, KT);
           if constexpr (PAIR) {
             mbar_arrive_expect_cluster(full_lead(s), nbox * kTileBoxRows * kTileK * 2);
             for (uint32_t i = 0; i < nbox; i++)
-              tma_load_rows_pair(xt + i * kTileBoxRows * kTileK * 2, &act_map, it * kTileK, row0 + i * kTileBoxRows, full_lead(s));
+              tma_load_rows_pair(xt + i * kTileBoxRows * kTileK * 2, &act_map, x0, row0 + i * kTileBoxRows, full_lead(s));
           } else {
             mbar_arrive_expect(full_bar(s), nbox * kTileBoxRows * kTileK * 2);
             for (uint32_t i = 0; i < nbox; i++)
-              tma_load_rows(xt + i * kTileBoxRows * kTileK * 2, &act_map, it * kTileK, row0 + i * kTileBoxRows, full_bar(s));
+              tma_load_rows(xt + i * kTileBoxRows * kTileK * 2, &act_map, x0, row0 + i * kTileBoxRows, full_bar(s));
           }
         }
       }
