@@ -647,10 +647,11 @@ __device__ __forceinline__ void short_pack(const ShortRoute &rt, const uint32_t 
     rt.o.tiles[tile] = MoeTile{e, e, first, n};
     for (uint32_t i = 0; i * rt.group_max < n; i++) rt.o.groups[group + i] = MoeGroup{e, first + i * rt.group_max, min(rt.group_max, n - i * rt.group_max)};
   }
-  if (tid == 0) {
+  if (tid < 32) {
     uint32_t hit = 0, groups = 0, rows = 0;
-    for (uint32_t i = 0; i < A; i++) hit += s_groups[i] != 0, groups += s_groups[i], rows += s_ids[i] < rt.NE;
-    rt.o.counters[0] = hit, rt.o.counters[1] = groups, rt.o.counters[2] = hit, rt.o.counters[3] = rows, rt.o.counters[4] = 0, rt.o.counters[5] = 0;
+    for (uint32_t i = tid; i < A; i += 32) hit += s_groups[i] != 0, groups += s_groups[i], rows += s_ids[i] < rt.NE;
+    hit = __reduce_add_sync(0xffffffffu, hit), groups = __reduce_add_sync(0xffffffffu, groups), rows = __reduce_add_sync(0xffffffffu, rows);
+    if (tid == 0) rt.o.counters[0] = hit, rt.o.counters[1] = groups, rt.o.counters[2] = hit, rt.o.counters[3] = rows, rt.o.counters[4] = 0, rt.o.counters[5] = 0;
   }
 }
 

@@ -500,9 +500,10 @@ uint32_t tensor_budget_for(const moe_layer *l, uint64_t R) {
 void launch_router_rows(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
   const uint32_t E = l->E, NE = l->NE, N = l->N;
   // Rows a CTA takes: the fewer, the more CTAs share the step's multiply-adds and the shorter a lane's chain of them, for
-  // one more reading of the router's 4 MB out of L2 a pass. Up to 16 rows 2 (or the one), above 4, while the passes are
-  // few; 8 in the long steps of a layer kept off the tensor cores, where the readings would be what counts.
-  const uint32_t tm = T == 1 ? 1 : T <= 16 ? 2 : T <= kRouterExactRows ? 4 : 8, warps = T <= 4 ? 1 : tm <= 4 ? 4 : 8;
+  // one more reading of the router's 4 MB out of L2 a pass: 2 rows (13 rows: 35 -> 12.6 us against 8, ncu, cold; 32 rows by
+  // fours, whose registers leave no room for sixteen loads in flight, 27); 8 in the long steps of a layer kept off the
+  // tensor cores, where the readings would be what counts.
+  const uint32_t tm = T == 1 ? 1 : T <= kRouterExactRows ? 2 : 8, warps = T <= 4 ? 1 : tm == 2 ? 4 : 8;
   const size_t smem = (size_t)tm * kRouterPieces * (E / kRouterPieces + 4) * sizeof(float);
   if (!l->rows_attr_set) {
     const size_t row = (size_t)kRouterPieces * (E / kRouterPieces + 4) * sizeof(float);
@@ -510,7 +511,7 @@ void launch_router_rows(moe_layer *l, const float *x, uint32_t T, cudaStream_t s
       if (rows * row > 48 * 1024) CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(rows * row)));
     };
     allow(k_router_logits_rows<1>, 1), allow(k_router_logits_rows<1, 16>, 1), allow(k_router_logits_rows<2>, 2), allow(k_router_logits_rows<2, 16>, 2);
-    allow(k_router_logits_rows<4>, 4), allow(k_router_logits_rows<8>, 8);
+    allow(k_router_logits_rows<8>, 8);
     l->rows_attr_set = true;
   }
   const uint32_t passes = (T + tm - 1) / tm;
@@ -522,7 +523,7 @@ void launch_router_rows(moe_layer *l, const float *x, uint32_t T, cudaStream_t s
   const dim3 grid(sq.ctas + (N + 4 * warps - 1) / (4 * warps), passes);
   const bool deep = (E / kRouterPieces) % 64 == 0;  // sixteen loads in flight a lane: a step of one row is all latency
   auto kernel = tm == 1 ? (deep ? k_router_logits_rows<1, 16> : k_router_logits_rows<1>)
-                        : tm == 2 ? (deep ? k_router_logits_rows<2, 16> : k_router_logits_rows<2>) : tm == 4 ? k_router_logits_rows<4> : k_router_logits_rows<8>;
+                        : tm == 2 ? (deep ? k_router_logits_rows<2, 16> : k_router_logits_rows<2>) : k_router_logits_rows<8>;
   launched(l, launch_kernel(l->ctx.pdl, kernel, grid, dim3(32 * warps), smem, st, x, T, E, l->router.get(), N, l->bias.get(), NE, l->rl.get(), sq),
            "router logits");
 }

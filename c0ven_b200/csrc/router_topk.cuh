@@ -162,26 +162,36 @@ __device__ __forceinline__ void router_topk_row(uint32_t t, const float *__restr
     const char *row = (const char *)(ap.x + (uint64_t)t * ap.E);
     for (uint32_t b = lane * 128; b < ap.E * 4; b += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + b));
   }
+  // All of the lane's logits are asked for before any is used.
+  float f[kMaxPerLane];
+  float *const at = ap.logits + (uint64_t)t * NE + lane;
+#pragma unroll
+  for (int j = 0; j < kMaxPerLane; j++)
+    if ((uint32_t)j < per) f[j] = ap.logits ? at[32 * j] : rl[(uint64_t)t * (NE + 1) + lane + 32 * j];
+  if (ap.logits && ap.parts > 1) {
+    for (uint32_t p = 1; p < ap.parts; p++) {
+      float more[kMaxPerLane];
+#pragma unroll
+      for (int j = 0; j < kMaxPerLane; j++)
+        if ((uint32_t)j < per) more[j] = at[p * ap.part_stride + 32 * j];
+#pragma unroll
+      for (int j = 0; j < kMaxPerLane; j++)
+        if ((uint32_t)j < per) f[j] += more[j];
+    }
+#pragma unroll
+    for (int j = 0; j < kMaxPerLane; j++)
+      if ((uint32_t)j < per) at[32 * j] = f[j];
+  }
 #pragma unroll
   for (int j = 0; j < kMaxPerLane; j++) {
     key[j] = 0;
     if ((uint32_t)j < per) {
-      const uint32_t e = lane + 32 * j;
-      float f;
       if (ap.logits) {
-        float *at = ap.logits + (uint64_t)t * NE + e;
-        f = *at;
-        if (ap.parts > 1) {
-          for (uint32_t p = 1; p < ap.parts; p++) f += at[p * ap.part_stride];
-          *at = f;
-        }
-        if (bias) f = __fadd_rn(f, bias[e]);
-        finite = finite && isfinite(f);
-      } else {
-        f = rl[(uint64_t)t * (NE + 1) + e];
+        if (bias) f[j] = __fadd_rn(f[j], bias[lane + 32 * j]);
+        finite = finite && isfinite(f[j]);
       }
-      key[j] = order_key(f);
-      mx = fmaxf(mx, f);
+      key[j] = order_key(f[j]);
+      mx = fmaxf(mx, f[j]);
     }
   }
   if (ap.logits) {
