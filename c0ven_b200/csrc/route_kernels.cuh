@@ -277,7 +277,7 @@ __host__ __device__ inline bool n_is_tensor(uint32_t n, uint32_t tensor_min) { r
 // thread reading all 512 lengths to find its rank took longer than all the rest).
 __device__ __forceinline__ uint32_t pack_scan_block(uint32_t e, uint32_t run, uint32_t NE, uint32_t first_expert, uint32_t tensor_min,
                                                     uint32_t tensor_budget, uint32_t group_max, const PackOut &o) {
-  constexpr uint32_t kWarps = 16, kSums = 8;
+  constexpr uint32_t kWarps = 16, kSums = 7;
   __shared__ uint32_t s_sum[kSums][kWarps], s_ge[4][kWarps], s_rows_ge[4][kWarps];
   __shared__ uint16_t s_len[kWarps][kTileN];  // short tiles of a length in a warp; then how many of that length come before the warp's
   __shared__ uint32_t s_bin[kTileN / 32];
@@ -333,11 +333,11 @@ __device__ __forceinline__ uint32_t pack_scan_block(uint32_t e, uint32_t run, ui
       if (lane >= off) v[j] += u;
     }
   const uint32_t hit = __popc(__ballot_sync(0xffffffffu, n > 0)), big = __reduce_add_sync(0xffffffffu, nb),
-                 bigrows = __reduce_add_sync(0xffffffffu, tensor ? n : 0), tall = __popc(__ballot_sync(0xffffffffu, len > o.mma_rows));
+                 bigrows = __reduce_add_sync(0xffffffffu, tensor ? n : 0);
   if (in) {
     for (uint32_t i = lane; i < kTileN / 2; i += 32) ((uint32_t *)s_len[warp])[i] = 0;
     if (lane == 31) s_sum[0][warp] = v[0], s_sum[1][warp] = v[1], s_sum[2][warp] = v[2], s_sum[3][warp] = v[3];
-    if (lane == 0) s_sum[4][warp] = hit, s_sum[5][warp] = big, s_sum[6][warp] = bigrows, s_sum[7][warp] = tall;
+    if (lane == 0) s_sum[4][warp] = hit, s_sum[5][warp] = big, s_sum[6][warp] = bigrows;
     __syncwarp();
   }
   const uint32_t same = __match_any_sync(0xffffffffu, len);
@@ -389,7 +389,7 @@ __device__ __forceinline__ uint32_t pack_scan_block(uint32_t e, uint32_t run, ui
   }
   if (e == 511) {
     o.counters[0] = all[1], o.counters[1] = all[2], o.counters[2] = all[4], o.counters[3] = all[0];
-    o.counters[4] = all[5], o.counters[5] = all[6], o.counters[6] = all[3] + all[7];
+    o.counters[4] = all[5], o.counters[5] = all[6];
   }
   return first;
 }
