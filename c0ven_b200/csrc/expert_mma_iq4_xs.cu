@@ -1,0 +1,3 @@
+// k_expert_mma for IQ4_XS weights (expert_mma.cuh).
+#define EXPERT_MMA_QT moe::QT_IQ4_XS
+#include "expert_mma_inst.cuh"

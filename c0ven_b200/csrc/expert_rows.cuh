@@ -48,6 +48,10 @@ struct BigTile {
   uint32_t slot, start, count;
 };
 
+// Which experts with one short tile go to the few-rows kernel: none; those of up to 16 rows, or 32 in a step that hits many
+// experts; all of them if none has more than 8, else none.
+enum FewRows { FEW_NONE, FEW_BY_ROWS, FEW_IF_ALL };
+
 // What a pack leaves: the step's assignments by expert, and the lists the experts' kernels walk.
 struct PackOut {
   uint32_t *cnt, *base;    // NE each
@@ -55,7 +59,9 @@ struct PackOut {
   MoeTile *tiles;          // expert order, <= 64 rows each (prompt.cl:719-723)
   MoeGroup *groups;        // <= group_max rows each: the experts with fewer than tensor_min rows
   BigTile *big;            // <= kTileN rows each: the others, for the tensor-core kernels
-  uint32_t *counters;      // [0] tiles, [1] groups, [2] experts hit, [3] rows, [4] big tiles, [5] their rows
+  uint32_t *counters;      // [0] tiles, [1] groups, [2] experts hit, [3] rows, [4] big tiles, [5] their rows, [6] the first of the
+                           // big tiles that go to the few-rows kernel (expert_mma.cuh): short ones, at the list's end
+  uint32_t few_rows;       // how the scan settles which (FewRows)
 };
 
 // A short step's route: exact logits in; ids, weights, gates and the lists out, those of at most kShortMax assignments by
@@ -651,7 +657,7 @@ __device__ __forceinline__ void short_pack(const ShortRoute &rt, const uint32_t 
     uint32_t hit = 0, groups = 0, rows = 0;
     for (uint32_t i = tid; i < A; i += 32) hit += s_groups[i] != 0, groups += s_groups[i], rows += s_ids[i] < rt.NE;
     hit = __reduce_add_sync(0xffffffffu, hit), groups = __reduce_add_sync(0xffffffffu, groups), rows = __reduce_add_sync(0xffffffffu, rows);
-    if (tid == 0) rt.o.counters[0] = hit, rt.o.counters[1] = groups, rt.o.counters[2] = hit, rt.o.counters[3] = rows, rt.o.counters[4] = 0, rt.o.counters[5] = 0;
+    if (tid == 0) rt.o.counters[0] = hit, rt.o.counters[1] = groups, rt.o.counters[2] = hit, rt.o.counters[3] = rows, rt.o.counters[4] = 0, rt.o.counters[5] = 0, rt.o.counters[6] = 0;
   }
 }
 

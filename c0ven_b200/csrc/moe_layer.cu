@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "cuda_rt.h"
+#include "expert_mma.cuh"
 #include "expert_rows.cuh"
 #include "expert_tiles.cuh"
 #include "formats.h"
@@ -67,6 +68,28 @@ static cudaError_t launch_down_combine_type(uint32_t qt, const DownCombineArgs &
     case QT_Q2_0: return launch_down_combine<QT_Q2_0>(a, grid, ctx, st);
     default: return cudaErrorInvalidValue;
   }
+}
+
+template <int QT, int NMAT>
+cudaError_t launch_expert_mma(const ExpertMmaArgs &a, uint32_t most_rows, uint32_t max_entries, const LaunchCtx &ctx, cudaStream_t st);
+
+static cudaError_t launch_mma(uint32_t qt, int nmat, const ExpertMmaArgs &a, uint32_t most_rows, uint32_t max_entries, const LaunchCtx &ctx, cudaStream_t st) {
+#define MMA_CASE(T)                                                                                     \
+  case T:                                                                                               \
+    return nmat == 2 ? launch_expert_mma<T, 2>(a, most_rows, max_entries, ctx, st) : launch_expert_mma<T, 1>(a, most_rows, max_entries, ctx, st);
+  switch (qt) {
+    MMA_CASE(QT_Q8_0)
+    MMA_CASE(QT_Q4_K)
+    MMA_CASE(QT_Q6_K)
+    MMA_CASE(QT_IQ4_NL)
+    MMA_CASE(QT_IQ4_XS)
+    MMA_CASE(QT_IQ3_S)
+    MMA_CASE(QT_IQ3_XXS)
+    MMA_CASE(QT_IQ2_S)
+    MMA_CASE(QT_Q2_0)
+    default: return cudaErrorInvalidValue;
+  }
+#undef MMA_CASE
 }
 
 static cudaError_t launch_tiles(uint32_t qt, int nmat, const ExpertTilesArgs &a, const CUtensorMap &map, uint32_t max_tiles, const uint32_t *grid,
@@ -142,7 +165,9 @@ struct PackBuffers {
     // As long as any grid over it: the integer-dot kernel reads its entry before it knows the list's length.
     groups.alloc(max_rows + n);
   }
-  PackOut out() const { return PackOut{cnt.get(), base.get(), chunk_off.get(), tiles.get(), groups.get(), big.get(), counters.get()}; }
+  PackOut out(uint32_t few = FEW_NONE) const {
+    return PackOut{cnt.get(), base.get(), chunk_off.get(), tiles.get(), groups.get(), big.get(), counters.get(), few};
+  }
 };
 
 enum Stage { ST_QUANT, ST_ROUTER, ST_PACK, ST_GATE_UP, ST_DOWN, ST_SHARED, ST_COMBINE, ST_COPIES };
@@ -236,7 +261,7 @@ void launched(moe_layer *l, cudaError_t e, const char *what) {
 // out. Steps of more than two groups of chunks take the scan in two levels.
 struct PackJob {
   const int32_t *ids;
-  uint32_t entries, chunk_len, nchunks, first_expert, tensor_min, tensor_budget, group_max, src_div;
+  uint32_t entries, chunk_len, nchunks, first_expert, tensor_min, tensor_budget, group_max, src_div, few_rows;
 };
 void launch_pack(moe_layer *l, PackBuffers &pk, const PackJob &j, cudaStream_t st) {
   const uint32_t ngroups = (j.nchunks + kScanGroup - 1) / kScanGroup;
@@ -245,7 +270,7 @@ void launch_pack(moe_layer *l, PackBuffers &pk, const PackJob &j, cudaStream_t s
     k_pack_scan_groups<<<ngroups, 512, 0, st>>>(pk.chunk_hist.get(), j.nchunks, pk.nexp, pk.chunk_off.get(), groups);
     launched(l, cudaGetLastError(), "pack scan of the groups");
   }
-  k_pack_scan<<<1, 512, 0, st>>>(pk.chunk_hist.get(), j.nchunks, pk.nexp, j.first_expert, j.tensor_min, j.tensor_budget, j.group_max, pk.out(), groups,
+  k_pack_scan<<<1, 512, 0, st>>>(pk.chunk_hist.get(), j.nchunks, pk.nexp, j.first_expert, j.tensor_min, j.tensor_budget, j.group_max, pk.out(j.few_rows), groups,
                                  ngroups);
   launched(l, cudaGetLastError(), "pack scan");
   if (j.chunk_len > 512 || pk.nexp > 512) throw std::logic_error("pack fill: a chunk of at most 512 entries, at most 512 experts");
@@ -456,14 +481,16 @@ void setup_router_tensor(moe_layer *l, const float *router, const float *bias, c
   CUDA_OK(cudaStreamSynchronize(st));
 }
 
+// other: the other form of the rows (q8_0 and q8_K), made by the same kernel.
 // gate: with the rows' product with this vector wanted too (the shared expert's gate logit), its parts go to gate_parts.
 void quantize_rows(moe_layer *l, const float *src, uint64_t rows, uint32_t Kv, const ActBuffers &dst, cudaStream_t st,
-                   const float *gate = nullptr, float *gate_parts = nullptr, RouterSplit rs = RouterSplit{}) {
+                   const float *gate = nullptr, float *gate_parts = nullptr, RouterSplit rs = RouterSplit{}, const ActBuffers *other = nullptr) {
   const uint64_t nblk = rows * (Kv / 256);
   if (nblk == 0) return;
   const unsigned grid = (unsigned)((nblk + 7) / 8);
-  launched(l, launch_kernel(l->ctx.pdl, dst.q8k ? k_quant<true> : k_quant<false>, dim3(grid), dim3(256), 0, st, src, nblk, dst.job(), gate, Kv / 256,
-                            gate_parts, rs),
+  auto kernel = other ? (dst.q8k ? k_quant<true, true> : k_quant<false, true>) : dst.q8k ? k_quant<true, false> : k_quant<false, false>;
+  launched(l, launch_kernel(l->ctx.pdl, kernel, dim3(grid), dim3(256), 0, st, src, nblk, dst.job(), gate, Kv / 256, gate_parts, rs,
+                            other ? other->job() : QuantJob{}),
            "quantize");
 }
 
@@ -494,6 +521,30 @@ uint32_t tensor_min_for(const moe_layer *l, uint64_t R) {
 // as in steps of a few rows, where two more launches would cost more than they could save.
 uint32_t tensor_budget_for(const moe_layer *l, uint64_t R) {
   return l->can_tensor && !l->cfg.tensor_min_rows && R >= 64 && R < 1280 ? l->sms / 2 : 0;
+}
+
+// Whether experts with few rows go to the few-rows kernel (expert_mma.cuh) rather than the tile kernels, in a call of R
+// expert rows over nexp experts, and by which rule (FewRows). With more than 24 rows an expert on average, too few of them
+// have 32 or less to pay for two more launches (2,000 rows of the benchmark's layer, 39 an expert: 850 -> 899 us in
+// IQ4_XS; 4,000 rows, skewed, over 64 experts: 237 -> 268).
+uint32_t few_rows_for(const moe_layer *l, uint64_t R, uint32_t nexp) {
+  const uint32_t tm = tensor_min_for(l, R);
+  if (!tm || l->cfg.tensor_min_rows || R < 64 || R > 24ull * nexp) return FEW_NONE;
+  if (!mma_takes(l->cfg.gate_type, l->E, kMmaRows) || !mma_takes(l->cfg.down_type, l->F, kMmaRows)) return FEW_NONE;
+  if (tm == 1) return FEW_BY_ROWS;
+  // Below that the list holds all of the step only if it hits 74 experts at most (tensor_budget_for): with this many more
+  // experts to hit and no skew it is empty, and the two launches cost for nothing (32 rows of Q8_0: 246 -> 256 us).
+  return std::min<uint64_t>(R, nexp) <= 128 ? FEW_IF_ALL : FEW_NONE;
+}
+
+// Whether groups of at most M rows go to the few-rows kernel: with more than two rows its eight columns are worth their
+// instructions whatever the type (200 rows of IQ3_S: 1085 -> 491 us); with one or two, where the integer-dot kernel's
+// decode is long and runs once a row (32 rows, even routing: Q4_K 309 -> 215 us, Q4_K with Q6_K 326 -> 251, IQ4_XS with
+// IQ4_NL 315 -> 276), not where it is nothing or a codebook's (Q8_0 246 -> 256, IQ3_S 272 -> 305, IQ2_S 281 -> 293).
+bool groups_take_mma(const moe_layer *l, int M) {
+  const uint32_t g = l->cfg.gate_type, d = l->cfg.down_type;
+  auto heavy = [](uint32_t t) { return t == QT_Q4_K || t == QT_Q6_K || t == QT_IQ4_XS || t == QT_IQ4_NL; };
+  return (M > 2 || (M == 2 && heavy(g) && heavy(d))) && mma_takes(g, l->E, kGroupMax) && mma_takes(d, l->F, kGroupMax);
 }
 
 // The exact fp32 router product of a step's rows, its x quantised by the same launch.
@@ -538,8 +589,7 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
   mark(l, ST_QUANT, st);
   if (approx)
     quantize_rows(l, x, T, E, l->xq_routed, st, l->router.get() + (size_t)NE * E, l->gate_parts.get(),
-                  RouterSplit{l->rx_hi.get(), l->rx_lo.get(), l->norm2_parts.get()});
-  if (approx && l->has_shared && !l->shared_x_same) quantize_rows(l, x, T, E, l->xq_shared, st);
+                  RouterSplit{l->rx_hi.get(), l->rx_lo.get(), l->norm2_parts.get()}, l->has_shared && !l->shared_x_same ? &l->xq_shared : nullptr);
   mark(l, ST_ROUTER, st);
   uint32_t router_parts = 1;
   if (!approx) {
@@ -568,7 +618,8 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
   if (nchunks == 1 && NE <= 512) {
     // One chunk: top-k, scan and fill in one CTA (the pack stage then has no kernel of its own).
     launched(l, launch_kernel(l->ctx.pdl, k_router_topk_pack, dim3(1), dim3(32 * kChunkTokens), chunk_len * sizeof(int32_t), st, l->rl.get(), l->bias.get(),
-                              T, NE, K, l->ids.get(), l->w.get(), l->gs.get(), tm, budget, group_cap(A, NE), l->pack.out(), l->pack.inv.get(),
+                              T, NE, K, l->ids.get(), l->w.get(), l->gs.get(), tm, budget, group_cap(A, NE),
+                              l->pack.out(l->local == NE ? few_rows_for(l, A, NE) : FEW_NONE), l->pack.inv.get(),
                               l->pack.row_src.get()),
              "router top-k and pack");
     mark(l, ST_PACK, st);
@@ -587,7 +638,7 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
       launched(l, cudaGetLastError(), "router top-k");
     }
     mark(l, ST_PACK, st);
-    launch_pack(l, l->pack, PackJob{l->ids.get(), (uint32_t)A, chunk_len, nchunks, 0, tm, budget, group_cap(A, NE), K}, st);
+    launch_pack(l, l->pack, PackJob{l->ids.get(), (uint32_t)A, chunk_len, nchunks, 0, tm, budget, group_cap(A, NE), K, l->local == NE ? few_rows_for(l, A, NE) : FEW_NONE}, st);
   }
   l->last_T = T, l->last_pack = &l->pack;
 }
@@ -616,7 +667,7 @@ void stage_experts(moe_layer *l, const ActSource &src, const PackBuffers &pk, ui
       tm ? (tm > 1 ? (uint32_t)std::min<uint64_t>(R, (uint64_t)nexp * ((tm - 2) / gmax + 1)) : 0) : (uint32_t)std::min<uint64_t>(R, R / gmax + nexp);
   // The pack may have lowered the threshold to 1 (tensor_budget_for): the tile launches are sized for that.
   const uint32_t tm_low = tm && tensor_budget_for(l, R) ? 1 : tm;
-  const uint32_t max_big = tm_low && R >= tm_low ? (uint32_t)(R / kTileN + std::min<uint64_t>(nexp, R / tm_low)) : 0;
+  const uint32_t max_big = tm_low && R >= tm_low && most >= tm_low ? (uint32_t)(R / kTileN + std::min<uint64_t>(nexp, R / tm_low)) : 0;
   // With MOE_FLAG_GATHER_IN_KERNEL, long steps of a GPU's own rows: the gate/up tile kernel gathers the rows by index
   // itself (cp.async.bulk.tensor's tile::gather4 form, 32 copies of four rows a stage for a pair's CTA instead of two
   // boxes of 64) and no copy to expert order runs. The copies then set that kernel's pace (1.39 -> 1.85 ms at 32,768
@@ -624,14 +675,18 @@ void stage_experts(moe_layer *l, const ActSource &src, const PackBuffers &pk, ui
   // (The same gather by the copy warp's own 16-byte asynchronous copies, cp.async, was slower still: 2.26 ms.)
   const bool gather_in_kernel = (l->cfg.flags & MOE_FLAG_GATHER_IN_KERNEL) && max_big && R >= kGatherInKernelRows &&
                                 src.h == l->xq_routed.h.get() && src.act_row != nullptr;
+  // The experts of a few rows: the short tiles at the list's end, or groups of up to eight rows.
+  static_assert(sizeof(BigTile) == sizeof(MoeGroup), "both lists are (slot, start, rows)");
+  const bool few = max_big && few_rows_for(l, R, nexp) != FEW_NONE, groups_mma = max_groups && groups_take_mma(l, M);
   if (max_big) {
     // The rows in expert order first (the reference's p_moe_scatter, kernels/models/qwen4exp/prompt.cl:744-754): a tile's
     // rows are then one box after another for the kernel's copies. Part of the pack stage: the gate/up stage times the
     // product's own kernels.
     if (!gather_in_kernel && !in_order) {
       if (!rows_in) throw std::logic_error("rows neither in expert order nor with their places laid out");
-      k_scatter_f16<<<rows_in, 256, 0, st>>>(src.h, pk.inv.get(), (uint32_t)(R / rows_in), E, l->xg.get());
-      launched(l, cudaGetLastError(), "rows to expert order");
+      launched(l, launch_kernel(l->ctx.pdl, k_scatter_f16, dim3(rows_in), dim3(256), 0, st, src.h, pk.inv.get(), (uint32_t)(R / rows_in), E, l->xg.get(),
+                                pk.counters.get() + 6),
+               "rows to expert order");
     }
   }
   mark(l, ST_GATE_UP, st);
@@ -639,7 +694,7 @@ void stage_experts(moe_layer *l, const ActSource &src, const PackBuffers &pk, ui
     ExpertTilesArgs a{};
     a.w0 = l->wg.get(), a.w1 = l->wu.get(), a.slice_bytes = l->gate_slice, a.K = E, a.R = F;
     a.qmap[0] = l->wg_q, a.qmap[1] = l->wu_q;
-    a.tiles = pk.big.get(), a.ntiles = pk.counters.get() + 4;
+    a.tiles = pk.big.get(), a.ntiles = pk.counters.get() + 6;
     a.out = l->h.get(), a.out_stride = F, a.limit = c.swiglu_limit, a.error = l->error.get();
     if (gather_in_kernel) {
       a.gather_rows = src.act_row;
@@ -648,7 +703,21 @@ void stage_experts(moe_layer *l, const ActSource &src, const PackBuffers &pk, ui
       launched(l, launch_tiles(c.gate_type, 2, a, l->xg_map, max_big, l->grid.get(), l->ctx, st), "experts gate/up tiles");
     }
   }
-  if (max_groups) {
+  auto mma_lists = [&](ExpertMmaArgs m, uint32_t type, int nmat, const char *what) {
+    if (few) m.entries = (const MoeGroup *)pk.big.get(), m.first = pk.counters.get() + 6, m.end = pk.counters.get() + 4;
+    if (groups_mma) m.entries2 = pk.groups.get(), m.end2 = pk.counters.get() + 1;
+    m.grid = l->grid.get();
+    launched(l, launch_mma(type, nmat, m, few ? kMmaRows : kGroupMax, (few ? (uint32_t)std::min<uint64_t>(nexp, R) : 0) + (groups_mma ? max_groups : 0), l->ctx, st),
+             what);
+  };
+  if (few || groups_mma) {
+    ExpertMmaArgs m{};
+    m.w0 = l->wg.get(), m.w1 = l->wu.get(), m.slice_bytes = l->gate_slice, m.K = E, m.R = F;
+    m.act = src.view, m.act_row = src.act_row;
+    m.out = l->h.get(), m.out_stride = F, m.limit = c.swiglu_limit;
+    mma_lists(m, c.gate_type, 2, "experts gate/up, few rows");
+  }
+  if (max_groups && !groups_mma) {
     ExpertRowsArgs a{};
     a.w0 = l->wg.get(), a.w1 = l->wu.get(), a.slice_bytes = l->gate_slice, a.K = E, a.R = F, a.rows_per_cta = 32;
     a.act = src.view, a.act_row = src.act_row;
@@ -662,11 +731,18 @@ void stage_experts(moe_layer *l, const ActSource &src, const PackBuffers &pk, ui
     ExpertTilesArgs a{};
     a.w0 = l->wd.get(), a.slice_bytes = l->down_slice, a.K = F, a.R = E;
     a.qmap[0] = l->wd_q;
-    a.tiles = pk.big.get(), a.ntiles = pk.counters.get() + 4;
+    a.tiles = pk.big.get(), a.ntiles = pk.counters.get() + 6;
     a.out = y, a.out_stride = E, a.out_f16 = y16, a.error = l->error.get();
     launched(l, launch_tiles(c.down_type, 1, a, l->hq_routed.h_map, max_big, l->grid.get(), l->ctx, st), "experts down tiles");
   }
-  if (max_groups) {
+  if (few || groups_mma) {
+    ExpertMmaArgs m{};
+    m.w0 = l->wd.get(), m.slice_bytes = l->down_slice, m.K = F, m.R = E;
+    m.act = l->hq_routed.view(), m.act_row = nullptr;
+    m.out = y, m.out_stride = E, m.out_f16 = y16;
+    mma_lists(m, c.down_type, 1, "experts down, few rows");
+  }
+  if (max_groups && !groups_mma) {
     ExpertRowsArgs a{};
     a.w0 = l->wd.get(), a.slice_bytes = l->down_slice, a.K = F, a.R = E, a.rows_per_cta = 128;
     a.act = l->hq_routed.view(), a.act_row = nullptr;
@@ -1103,7 +1179,8 @@ MOE_API moe_status moe_layer_experts_device(moe_layer *l, const void *rows_dev, 
     const uint32_t nchunks = (R + kLocalChunk - 1) / kLocalChunk;
     k_chunk_hist<<<nchunks, 256, 0, st>>>(ids_dev, R, kLocalChunk, nexp, l->cfg.expert_first, pk.chunk_hist.get());
     launched(l, cudaGetLastError(), "local counts");
-    launch_pack(l, pk, PackJob{ids_dev, R, kLocalChunk, nchunks, l->cfg.expert_first, tm, tensor_budget_for(l, R), group_cap(R, nexp), 1}, st);
+    launch_pack(l, pk, PackJob{ids_dev, R, kLocalChunk, nchunks, l->cfg.expert_first, tm, tensor_budget_for(l, R), group_cap(R, nexp), 1,
+                               few_rows_for(l, R, nexp)}, st);
     const uint8_t *wire = (const uint8_t *)rows_dev;
     const uint32_t dbytes = q8k ? E / 64 : E / 8;
     ActSource src{ActView{(const int8_t *)wire, (const float *)(wire + E), (const int16_t *)(wire + E + dbytes), wb, wb, wb}, nullptr,
@@ -1198,7 +1275,7 @@ MOE_API moe_status moe_layer_experts_partial_device(moe_layer *l, const void *ro
     k_chunk_hist<<<nchunks, 256, 0, st>>>(l->ids_local.get(), (uint32_t)entries, kLocalChunk, nexp, l->cfg.expert_first, pk.chunk_hist.get());
     launched(l, cudaGetLastError(), "local counts");
     launch_pack(l, pk, PackJob{l->ids_local.get(), (uint32_t)entries, kLocalChunk, nchunks, l->cfg.expert_first, tm, tensor_budget_for(l, A),
-                               group_cap(A, nexp), K}, st);
+                               group_cap(A, nexp), K, few_rows_for(l, A, nexp)}, st);
     const uint32_t dbytes = q8k ? E / 64 : E / 8;
     ActSource src{ActView{(const int8_t *)wire, (const float *)(wire + E), (const int16_t *)(wire + E + dbytes), wb2, wb2, wb2}, nullptr,
                   pk.row_src.get()};

@@ -61,9 +61,10 @@ __device__ __forceinline__ void router_split(const float4 &a, const float4 &b, u
   if (lane == 0) rs.norm2_parts[blk] = s;
 }
 
-template <bool Q8K>
+// BOTH: the rows in the other form too (job2): one reading of them for the two.
+template <bool Q8K, bool BOTH>
 static __global__ void __launch_bounds__(256) k_quant(const float *__restrict__ x, uint64_t nblk256, const QuantJob job, const float *__restrict__ gate,
-                                              uint32_t per_row, float *__restrict__ gate_parts, RouterSplit rs) {
+                                              uint32_t per_row, float *__restrict__ gate_parts, RouterSplit rs, const QuantJob job2) {
   dependents_may_launch(), wait_for_predecessors();
   const uint64_t blk = (uint64_t)blockIdx.x * 8 + threadIdx.x / 32;
   if (blk >= nblk256) return;
@@ -72,6 +73,7 @@ static __global__ void __launch_bounds__(256) k_quant(const float *__restrict__ 
   if (gate) gate_part(a, b, gate, per_row, blk, lane, gate_parts);
   if (rs.hi) router_split(a, b, blk, lane, rs);
   quantize_store<Q8K>(a, b, blk, lane, job);
+  if constexpr (BOTH) quantize_store<!Q8K>(a, b, blk, lane, job2);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -246,7 +248,9 @@ static __global__ void __launch_bounds__(128) k_received_ids(const uint32_t *__r
 // src[row_src[r]], reads a row once per place, in expert order, long after its last use left the L2: at 32,768 rows
 // of 2,048 values and ten places a row it read 1.0 GB from DRAM for the 134 MB of rows there are, and took twice as long.)
 static __global__ void __launch_bounds__(256) k_scatter_f16(const __half *__restrict__ src, const uint32_t *__restrict__ place_of, uint32_t per_row,
-                                                    uint32_t K, __half *__restrict__ dst) {
+                                                    uint32_t K, __half *__restrict__ dst, const uint32_t *__restrict__ ntiles) {
+  dependents_may_launch(), wait_for_predecessors();
+  if (*ntiles == 0) return;  // a short step none of whose experts goes to the tile kernels
   const uint64_t t = blockIdx.x;
   const uint32_t *places = place_of + t * per_row;
   for (uint32_t c = threadIdx.x; c < K / 8; c += 256) {
@@ -277,7 +281,7 @@ __host__ __device__ inline bool n_is_tensor(uint32_t n, uint32_t tensor_min) { r
 // thread reading all 512 lengths to find its rank took longer than all the rest).
 __device__ __forceinline__ uint32_t pack_scan_block(uint32_t e, uint32_t run, uint32_t NE, uint32_t first_expert, uint32_t tensor_min,
                                                     uint32_t tensor_budget, uint32_t group_max, const PackOut &o) {
-  constexpr uint32_t kWarps = 16, kSums = 7;
+  constexpr uint32_t kWarps = 16, kSums = 8;
   __shared__ uint32_t s_sum[kSums][kWarps], s_ge[4][kWarps], s_rows_ge[4][kWarps];
   __shared__ uint16_t s_len[kWarps][kTileN];  // short tiles of a length in a warp; then how many of that length come before the warp's
   __shared__ uint32_t s_bin[kTileN / 32];
@@ -312,6 +316,18 @@ __device__ __forceinline__ uint32_t pack_scan_block(uint32_t e, uint32_t run, ui
     }
   }
   const bool tensor = n_is_tensor(run, tensor_min);
+  // Rows up to which an expert with one short tile goes to the few-rows kernel. That kernel takes 16 weight rows a warp
+  // for as long as the row is, and longer with every eight activation rows, so it needs many warps: a step that hits 80
+  // experts (256 rows, skewed) was slower with experts of 32 rows there (243 us) than of 16 (231), one that hits 512
+  // (777 rows) faster (463 against 564). In a step that few experts share (FEW_IF_ALL: below 1,280 assignments) it wins
+  // where all have a few rows (13 rows over 73 experts in IQ2_S: 239 -> 187 us) and loses beside the tile kernels, which
+  // take a long expert in the time of a short one (64 rows, skewed: 217 -> 258).
+  uint32_t few = 0;
+  if (o.few_rows == FEW_BY_ROWS) {
+    few = __syncthreads_count(run > 0) < 256 ? 16 : 32;
+  } else if (o.few_rows == FEW_IF_ALL) {
+    few = __syncthreads_or(tensor && run > 8) ? 0 : 8;
+  }
   const uint32_t n = run, nt = (n + kTileRows - 1) / kTileRows, ng = tensor ? 0 : (n + group_max - 1) / group_max;
   const uint32_t nb = tensor ? (n + kTileN - 1) / kTileN : 0;
   // Big tiles, in the order the tile kernels deal them to their CTAs round by round. First the experts that have at
@@ -333,11 +349,11 @@ __device__ __forceinline__ uint32_t pack_scan_block(uint32_t e, uint32_t run, ui
       if (lane >= off) v[j] += u;
     }
   const uint32_t hit = __popc(__ballot_sync(0xffffffffu, n > 0)), big = __reduce_add_sync(0xffffffffu, nb),
-                 bigrows = __reduce_add_sync(0xffffffffu, tensor ? n : 0);
+                 bigrows = __reduce_add_sync(0xffffffffu, tensor ? n : 0), tall = __popc(__ballot_sync(0xffffffffu, len > few));
   if (in) {
     for (uint32_t i = lane; i < kTileN / 2; i += 32) ((uint32_t *)s_len[warp])[i] = 0;
     if (lane == 31) s_sum[0][warp] = v[0], s_sum[1][warp] = v[1], s_sum[2][warp] = v[2], s_sum[3][warp] = v[3];
-    if (lane == 0) s_sum[4][warp] = hit, s_sum[5][warp] = big, s_sum[6][warp] = bigrows;
+    if (lane == 0) s_sum[4][warp] = hit, s_sum[5][warp] = big, s_sum[6][warp] = bigrows, s_sum[7][warp] = tall;
     __syncwarp();
   }
   const uint32_t same = __match_any_sync(0xffffffffu, len);
@@ -389,7 +405,7 @@ __device__ __forceinline__ uint32_t pack_scan_block(uint32_t e, uint32_t run, ui
   }
   if (e == 511) {
     o.counters[0] = all[1], o.counters[1] = all[2], o.counters[2] = all[4], o.counters[3] = all[0];
-    o.counters[4] = all[5], o.counters[5] = all[6];
+    o.counters[4] = all[5], o.counters[5] = all[6], o.counters[6] = all[3] + all[7];
   }
   return first;
 }

@@ -1,0 +1,47 @@
+"""On a B200: the int8 tensor-instruction kernel for experts of a few rows, against the CPU oracle: as groups (a layer kept
+off the tile kernels, whose arithmetic it shares bit by bit but for f32 order) and as the short end of the tile list, with
+experts of more rows on the tile kernels in the same step; at the shortest rows, at lengths nothing is specialised for
+and at the longest a CTA holds."""
+import numpy as np
+import pytest
+
+from c0ven_b200 import MoELayer, synth
+from test_gpu_parity import INT_PATH_REL, TYPES, check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("n_embd,n_ff", [(256, 256), (768, 1280), (2048, 512), (4352, 256)])
+def test_groups(t, n_embd, n_ff):
+    layer = synth.make_layer(n_embd=n_embd, n_ff=n_ff, n_experts=64, n_used=4, gate_type=t, seed=t + n_embd)
+    gpu = MoELayer(layer, max_tokens=200, no_tensor=True)
+    for T in (9, 16, 17, 65, 200):  # groups of up to two; with more rows than experts, of up to eight
+        check(layer, gpu, synth.make_input(T, n_embd, seed=T), INT_PATH_REL)
+    gpu.close()
+
+
+@pytest.mark.parametrize("gate,down", [(t, t) for t in TYPES] + [(synth.Q4_K, synth.Q6_K), (synth.IQ4_XS, synth.IQ4_NL)])
+def test_short_tiles_beside_long_ones(gate, down):
+    """Rows that repeat route alike: experts that only one of the rows chose get its repeats, up to and past the 8 rows of
+    one instruction and the 32 of an entry."""
+    layer = synth.make_layer(n_embd=768, n_ff=512, n_experts=320, n_used=4, gate_type=gate, down_type=down, seed=gate * 50 + down)
+    repeats = [1, 7, 8, 9, 16, 17, 24, 25, 32, 33, 300, 2, 32]
+    x = np.repeat(synth.make_input(len(repeats), 768, seed=3), repeats, axis=0)
+    gpu = MoELayer(layer, max_tokens=len(x))
+    check(layer, gpu, x)
+    cnt = np.bincount(gpu.route(len(x))[0].reshape(-1), minlength=320)
+    assert {1, 7, 8, 9, 16, 17, 24, 25, 32, 33, 300} <= set(cnt.tolist())
+    gpu.close()
+
+
+@pytest.mark.parametrize("t", TYPES)
+def test_both_lists_in_one_launch(t):
+    """Steps of 64 to 1,279 assignments: all experts on the tile list (few experts), on the groups' list, or on both (an
+    expert that many rows chose beside others of one or two), with and without one that needs the tile kernels."""
+    layer = synth.make_layer(n_embd=512, n_ff=256, n_experts=320, n_used=4, gate_type=t, seed=t)
+    gpu = MoELayer(layer, max_tokens=300)
+    base = synth.make_input(300, 512, seed=t)
+    for T, repeats in ((16, 1), (17, 4), (32, 1), (33, 1), (200, 1), (120, 20), (200, 40)):
+        check(layer, gpu, np.concatenate([np.repeat(base[:1], repeats, axis=0), base[1:T - repeats + 1]]))
+    gpu.close()
