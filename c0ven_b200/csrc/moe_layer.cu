@@ -267,16 +267,16 @@ void launch_pack(moe_layer *l, PackBuffers &pk, const PackJob &j, cudaStream_t s
   const uint32_t ngroups = (j.nchunks + kScanGroup - 1) / kScanGroup;
   uint32_t *groups = ngroups > 2 ? pk.group_off.get() : nullptr;
   if (groups) {
-    k_pack_scan_groups<<<ngroups, 512, 0, st>>>(pk.chunk_hist.get(), j.nchunks, pk.nexp, pk.chunk_off.get(), groups);
-    launched(l, cudaGetLastError(), "pack scan of the groups");
+    launched(l, launch_kernel(l->ctx.pdl, k_pack_scan_groups, dim3(ngroups), dim3(512), 0, st, pk.chunk_hist.get(), j.nchunks, pk.nexp, pk.chunk_off.get(), groups),
+             "pack scan of the groups");
   }
-  k_pack_scan<<<1, 512, 0, st>>>(pk.chunk_hist.get(), j.nchunks, pk.nexp, j.first_expert, j.tensor_min, j.tensor_budget, j.group_max, pk.out(j.few_rows), groups,
-                                 ngroups);
-  launched(l, cudaGetLastError(), "pack scan");
+  launched(l, launch_kernel(l->ctx.pdl, k_pack_scan, dim3(1), dim3(512), 0, st, pk.chunk_hist.get(), j.nchunks, pk.nexp, j.first_expert, j.tensor_min,
+                            j.tensor_budget, j.group_max, pk.out(j.few_rows), groups, ngroups),
+           "pack scan");
   if (j.chunk_len > 512 || pk.nexp > 512) throw std::logic_error("pack fill: a chunk of at most 512 entries, at most 512 experts");
-  k_pack_fill<<<j.nchunks, 512, 16 * pk.nexp * sizeof(uint32_t), st>>>(j.ids, j.entries, j.chunk_len, pk.nexp, pk.base.get(), pk.chunk_off.get(), j.src_div,
-                                                                 pk.inv.get(), pk.row_src.get(), j.first_expert, groups);
-  launched(l, cudaGetLastError(), "pack fill");
+  launched(l, launch_kernel(l->ctx.pdl, k_pack_fill, dim3(j.nchunks), dim3(512), 16 * pk.nexp * sizeof(uint32_t), st, j.ids, j.entries, j.chunk_len, pk.nexp,
+                            pk.base.get(), pk.chunk_off.get(), j.src_div, pk.inv.get(), pk.row_src.get(), j.first_expert, groups),
+           "pack fill");
 }
 
 void mark(moe_layer *l, int stage, cudaStream_t st) {
@@ -607,8 +607,9 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
     router_parts = 4 * tiles <= l->sms ? 4 : 2 * tiles <= l->sms ? 2 : 1;
     const RouterMmaArgs ra{T, E, NE, ne_tile, l->rw_unscale.get(), router_parts, l->approx.get(), l->error.get()};
     const uint32_t items = tiles * router_parts;
-    k_router_mma<<<std::min(items, l->sms), kRouterThreads, kRouterSmemBytes, st>>>(ra, l->rx_hi_map, l->rx_lo_map, l->rw_hi_map, l->rw_lo_map);
-    launched(l, cudaGetLastError(), "router logits");
+    launched(l, launch_kernel(l->ctx.pdl, k_router_mma, dim3(std::min(items, l->sms)), dim3(kRouterThreads), kRouterSmemBytes, st, ra, l->rx_hi_map,
+                              l->rx_lo_map, l->rw_hi_map, l->rw_lo_map),
+             "router logits");
   }
   const uint32_t nchunks = (T + kChunkTokens - 1) / kChunkTokens;
   // On one GPU the pack also lists the groups and big tiles of the experts' kernels; expert parallel, it only sorts.
@@ -627,11 +628,11 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
     if (approx) {
       const RouterApprox ap{l->approx.get(), x, l->router.get(), l->norm2_parts.get(), l->gate_parts.get(), E, E / 256, router_parts, (uint64_t)T * NE,
                             l->router_eps_rel, l->router_eps_abs};
-      k_router_topk_rows<<<(T + kTopkRowsPerCta - 1) / kTopkRowsPerCta, 32 * kTopkRowsPerCta, 0, st>>>(ap, l->bias.get(), T, NE, K, l->ids.get(),
-                                                                                                  l->w.get(), l->gs.get());
-      launched(l, cudaGetLastError(), "router top-k");
-      k_chunk_hist<<<nchunks, 256, 0, st>>>(l->ids.get(), (uint32_t)A, chunk_len, NE, 0, l->pack.chunk_hist.get());
-      launched(l, cudaGetLastError(), "chunk counts");
+      launched(l, launch_kernel(l->ctx.pdl, k_router_topk_rows, dim3((T + kTopkRowsPerCta - 1) / kTopkRowsPerCta), dim3(32 * kTopkRowsPerCta), 0, st, ap,
+                                l->bias.get(), T, NE, K, l->ids.get(), l->w.get(), l->gs.get()),
+               "router top-k");
+      launched(l, launch_kernel(l->ctx.pdl, k_chunk_hist, dim3(nchunks), dim3(256), 0, st, l->ids.get(), (uint32_t)A, chunk_len, NE, 0, l->pack.chunk_hist.get()),
+               "chunk counts");
     } else {
       k_router_topk<<<nchunks, 32 * kChunkTokens, 0, st>>>(l->rl.get(), RouterApprox{}, l->bias.get(), T, NE, K, l->ids.get(), l->w.get(),
                                                           l->gs.get(), l->pack.chunk_hist.get());
@@ -861,15 +862,15 @@ void forward_short(moe_layer *l, const float *x, uint32_t T, float *out, cudaStr
 }
 
 constexpr uint32_t kGraphMaxRows = 64;
+constexpr uint32_t kPdlMaxRows = 4096;  // longer steps' kernels run for longer than a launch takes
 constexpr uint64_t kSharedInlineRows = 65536;  // expert rows from which the shared expert runs after the routed ones, not beside them
 
 // The whole block on device buffers, queued on st: a GPU that holds every expert.
 void forward_device(moe_layer *l, const float *x, uint32_t T, float *out, cudaStream_t st) {
   if (l->local != l->NE) throw BadArgument("this call needs every expert on the GPU; an expert-parallel layer goes stage by stage");
   const uint64_t A = (uint64_t)T * l->K;
-  // Launch-bound steps (the ones that are also replayed from a graph): each kernel a programmatic dependent of the one
-  // before it in its stream.
-  l->ctx.pdl = T <= kGraphMaxRows && !l->profile && l->pdl_ok;
+  // Steps whose short kernels' launches count: each a programmatic dependent of the one before it in its stream.
+  l->ctx.pdl = T <= kPdlMaxRows && !l->profile && l->pdl_ok;
   struct PdlOff {
     LaunchCtx &c;
     ~PdlOff() { c.pdl = false; }

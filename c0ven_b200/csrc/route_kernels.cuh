@@ -193,6 +193,7 @@ static __global__ void __launch_bounds__(32 * kTopkRowsPerCta) k_router_topk_row
                                                                                  uint32_t NE, uint32_t K, int32_t *__restrict__ ids,
                                                                                  float *__restrict__ w, float *__restrict__ gs) {
   __shared__ __align__(16) uint8_t ex_smem[kTopkRowsPerCta * kExWarpBytes];
+  dependents_may_launch(), wait_for_predecessors();
   router_topk_block(nullptr, ap, bias, T, NE, K, ids, w, gs, nullptr, nullptr, ap.E % (kRouterPieces * kExChunk) == 0 ? ex_smem : nullptr);
 }
 
@@ -211,6 +212,7 @@ static __global__ void __launch_bounds__(32 * kChunkTokens) k_router_topk(const 
 static __global__ void __launch_bounds__(256) k_chunk_hist(const int32_t *__restrict__ ids, uint32_t A, uint32_t chunk_len,
                                                    uint32_t NE, uint32_t first_expert, uint32_t *__restrict__ chunk_hist) {
   __shared__ uint32_t hist[512];
+  dependents_may_launch(), wait_for_predecessors();
   for (uint32_t i = threadIdx.x; i < NE; i += blockDim.x) hist[i] = 0;
   __syncthreads();
   const uint32_t a0 = blockIdx.x * chunk_len, a1 = min(A, a0 + chunk_len);
@@ -417,6 +419,7 @@ __device__ __forceinline__ uint32_t pack_scan_block(uint32_t e, uint32_t run, ui
 constexpr uint32_t kScanGroup = 32;
 static __global__ void __launch_bounds__(512) k_pack_scan_groups(const uint32_t *__restrict__ chunk_hist, uint32_t nchunks, uint32_t NE,
                                                          uint32_t *__restrict__ chunk_off, uint32_t *__restrict__ group_tot) {
+  dependents_may_launch(), wait_for_predecessors();
   const uint32_t e = threadIdx.x, c_begin = blockIdx.x * kScanGroup, c_end = min(nchunks, c_begin + kScanGroup);
   if (e >= NE) return;
   uint32_t run = 0;
@@ -437,6 +440,7 @@ static __global__ void __launch_bounds__(512) k_pack_scan_groups(const uint32_t 
 static __global__ void __launch_bounds__(512) k_pack_scan(const uint32_t *__restrict__ chunk_hist, uint32_t nchunks, uint32_t NE,
                                                   uint32_t first_expert, uint32_t tensor_min, uint32_t tensor_budget, uint32_t group_max,
                                                   PackOut o, uint32_t *__restrict__ groups = nullptr, uint32_t ngroups = 0) {
+  dependents_may_launch(), wait_for_predecessors();
   const uint32_t e = threadIdx.x;
   uint32_t run = 0;
   if (e < NE && groups) {
@@ -474,6 +478,7 @@ static __global__ void __launch_bounds__(512) k_pack_fill(const int32_t *__restr
                                                   const uint32_t *__restrict__ base, const uint32_t *__restrict__ chunk_off,
                                                   uint32_t src_div, uint32_t *__restrict__ inv, uint32_t *__restrict__ row_src,
                                                   uint32_t first_expert = 0, const uint32_t *__restrict__ group_off = nullptr) {
+  dependents_may_launch(), wait_for_predecessors();
   // A thread an entry (chunk_len <= 512). An entry's row is its expert's first row for this chunk plus the number of
   // the chunk's earlier entries with the same expert: those of earlier warps, counted per (warp, expert) in shared
   // memory and summed over the warps, and those of lower lanes of its own warp, which match_any names. (A thread an

@@ -40,6 +40,7 @@ static __global__ void __launch_bounds__(kRouterThreads, 1)
     k_router_mma(const RouterMmaArgs a, const __grid_constant__ CUtensorMap x_hi, const __grid_constant__ CUtensorMap x_lo,
                  const __grid_constant__ CUtensorMap w_hi, const __grid_constant__ CUtensorMap w_lo) {
   using namespace tc;
+  dependents_may_launch(), wait_for_predecessors();
   constexpr uint32_t S = kRouterStages, kCols = 512;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
