@@ -579,8 +579,9 @@ void launch_router_rows(moe_layer *l, const float *x, uint32_t T, cudaStream_t s
            "router logits");
 }
 
-// Quantise x, the router's logits and top-k, and the pack of the step's T * K assignments over every expert.
-void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
+// Quantise x, the router's logits and top-k, and the pack of the step's T * K assignments over every expert. fork: an
+// event recorded once x is quantised, null for none.
+void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st, Event *fork = nullptr) {
   const uint32_t E = l->E, NE = l->NE, K = l->K;
   const uint64_t A = (uint64_t)T * K;
   // Steps of up to kRouterExactRows rows (and every step of a layer kept off the tensor cores) take the exact fp32
@@ -590,10 +591,12 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
   if (approx)
     quantize_rows(l, x, T, E, l->xq_routed, st, l->router.get() + (size_t)NE * E, l->gate_parts.get(),
                   RouterSplit{l->rx_hi.get(), l->rx_lo.get(), l->norm2_parts.get()}, l->has_shared && !l->shared_x_same ? &l->xq_shared : nullptr);
+  if (approx && fork) fork->record(st);
   mark(l, ST_ROUTER, st);
   uint32_t router_parts = 1;
   if (!approx) {
     launch_router_rows(l, x, T, st);
+    if (fork) fork->record(st);
   } else {
     if (!l->router_attr_set) {
       CUDA_OK(cudaFuncSetAttribute(k_router_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRouterSmemBytes));
@@ -884,9 +887,10 @@ void forward_device(moe_layer *l, const float *x, uint32_t T, float *out, cudaSt
   const bool beside = l->has_shared && !l->profile && A < kSharedInlineRows;
   // (The quantiser of a short step, whose exact router reads x itself, was tried on the second stream as well, ahead of
   // the shared expert: 5 us slower at one row, 2 % faster on a stack of 48 layers of 32 rows; not kept.)
-  stage_route(l, x, T, st);
+  // It is forked off as soon as x is quantised, beside the router and the pack, which leave most SMs idle: queued after
+  // them, its tile kernels, a CTA of which takes an SM's whole shared memory, meet the routed experts' CTAs everywhere.
+  stage_route(l, x, T, st, beside ? l->fork_ev.get() : nullptr);
   if (beside) {
-    l->fork_ev->record(st);
     CUDA_OK(cudaStreamWaitEvent(l->aux->get(), l->fork_ev->get(), 0));
     stage_shared(l, T, l->aux->get());
     l->join_ev->record(l->aux->get());
