@@ -44,6 +44,11 @@ struct LaunchCtx {
 // (it then waits where this one waits), the second waits until the kernels before have completed and their writes are
 // visible. Both do nothing in a kernel launched the ordinary way. They stand at a kernel's top, before it reads or
 // writes anything another kernel touches.
+//
+// What an earlier kernel of the chain wrote (rows, codes, ids, lists, counters) is read by plain loads after the wait, never
+// through the read-only path: such a load (__ldg, ld.global.nc, or a kernel's const __restrict__ parameter, which the
+// compiler may turn into one) is defined only for data that nothing writes while the kernel lives, and a dependent's life
+// begins before its predecessors' writes. __ldg and const __restrict__ are for weights, codebooks and biases.
 __device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -553,7 +553,7 @@ __device__ __forceinline__ void mma_entry(const ExpertMmaArgs &a, const MoeGroup
   for (uint32_t i = tid; i < n * (K / 16); i += 256) {
     const uint32_t t = i / (K / 16), c = i % (K / 16);
     const uint64_t row = a.act_row ? a.act_row[start + t] : start + t;
-    *(int4 *)(smem + t * stride + 16 * c) = __ldg((const int4 *)(a.act.q + row * a.act.q_stride) + c);
+    *(int4 *)(smem + t * stride + 16 * c) = ((const int4 *)(a.act.q + row * a.act.q_stride))[c];
   }
   for (uint32_t i = tid; i < n * per_row; i += 256) {
     const uint32_t t = i / per_row, c = i % per_row;
@@ -617,7 +617,7 @@ template <int QT, int NMAT, int MOST>
 __global__ void __launch_bounds__(256, mma_ahead(QT) || MOST > 1 ? 2 : 3) k_expert_mma(const ExpertMmaArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   dependents_may_launch(), wait_for_predecessors();
-  const uint32_t first = a.end ? __ldg(a.first) : 0, n1 = a.end ? __ldg(a.end) - first : 0, n2 = a.end2 ? __ldg(a.end2) : 0;
+  const uint32_t first = a.end ? *a.first : 0, n1 = a.end ? *a.end - first : 0, n2 = a.end2 ? *a.end2 : 0;
   for (uint32_t i = blockIdx.y; i < n1 + n2; i += gridDim.y) {
     const MoeGroup en = i < n1 ? a.entries[first + i] : a.entries2[i - n1];
     if (i != blockIdx.y) __syncthreads();  // the entry before has been read out of shared memory

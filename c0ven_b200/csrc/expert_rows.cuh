@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(256) k_expert_rows(const ExpertRowsArgs a, con
   } else if (a.groups) {
     // Both loads go out together: the list is as long as the grid, so the entry can be read before the count says
     // whether it is one (a CTA's life is a chain of dependent loads; this takes one link out).
-    const uint32_t ng = __ldg(a.ngroups);
+    const uint32_t ng = *a.ngroups;
     const MoeGroup g = a.groups[blockIdx.y];
     if (blockIdx.y >= ng) return;
     if (blockIdx.z * M >= g.n) return;

@@ -63,7 +63,7 @@ __device__ __forceinline__ void router_split(const float4 &a, const float4 &b, u
 
 // BOTH: the rows in the other form too (job2): one reading of them for the two.
 template <bool Q8K, bool BOTH>
-static __global__ void __launch_bounds__(256) k_quant(const float *__restrict__ x, uint64_t nblk256, const QuantJob job, const float *__restrict__ gate,
+static __global__ void __launch_bounds__(256) k_quant(const float *x, uint64_t nblk256, const QuantJob job, const float *__restrict__ gate,
                                               uint32_t per_row, float *__restrict__ gate_parts, RouterSplit rs, const QuantJob job2) {
   dependents_may_launch(), wait_for_predecessors();
   const uint64_t blk = (uint64_t)blockIdx.x * 8 + threadIdx.x / 32;
@@ -93,7 +93,7 @@ struct StepQuant {
   uint32_t ctas;    // in the grid's first extent; 0: x is quantised elsewhere
 };
 template <int TM, int D = 8>
-static __global__ void __launch_bounds__(256) k_router_logits_rows(const float *__restrict__ x, uint32_t T, uint32_t E,
+static __global__ void __launch_bounds__(256) k_router_logits_rows(const float *x, uint32_t T, uint32_t E,
                                                           const float *__restrict__ W, uint32_t N,
                                                           const float *__restrict__ bias, uint32_t NE,
                                                           float *__restrict__ rl, const StepQuant sq) {
@@ -172,7 +172,7 @@ static __global__ void __launch_bounds__(256) k_router_logits_rows(const float *
 // 512 words) and, when s_ids is not null, the chunk's ids there too (shared, kChunkTokens * K words). hist null: the
 // caller counts the chunks' experts itself (k_chunk_hist), and the block may be of any number of warps. ex_smem:
 // kExWarpBytes of shared memory for every warp of the block, or null.
-__device__ __forceinline__ void router_topk_block(const float *__restrict__ rl, const RouterApprox ap, const float *__restrict__ bias,
+__device__ __forceinline__ void router_topk_block(const float *rl, const RouterApprox ap, const float *__restrict__ bias,
                                                   uint32_t T, uint32_t NE, uint32_t K, int32_t *__restrict__ ids, float *__restrict__ w,
                                                   float *__restrict__ gs, uint32_t *hist, int32_t *s_ids, uint8_t *ex_smem = nullptr) {
   if (hist) {
@@ -209,7 +209,7 @@ static __global__ void __launch_bounds__(32 * kChunkTokens) k_router_topk(const 
 
 // The same counts for expert ids that come from elsewhere (the rows another GPU sent): chunk c holds entries
 // [c * chunk_len, (c + 1) * chunk_len) of ids.
-static __global__ void __launch_bounds__(256) k_chunk_hist(const int32_t *__restrict__ ids, uint32_t A, uint32_t chunk_len,
+static __global__ void __launch_bounds__(256) k_chunk_hist(const int32_t *ids, uint32_t A, uint32_t chunk_len,
                                                    uint32_t NE, uint32_t first_expert, uint32_t *__restrict__ chunk_hist) {
   __shared__ uint32_t hist[512];
   dependents_may_launch(), wait_for_predecessors();
@@ -249,15 +249,17 @@ static __global__ void __launch_bounds__(128) k_received_ids(const uint32_t *__r
 // thread reads 16 bytes of it once and writes them per_row times. (The same copy taken from the places' side, dst[r] =
 // src[row_src[r]], reads a row once per place, in expert order, long after its last use left the L2: at 32,768 rows
 // of 2,048 values and ten places a row it read 1.0 GB from DRAM for the 134 MB of rows there are, and took twice as long.)
-static __global__ void __launch_bounds__(256) k_scatter_f16(const __half *__restrict__ src, const uint32_t *__restrict__ place_of, uint32_t per_row,
-                                                    uint32_t K, __half *__restrict__ dst, const uint32_t *__restrict__ ntiles) {
+static __global__ void __launch_bounds__(256) k_scatter_f16(const __half *src, const uint32_t *place_of, uint32_t per_row,
+                                                    uint32_t K, __half *__restrict__ dst, const uint32_t *ntiles) {
   dependents_may_launch(), wait_for_predecessors();
   if (*ntiles == 0) return;  // a short step none of whose experts goes to the tile kernels
   const uint64_t t = blockIdx.x;
-  const uint32_t *places = place_of + t * per_row;
+  __shared__ uint32_t places[16];  // n_used at most
+  if (threadIdx.x < per_row) places[threadIdx.x] = place_of[t * per_row + threadIdx.x];
+  __syncthreads();
   for (uint32_t c = threadIdx.x; c < K / 8; c += 256) {
-    const uint4 v = __ldg((const uint4 *)(src + t * K) + c);
-    for (uint32_t k = 0; k < per_row; k++) ((uint4 *)(dst + (uint64_t)__ldg(places + k) * K))[c] = v;
+    const uint4 v = ((const uint4 *)(src + t * K))[c];
+    for (uint32_t k = 0; k < per_row; k++) ((uint4 *)(dst + (uint64_t)places[k] * K))[c] = v;
   }
 }
 
@@ -417,7 +419,7 @@ __device__ __forceinline__ uint32_t pack_scan_block(uint32_t e, uint32_t run, ui
 // of the chunks, and k_pack_fill adds a chunk's group's offset to the chunk's own. (One CTA walking a thousand chunks
 // took 133 us of a 32,768-row step.)
 constexpr uint32_t kScanGroup = 32;
-static __global__ void __launch_bounds__(512) k_pack_scan_groups(const uint32_t *__restrict__ chunk_hist, uint32_t nchunks, uint32_t NE,
+static __global__ void __launch_bounds__(512) k_pack_scan_groups(const uint32_t *chunk_hist, uint32_t nchunks, uint32_t NE,
                                                          uint32_t *__restrict__ chunk_off, uint32_t *__restrict__ group_tot) {
   dependents_may_launch(), wait_for_predecessors();
   const uint32_t e = threadIdx.x, c_begin = blockIdx.x * kScanGroup, c_end = min(nchunks, c_begin + kScanGroup);
@@ -437,7 +439,7 @@ static __global__ void __launch_bounds__(512) k_pack_scan_groups(const uint32_t 
 }
 
 // groups: null, or the groups' totals left by k_pack_scan_groups, [ngroups][NE], which become the groups' offsets in place.
-static __global__ void __launch_bounds__(512) k_pack_scan(const uint32_t *__restrict__ chunk_hist, uint32_t nchunks, uint32_t NE,
+static __global__ void __launch_bounds__(512) k_pack_scan(const uint32_t *chunk_hist, uint32_t nchunks, uint32_t NE,
                                                   uint32_t first_expert, uint32_t tensor_min, uint32_t tensor_budget, uint32_t group_max,
                                                   PackOut o, uint32_t *__restrict__ groups = nullptr, uint32_t ngroups = 0) {
   dependents_may_launch(), wait_for_predecessors();
@@ -474,10 +476,10 @@ static __global__ void __launch_bounds__(512) k_pack_scan(const uint32_t *__rest
 // One CTA per chunk: the chunk's entries take their expert's rows in the order they stand in.
 // inv[a] = row; row_src[row] = a / src_div (the activation row the assignment reads: its token). Dynamic shared
 // memory 16 * NE words.
-static __global__ void __launch_bounds__(512) k_pack_fill(const int32_t *__restrict__ ids, uint32_t A, uint32_t chunk_len, uint32_t NE,
-                                                  const uint32_t *__restrict__ base, const uint32_t *__restrict__ chunk_off,
+static __global__ void __launch_bounds__(512) k_pack_fill(const int32_t *ids, uint32_t A, uint32_t chunk_len, uint32_t NE,
+                                                  const uint32_t *base, const uint32_t *chunk_off,
                                                   uint32_t src_div, uint32_t *__restrict__ inv, uint32_t *__restrict__ row_src,
-                                                  uint32_t first_expert = 0, const uint32_t *__restrict__ group_off = nullptr) {
+                                                  uint32_t first_expert = 0, const uint32_t *group_off = nullptr) {
   dependents_may_launch(), wait_for_predecessors();
   // A thread an entry (chunk_len <= 512). An entry's row is its expert's first row for this chunk plus the number of
   // the chunk's earlier entries with the same expert: those of earlier warps, counted per (warp, expert) in shared
@@ -513,7 +515,7 @@ static __global__ void __launch_bounds__(512) k_pack_fill(const int32_t *__restr
 
 // A step of one chunk (at most kChunkTokens rows): top-k, scan and fill in one CTA, three launches less for the steps
 // that launches bound. Dynamic shared memory kChunkTokens * K words for the chunk's ids.
-static __global__ void __launch_bounds__(32 * kChunkTokens, 1) k_router_topk_pack(const float *__restrict__ rl, const float *__restrict__ bias, uint32_t T,
+static __global__ void __launch_bounds__(32 * kChunkTokens, 1) k_router_topk_pack(const float *rl, const float *__restrict__ bias, uint32_t T,
                                                                        uint32_t NE, uint32_t K, int32_t *__restrict__ ids, float *__restrict__ w,
                                                                        float *__restrict__ gs, uint32_t tensor_min, uint32_t tensor_budget,
                                                                        uint32_t group_max, PackOut o, uint32_t *__restrict__ inv,
@@ -554,10 +556,8 @@ __device__ __forceinline__ float4 load_row4(const __half *y, uint64_t row, uint3
   return make_float4(a.x, a.y, b.x, b.y);
 }
 template <class Y>
-static __global__ void __launch_bounds__(256) k_combine(const Y *__restrict__ y, const uint32_t *__restrict__ inv,
-                                                       const float *__restrict__ w, const float *__restrict__ gs,
-                                                       const float *__restrict__ s, uint32_t K, uint32_t E, float *__restrict__ out,
-                                                       const float *__restrict__ res) {
+static __global__ void __launch_bounds__(256) k_combine(const Y *y, const uint32_t *inv, const float *w, const float *gs, const float *s, uint32_t K,
+                                                       uint32_t E, float *out, const float *res) {
   dependents_may_launch(), wait_for_predecessors();
   const uint32_t t = blockIdx.x;
   __shared__ uint32_t rows[16];

@@ -45,7 +45,7 @@ struct RouterApprox {
 // The logits of up to four experts for row x, each exactly as k_router_logits_rows and the CPU oracle sum it: eight
 // pieces of the row, each a chain of fused multiply-adds from 0 in index order, the pieces added in order, the bias
 // last. Lane 8 j + s takes piece s of expert ex[j]; lanes 8 j .. 8 j + 7 return expert ex[j]'s logit.
-__device__ __forceinline__ float exact_logits4(const float *__restrict__ x, const float *__restrict__ W, const float *__restrict__ bias,
+__device__ __forceinline__ float exact_logits4(const float *x, const float *__restrict__ W, const float *__restrict__ bias,
                                                uint32_t E, uint32_t e, uint32_t lane) {
   const uint32_t piece = E / kRouterPieces, s = lane % 8;
   const float4 *xp = (const float4 *)(x + s * piece), *wp = (const float4 *)(W + (uint64_t)e * E + s * piece);
@@ -55,7 +55,7 @@ __device__ __forceinline__ float exact_logits4(const float *__restrict__ x, cons
   for (uint32_t i = 0; i < piece / 4; i += 8) {
     float4 xv[8], wv[8];
 #pragma unroll
-    for (int j = 0; j < 8; j++) xv[j] = __ldg(xp + i + j), wv[j] = __ldg(wp + i + j);
+    for (int j = 0; j < 8; j++) xv[j] = xp[i + j], wv[j] = __ldg(wp + i + j);
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       p = fmaf(xv[j].x, wv[j].x, p);
@@ -85,7 +85,7 @@ constexpr uint32_t kExWarpBytes = 2 * kExBuf;            // two chunks: 11,520 b
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
 }
-__device__ __forceinline__ float exact_logits4_staged(const float *__restrict__ x, const float *__restrict__ W, const float *__restrict__ bias,
+__device__ __forceinline__ float exact_logits4_staged(const float *x, const float *__restrict__ W, const float *__restrict__ bias,
                                                       uint32_t E, uint32_t e, uint32_t lane, uint8_t *buf) {
   const uint32_t piece = E / kRouterPieces, nch = piece / kExChunk, s = lane % 8, g = lane / 8;
   const uint32_t buf32 = (uint32_t)__cvta_generic_to_shared(buf);
@@ -147,7 +147,7 @@ __device__ __forceinline__ float exact_logits4_staged(const float *__restrict__ 
 // with exact logits where they were needed, and the first K are the row's experts, in rank order. A row with more
 // than 32 candidates (all logits equal, as for a row of zeros) or a logit that is not finite (an x beyond f16's range)
 // has every logit recomputed exactly instead.
-__device__ __forceinline__ void router_topk_row(uint32_t t, const float *__restrict__ rl, const RouterApprox &ap, const float *__restrict__ bias,
+__device__ __forceinline__ void router_topk_row(uint32_t t, const float *rl, const RouterApprox &ap, const float *__restrict__ bias,
                                                 uint32_t NE, uint32_t K, int32_t *__restrict__ ids, float *__restrict__ w,
                                                 float *__restrict__ gs, uint32_t *hist, int32_t *s_ids, uint8_t *ex_buf) {
   auto exact4 = [&](const float *xr, uint32_t e, uint32_t ln) {
