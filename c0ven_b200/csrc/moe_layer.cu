@@ -231,7 +231,7 @@ struct moe_layer {
   DeviceBuffer<float> w_local;
   uint32_t dest_world = 0;
   ActBuffers xq_routed, xq_shared, hq_routed, hq_shared;
-  bool shared_x_same = true, rows_attr_set = false, shared_on_tensor = false;
+  bool shared_x_same = true, shared_on_tensor = false;
   bool pdl_ok = true;  // off when C0VEN_NO_PDL is set in the environment at create
   uint32_t last_T = 0, last_tensor_min = 0;
   const float *residual = nullptr;  // of the call being queued: rows the combine adds last (moe_layer_forward_residual_device)
@@ -308,6 +308,7 @@ void check_config(const moe_layer_config &c, const moe_layer_weights &w) {
     bad("a shared expert needs its gate vector and three matrices");
 }
 
+uint32_t router_rows_cta(uint32_t T, uint32_t E);
 void setup_router_tensor(moe_layer *l, const float *router, const float *bias, cudaStream_t st);
 
 void create(moe_layer *l, const moe_layer_config &c, const moe_layer_weights &w) {
@@ -348,6 +349,9 @@ void create(moe_layer *l, const moe_layer_config &c, const moe_layer_weights &w)
     const uint64_t dense = l->has_shared && (!l->can_tensor || tm > T) ? ((uint64_t)T + 7) / 8 : 0;
     if (routed > 65535 || dense > 65535)
       throw BadArgument("max_tokens (or max_expert_rows) is too large for the integer-dot kernels' grid: lower it, or leave the tensor-core kernels on");
+    // The exact router's passes over a step's rows are its grid's second extent.
+    if (!l->can_tensor && (T + router_rows_cta(T, E) - 1) / router_rows_cta(T, E) > 65535)
+      throw BadArgument("max_tokens is too large for the exact router's grid: lower it, or leave the tensor-core kernels on");
   }
 
   // The router's rows, then the shared expert's gate vector as row NE (zeros without one).
@@ -547,24 +551,33 @@ bool groups_take_mma(const moe_layer *l, int M) {
   return (M > 2 || (M == 2 && heavy(g) && heavy(d))) && mma_takes(g, l->E, kGroupMax) && mma_takes(d, l->F, kGroupMax);
 }
 
+// Shared memory of the exact router's CTA: tm rows of x, each in padded pieces.
+size_t router_rows_smem(uint32_t tm, uint32_t E) { return (size_t)tm * kRouterPieces * (E / kRouterPieces + 4) * sizeof(float); }
+constexpr size_t kRouterRowsMaxSmem = 227 * 1024;  // what a CTA can have
+
+// Rows of x a CTA of the exact router takes. The fewer, the more CTAs share the step's multiply-adds and the shorter a lane's
+// chain of them, for one more reading of the router's 4 MB out of L2 a pass: 2 rows (13 rows: 35 -> 12.6 us against 8, ncu,
+// cold; 32 rows by fours, whose registers leave no room for sixteen loads in flight, 27); 8 in the long steps of a layer
+// kept off the tensor cores, where the readings would be what counts, as long as 8 rows fit a CTA (7,232 values a row).
+uint32_t router_rows_cta(uint32_t T, uint32_t E) { return T == 1 ? 1 : T <= kRouterExactRows || router_rows_smem(8, E) > kRouterRowsMaxSmem ? 2 : 8; }
+
+template <int TM, int D>
+cudaError_t launch_router_form(moe_layer *l, const float *x, uint32_t T, dim3 grid, uint32_t threads, const StepQuant &sq, cudaStream_t st) {
+  const size_t smem = router_rows_smem(TM, l->E);
+  if (smem > 48 * 1024) {
+    // Set once per device, to the most that any layer's rows take: layers of several sizes share the kernel.
+    static std::atomic<uint32_t> attr_done{0};
+    const cudaError_t e = ensure_dynamic_smem(k_router_logits_rows<TM, D>, std::min(kRouterRowsMaxSmem, router_rows_smem(TM, kRowsMaxK)), attr_done, l->cfg.device);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_kernel(l->ctx.pdl, k_router_logits_rows<TM, D>, grid, dim3(threads), smem, st, x, T, l->E, l->router.get(), l->N, l->bias.get(), l->NE,
+                       l->rl.get(), sq);
+}
+
 // The exact fp32 router product of a step's rows, its x quantised by the same launch.
 void launch_router_rows(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
-  const uint32_t E = l->E, NE = l->NE, N = l->N;
-  // Rows a CTA takes: the fewer, the more CTAs share the step's multiply-adds and the shorter a lane's chain of them, for
-  // one more reading of the router's 4 MB out of L2 a pass: 2 rows (13 rows: 35 -> 12.6 us against 8, ncu, cold; 32 rows by
-  // fours, whose registers leave no room for sixteen loads in flight, 27); 8 in the long steps of a layer kept off the
-  // tensor cores, where the readings would be what counts.
-  const uint32_t tm = T == 1 ? 1 : T <= kRouterExactRows ? 2 : 8, warps = T <= 4 ? 1 : tm == 2 ? 4 : 8;
-  const size_t smem = (size_t)tm * kRouterPieces * (E / kRouterPieces + 4) * sizeof(float);
-  if (!l->rows_attr_set) {
-    const size_t row = (size_t)kRouterPieces * (E / kRouterPieces + 4) * sizeof(float);
-    auto allow = [&](auto kernel, size_t rows) {
-      if (rows * row > 48 * 1024) CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(rows * row)));
-    };
-    allow(k_router_logits_rows<1>, 1), allow(k_router_logits_rows<1, 16>, 1), allow(k_router_logits_rows<2>, 2), allow(k_router_logits_rows<2, 16>, 2);
-    allow(k_router_logits_rows<8>, 8);
-    l->rows_attr_set = true;
-  }
+  const uint32_t E = l->E, N = l->N;
+  const uint32_t tm = router_rows_cta(T, E), warps = T <= 4 ? 1 : tm == 2 ? 4 : 8;
   const uint32_t passes = (T + tm - 1) / tm;
   StepQuant sq{};
   sq.job[0] = l->xq_routed.job();
@@ -573,10 +586,9 @@ void launch_router_rows(moe_layer *l, const float *x, uint32_t T, cudaStream_t s
   sq.ctas = (uint32_t)((sq.nblk + (uint64_t)warps * passes - 1) / (warps * passes));
   const dim3 grid(sq.ctas + (N + 4 * warps - 1) / (4 * warps), passes);
   const bool deep = (E / kRouterPieces) % 64 == 0;  // sixteen loads in flight a lane: a step of one row is all latency
-  auto kernel = tm == 1 ? (deep ? k_router_logits_rows<1, 16> : k_router_logits_rows<1>)
-                        : tm == 2 ? (deep ? k_router_logits_rows<2, 16> : k_router_logits_rows<2>) : k_router_logits_rows<8>;
-  launched(l, launch_kernel(l->ctx.pdl, kernel, grid, dim3(32 * warps), smem, st, x, T, E, l->router.get(), N, l->bias.get(), NE, l->rl.get(), sq),
-           "router logits");
+  auto launch = tm == 1 ? (deep ? launch_router_form<1, 16> : launch_router_form<1, 8>)
+                        : tm == 2 ? (deep ? launch_router_form<2, 16> : launch_router_form<2, 8>) : launch_router_form<8, 8>;
+  launched(l, launch(l, x, T, grid, 32 * warps, sq, st), "router logits");
 }
 
 // Quantise x, the router's logits and top-k, and the pack of the step's T * K assignments over every expert. fork: an

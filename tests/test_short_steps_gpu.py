@@ -69,3 +69,25 @@ def test_without_a_shared_expert_and_equal_logits():
     assert np.all(gpu.forward(x) == 0)
     assert np.array_equal(gpu.route(2)[0], O.moe_forward(layer, x)[1])
     gpu.close()
+
+
+@pytest.mark.parametrize("n_embd,no_tensor", [(8192, False), (8192, True), (16384, False), (16384, True)])
+def test_rows_too_long_for_eight_of_them_in_a_router_cta(n_embd, no_tensor):
+    """Eight rows of more than 7,232 values pass a CTA's shared memory: steps of one or two rows a CTA run all the same, and
+    the long steps of a layer kept off the tensor cores take two."""
+    layer = synth.make_layer(n_embd=n_embd, n_ff=256, n_experts=32, n_used=2, gate_type=synth.Q4_K, down_type=synth.Q8_0, seed=n_embd)
+    gpu = MoELayer(layer, max_tokens=70, no_tensor=no_tensor)
+    for T in (1, 2, 9, 64, 70):
+        check(layer, gpu, synth.make_input(T, n_embd, seed=T))
+    gpu.close()
+
+
+def test_layers_of_several_row_lengths_in_turn():
+    """The router's kernels are shared by the process's layers: a layer of shorter rows leaves those of longer ones running."""
+    layers = [synth.make_layer(n_embd=n, n_ff=256, n_experts=32, n_used=2, gate_type=synth.Q8_0, seed=n) for n in (7168, 2048, 512)]
+    gpus = [MoELayer(layer, max_tokens=70, no_tensor=True) for layer in layers]
+    for T in (70, 2):
+        for layer, gpu in list(zip(layers, gpus)) + [(layers[0], gpus[0])]:
+            check(layer, gpu, synth.make_input(T, layer["n_embd"], seed=T))
+    for gpu in gpus:
+        gpu.close()
