@@ -544,8 +544,10 @@ uint32_t few_rows_for(const moe_layer *l, uint64_t R, uint32_t nexp) {
 // Whether groups of at most M rows go to the few-rows kernel: with more than two rows its eight columns are worth their
 // instructions whatever the type (200 rows of IQ3_S: 1085 -> 491 us); with one or two, where the integer-dot kernel's
 // decode is long and runs once a row (32 rows, even routing: Q4_K 309 -> 215 us, Q4_K with Q6_K 326 -> 251, IQ4_XS with
-// IQ4_NL 315 -> 276), not where it is nothing or a codebook's (Q8_0 246 -> 256, IQ3_S 272 -> 305, IQ2_S 281 -> 293).
+// IQ4_NL 315 -> 276), not where it is nothing or a codebook's (Q8_0 246 -> 256, IQ3_S 272 -> 305, IQ2_S 281 -> 293). Never
+// in a layer kept off the tensor cores (MOE_FLAG_NO_TENSOR), whose products are the integer-dot kernels' whatever the rows.
 bool groups_take_mma(const moe_layer *l, int M) {
+  if (!l->can_tensor) return false;
   const uint32_t g = l->cfg.gate_type, d = l->cfg.down_type;
   auto heavy = [](uint32_t t) { return t == QT_Q4_K || t == QT_Q6_K || t == QT_IQ4_XS || t == QT_IQ4_NL; };
   return (M > 2 || (M == 2 && heavy(g) && heavy(d))) && mma_takes(g, l->E, kGroupMax) && mma_takes(d, l->F, kGroupMax);

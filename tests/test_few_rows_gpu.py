@@ -1,7 +1,7 @@
-"""On a B200: the int8 tensor-instruction kernel for experts of a few rows, against the CPU oracle: as groups (a layer kept
-off the tile kernels, whose arithmetic it shares bit by bit but for f32 order) and as the short end of the tile list, with
-experts of more rows on the tile kernels in the same step; at the shortest rows, at lengths nothing is specialised for
-and at the longest a CTA holds."""
+"""On a B200: the int8 tensor-instruction kernel for experts of a few rows, against the CPU oracle: as groups (with a
+threshold for the tile kernels that no expert reaches; its arithmetic is the integer-dot kernels' but for f32 order) and as
+the short end of the tile list, with experts of more rows on the tile kernels in the same step; at the shortest rows and at
+lengths nothing is specialised for."""
 import numpy as np
 import pytest
 
@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("n_embd,n_ff", [(256, 256), (768, 1280), (2048, 512), (4352, 256)])
 def test_groups(t, n_embd, n_ff):
     layer = synth.make_layer(n_embd=n_embd, n_ff=n_ff, n_experts=64, n_used=4, gate_type=t, seed=t + n_embd)
-    gpu = MoELayer(layer, max_tokens=200, no_tensor=True)
+    gpu = MoELayer(layer, max_tokens=200, tensor_min_rows=256)
     for T in (9, 16, 17, 65, 200):  # groups of up to two; with more rows than experts, of up to eight
         check(layer, gpu, synth.make_input(T, n_embd, seed=T), INT_PATH_REL)
     gpu.close()
@@ -44,4 +44,20 @@ def test_both_lists_in_one_launch(t):
     base = synth.make_input(300, 512, seed=t)
     for T, repeats in ((16, 1), (17, 4), (32, 1), (33, 1), (200, 1), (120, 20), (200, 40)):
         check(layer, gpu, np.concatenate([np.repeat(base[:1], repeats, axis=0), base[1:T - repeats + 1]]))
+    gpu.close()
+
+
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("n_embd,n_ff", [(512, 256), (2048, 512)])
+def test_a_layer_kept_off_the_tensor_cores_keeps_its_integer_dots(t, n_embd, n_ff):
+    """MOE_FLAG_NO_TENSOR: the integer-dot kernels sum a row in one order however many rows a group holds (up to two, four at
+    a time, eight), so a row's output has the same bits whatever step it comes in."""
+    layer = synth.make_layer(n_embd=n_embd, n_ff=n_ff, n_experts=32, n_used=2, gate_type=t, seed=t)
+    gpu = MoELayer(layer, max_tokens=65, no_tensor=True)
+    x = synth.make_input(65, n_embd, seed=t)
+    few = check(layer, gpu, x[:16], INT_PATH_REL).copy()
+    assert gpu.groups()[:, 2].max() == 2
+    for T in (40, 65):
+        assert np.array_equal(check(layer, gpu, x[:T], INT_PATH_REL)[:16], few), T
+        assert gpu.groups()[:, 2].max() > 4
     gpu.close()
