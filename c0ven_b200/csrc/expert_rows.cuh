@@ -690,8 +690,13 @@ enum RowsForm { ROWS_LISTED, ROWS_ROUTED, ROWS_QUANT };
 // the CTAs that find their place and leave are too many (4 rows: 55 us against 29).
 // ROWS_QUANT (NMAT 1, steps of a few rows): the rows come as f32 (act_f32) and every CTA quantises those it stages, so that no
 // quantiser runs between the two products.
+//
+// Q6_K's forms for one and two rows are held to 128 registers, two CTAs an SM: left to itself the compiler takes up to 148 and
+// one CTA is left (32 rows of Q6_K with Q8_0, 235 experts: 377 us against 308; one row of Q6_K 59 against 56). The other
+// types' forms find their own balance (0: no minimum).
+__host__ __device__ constexpr int rows_min_ctas(int qt, int m) { return qt == QT_Q6_K && m <= 2 ? 2 : 0; }
 template <int QT, int NMAT, int M, int G, int UPL, int FORM>
-__global__ void __launch_bounds__(256) k_expert_rows(const ExpertRowsArgs a, const uint32_t *__restrict__ grid_global) {
+__global__ void __launch_bounds__(256, rows_min_ctas(QT, M)) k_expert_rows(const ExpertRowsArgs a, const uint32_t *__restrict__ grid_global) {
   extern __shared__ __align__(16) uint8_t smem[];
   dependents_may_launch(), wait_for_predecessors();
   constexpr bool q8k = act_is_q8k(QT);
