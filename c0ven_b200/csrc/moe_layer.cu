@@ -558,10 +558,12 @@ size_t router_rows_smem(uint32_t tm, uint32_t E) { return (size_t)tm * kRouterPi
 constexpr size_t kRouterRowsMaxSmem = 227 * 1024;  // what a CTA can have
 
 // Rows of x a CTA of the exact router takes. The fewer, the more CTAs share the step's multiply-adds and the shorter a lane's
-// chain of them, for one more reading of the router's 4 MB out of L2 a pass: 2 rows (13 rows: 35 -> 12.6 us against 8, ncu,
-// cold; 32 rows by fours, whose registers leave no room for sixteen loads in flight, 27); 8 in the long steps of a layer
-// kept off the tensor cores, where the readings would be what counts, as long as 8 rows fit a CTA (7,232 values a row).
-uint32_t router_rows_cta(uint32_t T, uint32_t E) { return T == 1 ? 1 : T <= kRouterExactRows || router_rows_smem(8, E) > kRouterRowsMaxSmem ? 2 : 8; }
+// chain of them, for one more reading of the router's 4 MB out of L2 a pass: 2 rows in steps of up to 32 (13 rows: 35 -> 12.6
+// us against 8, ncu, cold; 32 rows by fours, whose registers leave no room for sixteen loads in flight, 27); 8 in longer
+// ones, where the readings count (the layer in Q8_0, by 2 and by 8 rows: 40 rows 277 and 266 us, 48 rows 305 and 293; at
+// 32 it depends on the layer: 235 and 229 of 512 experts, 242 and 255 of 128), as long as 8 fit a CTA (7,232 values a row).
+constexpr uint32_t kRouterTwoRows = 32;
+uint32_t router_rows_cta(uint32_t T, uint32_t E) { return T == 1 ? 1 : T <= kRouterTwoRows || router_rows_smem(8, E) > kRouterRowsMaxSmem ? 2 : 8; }
 
 template <int TM, int D>
 cudaError_t launch_router_form(moe_layer *l, const float *x, uint32_t T, dim3 grid, uint32_t threads, const StepQuant &sq, cudaStream_t st) {
@@ -592,6 +594,11 @@ void launch_router_rows(moe_layer *l, const float *x, uint32_t T, cudaStream_t s
                         : tm == 2 ? (deep ? launch_router_form<2, 16> : launch_router_form<2, 8>) : launch_router_form<8, 8>;
   launched(l, launch(l, x, T, grid, 32 * warps, sq, st), "router logits");
 }
+
+// Steps of up to this many rows take the top-k and the pack in one launch. One CTA's warps share an SM's issue slots: with
+// more rows the top-k of four rows a CTA and the pack's own launches, each a dependent of the one before, take less (the
+// layer in Q8_0: 9 rows 124 us either way, 16 rows 164 and 160, 32 rows 250 and 235).
+constexpr uint32_t kTopkPackRows = 8;
 
 // Quantise x, the router's logits and top-k, and the pack of the step's T * K assignments over every expert. fork: an
 // event recorded once x is quantised, null for none.
@@ -633,8 +640,8 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st, Even
   const uint32_t tm = l->local == NE ? tensor_min_for(l, A) : 0, budget = l->local == NE ? tensor_budget_for(l, A) : 0;
   l->last_tensor_min = tm;
   const uint32_t chunk_len = kChunkTokens * K;
-  if (nchunks == 1 && NE <= 512) {
-    // One chunk: top-k, scan and fill in one CTA (the pack stage then has no kernel of its own).
+  if (T <= kTopkPackRows && NE <= 512) {
+    // Top-k, scan and fill in one CTA (the pack stage then has no kernel of its own).
     launched(l, launch_kernel(l->ctx.pdl, k_router_topk_pack, dim3(1), dim3(32 * kChunkTokens), chunk_len * sizeof(int32_t), st, l->rl.get(), l->bias.get(),
                               T, NE, K, l->ids.get(), l->w.get(), l->gs.get(), tm, budget, group_cap(A, NE),
                               l->pack.out(l->local == NE ? few_rows_for(l, A, NE) : FEW_NONE), l->pack.inv.get(),
@@ -642,19 +649,14 @@ void stage_route(moe_layer *l, const float *x, uint32_t T, cudaStream_t st, Even
              "router top-k and pack");
     mark(l, ST_PACK, st);
   } else {
-    if (approx) {
-      const RouterApprox ap{l->approx.get(), x, l->router.get(), l->norm2_parts.get(), l->gate_parts.get(), E, E / 256, router_parts, (uint64_t)T * NE,
-                            l->router_eps_rel, l->router_eps_abs};
-      launched(l, launch_kernel(l->ctx.pdl, k_router_topk_rows, dim3((T + kTopkRowsPerCta - 1) / kTopkRowsPerCta), dim3(32 * kTopkRowsPerCta), 0, st, ap,
-                                l->bias.get(), T, NE, K, l->ids.get(), l->w.get(), l->gs.get()),
-               "router top-k");
-      launched(l, launch_kernel(l->ctx.pdl, k_chunk_hist, dim3(nchunks), dim3(256), 0, st, l->ids.get(), (uint32_t)A, chunk_len, NE, 0, l->pack.chunk_hist.get()),
-               "chunk counts");
-    } else {
-      k_router_topk<<<nchunks, 32 * kChunkTokens, 0, st>>>(l->rl.get(), RouterApprox{}, l->bias.get(), T, NE, K, l->ids.get(), l->w.get(),
-                                                          l->gs.get(), l->pack.chunk_hist.get());
-      launched(l, cudaGetLastError(), "router top-k");
-    }
+    const RouterApprox ap = approx ? RouterApprox{l->approx.get(), x, l->router.get(), l->norm2_parts.get(), l->gate_parts.get(), E, E / 256, router_parts,
+                                                  (uint64_t)T * NE, l->router_eps_rel, l->router_eps_abs}
+                                   : RouterApprox{};
+    launched(l, launch_kernel(l->ctx.pdl, k_router_topk_rows, dim3((T + kTopkRowsPerCta - 1) / kTopkRowsPerCta), dim3(32 * kTopkRowsPerCta), 0, st,
+                              l->rl.get(), ap, l->bias.get(), T, NE, K, l->ids.get(), l->w.get(), l->gs.get()),
+             "router top-k");
+    launched(l, launch_kernel(l->ctx.pdl, k_chunk_hist, dim3(nchunks), dim3(256), 0, st, l->ids.get(), (uint32_t)A, chunk_len, NE, 0, l->pack.chunk_hist.get()),
+             "chunk counts");
     mark(l, ST_PACK, st);
     launch_pack(l, l->pack, PackJob{l->ids.get(), (uint32_t)A, chunk_len, nchunks, 0, tm, budget, group_cap(A, NE), K, l->local == NE ? few_rows_for(l, A, NE) : FEW_NONE}, st);
   }

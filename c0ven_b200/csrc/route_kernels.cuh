@@ -186,15 +186,16 @@ __device__ __forceinline__ void router_topk_block(const float *rl, const RouterA
 }
 
 // The top-k alone, a few rows a CTA and no barrier in it: for long steps, whose rows wait on memory for their exact
-// recomputations; with many small CTAs an SM always has rows that are not waiting, and no row waits for the slowest of
-// its chunk. The chunks' counts then come from k_chunk_hist.
+// recomputations (with many small CTAs an SM always has rows that are not waiting, and no row waits for the slowest of its
+// chunk), and for exact logits where the step's rows are more than one CTA's warps should take one after another. The
+// chunks' counts then come from k_chunk_hist.
 constexpr uint32_t kTopkRowsPerCta = 4;
-static __global__ void __launch_bounds__(32 * kTopkRowsPerCta) k_router_topk_rows(const RouterApprox ap, const float *__restrict__ bias, uint32_t T,
+static __global__ void __launch_bounds__(32 * kTopkRowsPerCta) k_router_topk_rows(const float *rl, const RouterApprox ap, const float *__restrict__ bias, uint32_t T,
                                                                                  uint32_t NE, uint32_t K, int32_t *__restrict__ ids,
                                                                                  float *__restrict__ w, float *__restrict__ gs) {
   __shared__ __align__(16) uint8_t ex_smem[kTopkRowsPerCta * kExWarpBytes];
   dependents_may_launch(), wait_for_predecessors();
-  router_topk_block(nullptr, ap, bias, T, NE, K, ids, w, gs, nullptr, nullptr, ap.E % (kRouterPieces * kExChunk) == 0 ? ex_smem : nullptr);
+  router_topk_block(rl, ap, bias, T, NE, K, ids, w, gs, nullptr, nullptr, ap.E % (kRouterPieces * kExChunk) == 0 ? ex_smem : nullptr);
 }
 
 static __global__ void __launch_bounds__(32 * kChunkTokens) k_router_topk(const float *__restrict__ rl, const RouterApprox ap,
@@ -513,8 +514,8 @@ static __global__ void __launch_bounds__(512) k_pack_fill(const int32_t *ids, ui
   row_src[row] = (a0 + i) / src_div;
 }
 
-// A step of one chunk (at most kChunkTokens rows): top-k, scan and fill in one CTA, three launches less for the steps
-// that launches bound. Dynamic shared memory kChunkTokens * K words for the chunk's ids.
+// A step of a few rows (one chunk of the pack at most, kChunkTokens rows): top-k, scan and fill in one CTA, four launches
+// less for the steps that launches bound. Dynamic shared memory kChunkTokens * K words for the chunk's ids.
 static __global__ void __launch_bounds__(32 * kChunkTokens, 1) k_router_topk_pack(const float *rl, const float *__restrict__ bias, uint32_t T,
                                                                        uint32_t NE, uint32_t K, int32_t *__restrict__ ids, float *__restrict__ w,
                                                                        float *__restrict__ gs, uint32_t tensor_min, uint32_t tensor_budget,
