@@ -680,8 +680,8 @@ enum RowsForm { ROWS_LISTED, ROWS_ROUTED, ROWS_QUANT };
 
 // NMAT 2: h[row][r] = swiglu(gate_r . x, up_r . x); NMAT 1: y[row][r] = down_r . h. One CTA of 8 warps per (row tile,
 // group); G lanes share a weight row (G = the row's units, up to 32), each taking UPL of its units (UPL 0: as many as
-// the row has, found at run time). Launch: grid (R / rows_per_cta, groups at most), 256 threads, dynamic shared memory
-// M * act_row_stride (+ 2 KB for IQ3_S's codebook).
+// the row has, found at run time). Launch: grid (R / (rows_per_cta * slabs), groups at most, CTAs that share a group), 256
+// threads, dynamic shared memory M * act_row_stride and a codebook type's codebook.
 //
 // ROWS_ROUTED (NMAT 2, steps of one or two rows): no top-k or list kernel runs in front. Every CTA takes the top-k of the
 // rows for itself, a warp a row (2 to 3 us, as long as it takes a kernel of its own, less that kernel's launch: 33.9 ->
@@ -875,13 +875,13 @@ __global__ void __launch_bounds__(256, rows_min_ctas(QT, M)) k_expert_rows(const
   }
 }
 
-// The down product of a step of one or two rows with everything after it: out[t][r] = sum over k, in rank order, of w[t][k] *
+// The down product of a step of one row with everything after it: out[t][r] = sum over k, in rank order, of w[t][k] *
 // (down_r of the row's k-th expert . h), + gs[t] * s[t][r], + res[t][r]. In place of a quantiser, k_expert_rows and
-// k_combine, whose launches such a step spends its time on: a warp takes an output row r for every assignment of the step
-// (an expert that two rows share is read again out of the caches), so a CTA holds all of the inner rows, which it
-// quantises itself (at most 32 rows; the same 2 KB of f32 a row by every CTA, out of L2: what
-// makes it the slower form for more rows, 37 us at 4 rows of Q6_K against 19 and a combine). The codes are left in q, d, bs
-// too, in expert order, by the CTAs in turn. G lanes a weight row, UPL units of it a lane.
+// k_combine, whose launches such a step spends its time on: a warp takes an output row r for every assignment of the step,
+// so a CTA holds all of the inner rows, which it quantises itself (the same 2 KB of f32 a row by every CTA, out of L2: what
+// makes it the slower form already for two rows, whose experts it would also read once a row: the layer in Q8_0 62 us
+// against 56, in Q2_0 80 against 64, of 2,560 x 768 values in Q4_K 92 against 78). The codes are left in q, d, bs too, in
+// expert order, by the CTAs in turn. G lanes a weight row, UPL units of it a lane.
 // Launch: grid by rows_per_warp * 8 output rows, 256 threads, dynamic shared memory A * act_row_stride + the codebook.
 struct DownCombineArgs {
   const uint8_t *w;
@@ -985,10 +985,5 @@ __global__ void __launch_bounds__(256) k_down_combine(const DownCombineArgs a, c
     __syncwarp();
   }
 }
-
-// Launches the instantiation for (M, K): host side of the kernels above. Returns cudaErrorInvalidValue for a shape no
-// instantiation takes. max_groups: the grid's second extent.
-template <int QT, int NMAT>
-cudaError_t launch_expert_rows(const ExpertRowsArgs &a, int M, uint32_t max_groups, const uint32_t *grid_global, cudaStream_t st);
 
 }  // namespace moe

@@ -531,6 +531,8 @@ uint32_t tensor_budget_for(const moe_layer *l, uint64_t R) {
 // expert rows over nexp experts, and by which rule (FewRows). With more than 24 rows an expert on average, too few of them
 // have 32 or less to pay for two more launches (2,000 rows of the benchmark's layer, 39 an expert: 850 -> 899 us in
 // IQ4_XS; 4,000 rows, skewed, over 64 experts: 237 -> 268).
+// Both products' rows have to fit: a CTA holds 32 of them, 2,816 values each at most (2,560 in Q6_K), also where no entry of
+// the step can have as many; layers of longer rows keep the tile kernels.
 uint32_t few_rows_for(const moe_layer *l, uint64_t R, uint32_t nexp) {
   const uint32_t tm = tensor_min_for(l, R);
   if (!tm || l->cfg.tensor_min_rows || R < 64 || R > 24ull * nexp) return FEW_NONE;
@@ -833,11 +835,16 @@ bool takes_short_form(const moe_layer *l, uint32_t T) {
   return !l->profile && T <= kShortRows && A <= kShortMax && (tm == 0 || T < tm) && tensor_budget_for(l, A) == 0;
 }
 
+// Whether a short step's gate/up kernel takes the top-k itself: with one or two rows, but not in the types whose decode needs
+// so many registers that two CTAs are on an SM, not three, so that the top-k is taken in more rounds of CTAs (one row: Q4_K
+// 53.4 us with it and 49.5 without, IQ4_XS 57.7 and 52.8, Q6_K 55.7 and 52.7; Q8_0 43 and 47, IQ3_S 41 and 50).
+bool gate_takes_route(uint32_t gate_type, uint32_t T) { return T <= 2 && gate_type != QT_Q4_K && gate_type != QT_Q6_K && gate_type != QT_IQ4_XS; }
+
 // A step of a few rows, in as few launches as its kernels can be put together into, for launches are what its time goes
 // into: the router with x quantised, the top-k with the lists, gate/up, the down product, which quantises its rows, and
-// the combine; with one or two rows the top-k is in the gate/up kernel and the combine in the down one. Beside the
-// routed experts', the shared expert's two. Stage by stage (forward_device) such a step is eleven launches, eight of them
-// one after another.
+// the combine; with one row the combine is in the down kernel, and with one or two the top-k may be in the gate/up kernel
+// (gate_takes_route). Beside the routed experts', the shared expert's two. Stage by stage (forward_device) such a step is
+// eleven launches, eight of them one after another.
 void forward_short(moe_layer *l, const float *x, uint32_t T, float *out, cudaStream_t st) {
   const uint32_t E = l->E, F = l->F, NE = l->NE, K = l->K, A = T * K;
   const moe_layer_config &c = l->cfg;
@@ -851,17 +858,17 @@ void forward_short(moe_layer *l, const float *x, uint32_t T, float *out, cudaStr
   }
   const uint32_t gmax = group_cap(A, NE);
   const ShortRoute rt{l->rl.get(), T, NE, K, gmax, l->ids.get(), l->w.get(), l->gs.get(), pk.inv.get(), pk.row_src.get(), pk.out()};
-  const bool routed = T <= 2;  // the top-k in the gate/up kernel
+  const bool routed = gate_takes_route(c.gate_type, T);
   if (!routed) launched(l, launch_kernel(l->ctx.pdl, k_short_route, dim3(1), dim3(32 * kShortRows), 0, st, rt), "router top-k and lists");
   l->last_T = T, l->last_pack = &pk, l->last_tensor_min = tensor_min_for(l, A);
-  const int M = routed ? (int)T : group_rows(std::min(gmax, T));
+  const int M = group_rows(std::min(gmax, T));
   ExpertRowsArgs a{};
   a.w0 = l->wg.get(), a.w1 = l->wu.get(), a.slice_bytes = l->gate_slice, a.K = E, a.R = F, a.rows_per_cta = 32;
   a.act = l->xq_routed.view(), a.act_row = pk.row_src.get(), a.groups = pk.groups.get(), a.ngroups = pk.counters.get() + 1;
   a.out = l->h.get(), a.out_stride = F, a.limit = c.swiglu_limit;
   if (routed) a.route = rt;
   launched(l, launch_rows(c.gate_type, 2, a, M, routed ? A + 1 : A, l->grid.get(), l->ctx, st), "experts gate/up");
-  if (T <= 2 && down_combine_takes(c.down_type, A, F)) {
+  if (T == 1 && down_combine_takes(c.down_type, A, F)) {
     if (l->has_shared) CUDA_OK(cudaStreamWaitEvent(st, l->join_ev->get(), 0));
     DownCombineArgs d{};
     d.w = l->wd.get(), d.slice_bytes = l->down_slice, d.K = F, d.R = E, d.T = T, d.used = K, d.NE = NE;
