@@ -811,14 +811,14 @@ __global__ void __launch_bounds__(256, rows_min_ctas(QT, M)) k_expert_rows(const
   __syncthreads();
 
   auto finish = [&](float (&acc)[NMAT][M], uint32_t r) {
+    // All M rows' sums, also where the group has fewer: leaving the loop at the group's last row made the whole kernel slower
+    // (groups of up to eight, 1,000 rows without the tensor cores: Q8_0 4.79 ms with every row's, 5.15 without; Q4_K 8.41, 8.96).
 #pragma unroll
-    for (int t = 0; t < M; t++) {
-      if ((uint32_t)t >= n) break;  // the same for the whole CTA
+    for (int t = 0; t < M; t++)
 #pragma unroll
       for (int m = 0; m < NMAT; m++)
 #pragma unroll
         for (int off = G / 2; off > 0; off >>= 1) acc[m][t] += __shfl_xor_sync(0xffffffffu, acc[m][t], off);
-    }
     if (li == 0 && r < a.R) {
 #pragma unroll
       for (int t = 0; t < M; t++)
