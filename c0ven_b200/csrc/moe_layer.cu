@@ -543,16 +543,18 @@ uint32_t few_rows_for(const moe_layer *l, uint64_t R, uint32_t nexp) {
   return std::min<uint64_t>(R, nexp) <= 128 ? FEW_IF_ALL : FEW_NONE;
 }
 
-// Whether groups of at most M rows go to the few-rows kernel: with more than two rows its eight columns are worth their
+// Whether groups of at most M rows, in a call of R expert rows, go to the few-rows kernel: with more than two rows its eight columns are worth their
 // instructions whatever the type (200 rows of IQ3_S: 1085 -> 491 us); with one or two, where the integer-dot kernel's
 // decode is long and runs once a row (32 rows, even routing: Q4_K 309 -> 215 us, Q4_K with Q6_K 326 -> 251, IQ4_XS with
-// IQ4_NL 315 -> 276), not where it is nothing or a codebook's (Q8_0 246 -> 256, IQ3_S 272 -> 305, IQ2_S 281 -> 293). Never
+// IQ4_NL 315 -> 276), not where it is nothing or a codebook's (Q8_0 246 -> 256, IQ3_S 272 -> 305, IQ2_S 281 -> 293), nor in
+// steps of so few rows that the kernel's warps, of 16 weight rows, are few (5 rows over 256 experts in Q4_K and Q6_K: 51 ->
+// 61 us for the experts' stage; 40 rows 92 either way). Never
 // in a layer kept off the tensor cores (MOE_FLAG_NO_TENSOR), whose products are the integer-dot kernels' whatever the rows.
-bool groups_take_mma(const moe_layer *l, int M) {
+bool groups_take_mma(const moe_layer *l, int M, uint64_t R) {
   if (!l->can_tensor) return false;
   const uint32_t g = l->cfg.gate_type, d = l->cfg.down_type;
   auto heavy = [](uint32_t t) { return t == QT_Q4_K || t == QT_Q6_K || t == QT_IQ4_XS || t == QT_IQ4_NL; };
-  return (M > 2 || (M == 2 && heavy(g) && heavy(d))) && mma_takes(g, l->E, kGroupMax) && mma_takes(d, l->F, kGroupMax);
+  return (M > 2 || (M == 2 && R >= 32 && heavy(g) && heavy(d))) && mma_takes(g, l->E, kGroupMax) && mma_takes(d, l->F, kGroupMax);
 }
 
 // Shared memory of the exact router's CTA: tm rows of x, each in padded pieces.
@@ -682,7 +684,9 @@ void stage_experts(moe_layer *l, const ActSource &src, const PackBuffers &pk, ui
   const uint32_t gmax = group_cap(R, nexp);
   int M = group_rows(std::min<uint64_t>(std::min<uint64_t>(gmax, most), tm ? std::min<uint64_t>(R, tm - 1) : R));
   // Groups of up to eight rows where an expert has two or three on average: the kernel for four, whose accumulators leave
-  // room for three CTAs on an SM, takes nearly all of them whole, and the odd longer one in two halves.
+  // room for three CTAs on an SM, takes nearly all of them whole, and the odd longer one in two halves. (In layers kept off
+  // the tensor cores, and with rows too long for the few-rows kernel, which has these groups otherwise. 100 rows without
+  // the tensor cores, by eight and by four: Q8_0 697 and 552 us, Q4_K 1,064 and 839, IQ3_S 626 and 585.)
   const uint32_t halves = M == 8 && R <= 3ull * nexp ? 2 : 1;
   M /= halves;
   const uint32_t max_groups =
@@ -699,7 +703,7 @@ void stage_experts(moe_layer *l, const ActSource &src, const PackBuffers &pk, ui
                                 src.h == l->xq_routed.h.get() && src.act_row != nullptr;
   // The experts of a few rows: the short tiles at the list's end, or groups of up to eight rows.
   static_assert(sizeof(BigTile) == sizeof(MoeGroup), "both lists are (slot, start, rows)");
-  const bool few = max_big && few_rows_for(l, R, nexp) != FEW_NONE, groups_mma = max_groups && groups_take_mma(l, M);
+  const bool few = max_big && few_rows_for(l, R, nexp) != FEW_NONE, groups_mma = max_groups && groups_take_mma(l, M, R);
   if (max_big) {
     // The rows in expert order first (the reference's p_moe_scatter, kernels/models/qwen4exp/prompt.cl:744-754): a tile's
     // rows are then one box after another for the kernel's copies. Part of the pack stage: the gate/up stage times the
