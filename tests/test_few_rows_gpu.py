@@ -24,21 +24,58 @@ def test_groups(t, n_embd, n_ff):
 @pytest.mark.parametrize("gate,down", [(t, t) for t in TYPES] + [(synth.Q4_K, synth.Q6_K), (synth.IQ4_XS, synth.IQ4_NL)])
 def test_short_tiles_beside_long_ones(gate, down):
     """Rows that repeat route alike: experts that only one of the rows chose get its repeats, up to and past the 8 rows of
-    one instruction and the 32 of an entry."""
+    one instruction and the 16 that an entry holds in a step that hits fewer than 256 experts; longer ones take the tiles."""
     layer = synth.make_layer(n_embd=768, n_ff=512, n_experts=320, n_used=4, gate_type=gate, down_type=down, seed=gate * 50 + down)
     repeats = [1, 7, 8, 9, 16, 17, 24, 25, 32, 33, 300, 2, 32]
     x = np.repeat(synth.make_input(len(repeats), 768, seed=3), repeats, axis=0)
     gpu = MoELayer(layer, max_tokens=len(x))
     check(layer, gpu, x)
     cnt = np.bincount(gpu.route(len(x))[0].reshape(-1), minlength=320)
-    assert {1, 7, 8, 9, 16, 17, 24, 25, 32, 33, 300} <= set(cnt.tolist())
+    assert {1, 7, 8, 9, 16, 17, 24, 25, 32, 33, 300} <= set(cnt.tolist()) and np.count_nonzero(cnt) < 256
+    gpu.close()
+
+
+@pytest.mark.parametrize("gate,down", [(t, t) for t in TYPES] + [(synth.Q4_K, synth.Q6_K), (synth.IQ4_XS, synth.IQ4_NL)])
+def test_entries_of_up_to_32_rows(gate, down):
+    """A step that hits 256 experts or more: those of up to 32 rows are entries of the kernel, in all four of its forms, and
+    longer ones stay on the tile kernels. (Below 256 the cut is at 16 rows: test_short_tiles_beside_long_ones.)"""
+    layer = synth.make_layer(n_embd=768, n_ff=512, n_experts=320, n_used=4, gate_type=gate, down_type=down, seed=gate * 51 + down)
+    repeats = list(range(9, 33))
+    x = synth.make_input(340 + len(repeats), 768, seed=3)
+    x = np.concatenate([x[len(repeats):], np.repeat(x[:len(repeats)], repeats, axis=0)])
+    gpu = MoELayer(layer, max_tokens=len(x))
+    check(layer, gpu, x)
+    cnt = np.bincount(gpu.route(len(x))[0].reshape(-1), minlength=320)
+    assert np.count_nonzero(cnt) >= 256 and 1280 <= cnt.sum() <= 24 * 320
+    for lo, hi in ((1, 8), (9, 16), (17, 24), (25, 32), (33, 256)):
+        assert np.count_nonzero((cnt >= lo) & (cnt <= hi)) >= 8, (lo, hi)
+    assert len(gpu.groups()) == 0
     gpu.close()
 
 
 @pytest.mark.parametrize("t", TYPES)
-def test_both_lists_in_one_launch(t):
-    """Steps of 64 to 1,279 assignments: all experts on the tile list (few experts), on the groups' list, or on both (an
-    expert that many rows chose beside others of one or two), with and without one that needs the tile kernels."""
+def test_both_lists_in_one_step(t):
+    """Steps of 64 to 1,279 assignments over up to 128 experts whose threshold the pack lowers to two rows: the experts with
+    one row are groups, the others the tile list, short enough for the kernel to take it whole (in the same launch where
+    groups of that size are its own) and, with rows that repeat, with an expert too long for that."""
+    layer = synth.make_layer(n_embd=512, n_ff=256, n_experts=128, n_used=4, gate_type=t, seed=t)
+    gpu = MoELayer(layer, max_tokens=60)
+    base = synth.make_input(60, 512, seed=t)
+    for T, repeats in ((32, 1), (40, 1), (44, 1), (50, 12)):  # 128 assignments: groups of up to two; more: of up to eight
+        x = np.concatenate([np.repeat(base[:1], repeats, axis=0), base[1:T - repeats + 1]])
+        check(layer, gpu, x)
+        cnt = np.bincount(gpu.route(T)[0].reshape(-1), minlength=128)
+        assert (cnt.max() <= 8) == (repeats == 1)
+        groups = gpu.groups()
+        assert len(groups) == np.count_nonzero(cnt == 1) > 0
+        assert gpu.stats()["last_tensor_rows"] - T == cnt[cnt > 1].sum() > 0  # T: the shared expert's rows
+    gpu.close()
+
+
+@pytest.mark.parametrize("t", TYPES)
+def test_one_list_or_the_other(t):
+    """Steps of 64 to 1,279 assignments: all experts on the tile list (few experts) or all on the groups' list, with and
+    without one that needs the tile kernels."""
     layer = synth.make_layer(n_embd=512, n_ff=256, n_experts=320, n_used=4, gate_type=t, seed=t)
     gpu = MoELayer(layer, max_tokens=300)
     base = synth.make_input(300, 512, seed=t)

@@ -1,6 +1,8 @@
-"""On a B200: steps of a few rows, which run in three launches (the router with the quantisers; gate/up with the top-k in
-every CTA; the down product with the combine), against the CPU oracle and against the same layer stage by stage (a
-profiled layer takes its steps that way). Around the edges of the rule: 8 rows, 64 assignments, 128 units a weight row."""
+"""On a B200: steps of a few rows against the CPU oracle and against the same layer stage by stage (a profiled layer takes
+its steps that way). One or two rows run in three launches: the router with the quantisers; gate/up with the top-k in
+every CTA; the down product with the combine. Up to eight rows and 64 assignments take five: the top-k with the lists and
+the combine have their own. Around the edges of the rules: 2 and 8 rows, 64 assignments, 128 units a weight row; and
+router rows of every length a layer may have."""
 import numpy as np
 import pytest
 
