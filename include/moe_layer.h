@@ -64,8 +64,12 @@ typedef struct {
   int32_t device;             /* CUDA device ordinal */
   float swiglu_limit;         /* ExpertShape::swiglu_limit; 0: off */
   uint32_t flags;             /* MOE_FLAG_* */
-  uint32_t tensor_min_rows;   /* an expert with at least this many rows in a call goes to the tensor-core kernels, one
-                                 with fewer to the integer-dot kernels; default 16 */
+  uint32_t tensor_min_rows;   /* an expert with at least this many rows in a call goes to the tile kernels (tcgen05, f16
+                                 products), one with fewer to the kernels for groups of at most 8 rows (int8 products,
+                                 by dp4a or by the warp-level tensor instruction). 0: the call decides: every expert to
+                                 the tile kernels from 1,280 assignments on; in shorter calls 16, or fewer rows where
+                                 few experts then take them; and experts of up to 32 rows may leave the tile kernels
+                                 for the int8 one */
   uint32_t max_expert_rows;   /* expert parallel: rows moe_layer_experts_device may receive; default max_tokens * n_used */
   uint32_t host_chunk_rows;   /* moe_layer_forward (host buffers): calls of at least twice this many rows are cut into
                                  chunks of about this many, and a chunk's copies to and from the GPU run beside its
@@ -112,11 +116,15 @@ typedef struct {
   uint64_t d2h_bytes;
   uint64_t last_tiles;        /* of the last call */
   uint64_t last_experts_hit;  /* distinct experts the last call's rows routed to */
-  uint64_t last_tensor_rows;  /* of its assignments, those the tensor-core kernels computed */
+  uint64_t last_tensor_rows;  /* of its assignments, those of experts listed for the tile kernels (tensor_min_rows), the
+                                 int8 kernel's share of that list with them; its rows too, where the shared expert ran
+                                 on the tile kernels */
 } moe_layer_stats;
 
 #define MOE_STAGES 8
-/* Stage names, in order: "quantize", "router", "pack", "gate_up", "down", "shared", "combine", "copies". */
+/* Stage names, in order: "quantize", "router", "pack", "gate_up", "down", "shared", "combine", "copies". In calls of up to
+ * 64 rows (and every call with MOE_FLAG_NO_TENSOR) the router's own launch quantises x: "quantize" is then empty and
+ * "router" holds both. "down" begins with the quantiser of its input. */
 
 /* Uploads the weights in the layout the kernels read and allocates every buffer a call needs. */
 MOE_API moe_status moe_layer_create(const moe_layer_config *config, const moe_layer_weights *weights, moe_layer **out);
@@ -238,7 +246,7 @@ MOE_API moe_status moe_layer_sync(moe_layer *l, uint32_t timeout_ms);
 MOE_API moe_status moe_layer_read_route(moe_layer *l, int32_t *ids, float *w, uint32_t *inv, moe_tile *tiles,
                                         uint32_t tiles_cap, uint32_t *ntiles);
 
-/* The last call's groups for the integer-dot kernels (the reference's MoeGroup, shared/moe_tile.h:20-33, as a range:
+/* The last call's groups of at most 8 rows, for the kernels of int8 products (the reference's MoeGroup, shared/moe_tile.h:20-33, as a range:
  * its assignments are rows start .. start + n of the expert order, which lists an expert's assignments in ascending
  * order, so a group holds what core/tests/step_rows_test.cpp:40-58 puts in it; the list is in expert order, not in
  * order of first assignment). Up to cap of them; *ngroups, how many there are. Waits for the stream. */
