@@ -591,8 +591,12 @@ void launch_router_rows(moe_layer *l, const float *x, uint32_t T, cudaStream_t s
   sq.job[0] = l->xq_routed.job();
   if (l->has_shared && !l->shared_x_same) sq.job[1] = l->xq_shared.job();
   sq.nblk = (uint64_t)T * (E / 256);
-  sq.ctas = (uint32_t)((sq.nblk + (uint64_t)warps * passes - 1) / (warps * passes));
-  const dim3 grid(sq.ctas + (N + 4 * warps - 1) / (4 * warps), passes);
+  // CTAs of eight rows: the quantisers get those SMs that the router's CTAs leave, one CTA a pass at least. With a CTA for every
+  // eight blocks they made 200 CTAs of 64 rows, and so SMs with two of the router's (42 us by ncu, cold; a rank of two
+  // routing 64 rows 86 us, 72 now; the layer in Q8_0 5 % less).
+  const uint32_t router_ctas = (N + 4 * warps - 1) / (4 * warps), most = (uint32_t)((sq.nblk + (uint64_t)warps * passes - 1) / (warps * passes));
+  sq.ctas = tm < 8 ? most : std::min(most, std::max(1u, l->sms / passes > router_ctas ? l->sms / passes - router_ctas : 1));
+  const dim3 grid(sq.ctas + router_ctas, passes);
   const bool deep = (E / kRouterPieces) % 64 == 0;  // sixteen loads in flight a lane: a step of one row is all latency
   auto launch = tm == 1 ? (deep ? launch_router_form<1, 16> : launch_router_form<1, 8>)
                         : tm == 2 ? (deep ? launch_router_form<2, 16> : launch_router_form<2, 8>) : launch_router_form<8, 8>;

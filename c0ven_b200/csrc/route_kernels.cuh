@@ -86,7 +86,8 @@ static __global__ void __launch_bounds__(256) k_quant(const float *x, uint64_t n
 // in flight per lane (a piece is a multiple of 4 D values: 8 always, 16 when the piece is a multiple of 64 values). A CTA
 // is 1 to 8 warps, by the step's rows (launch_router_rows).
 // The step's quantisers ride along: the first sq.ctas CTAs of every grid row share out the blocks of x among their warps,
-// so that quantising x is neither a launch of its own in front of the router nor behind it.
+// so that quantising x is neither a launch of its own in front of the router nor behind it. A warp takes as many blocks as
+// that leaves it.
 struct StepQuant {
   QuantJob job[2];  // the routed experts' form of x, and the shared expert's where it is another one
   uint64_t nblk;
@@ -102,16 +103,17 @@ static __global__ void __launch_bounds__(256) k_router_logits_rows(const float *
   if (blockIdx.x < sq.ctas) {
     wait_for_predecessors();
     const uint32_t lane = threadIdx.x % 32, warps = blockDim.x / 32;
-    const uint64_t blk = ((uint64_t)blockIdx.y * sq.ctas + blockIdx.x) * warps + threadIdx.x / 32;
-    if (blk >= sq.nblk) return;
-    const float4 a = ((const float4 *)(x + blk * 256))[2 * lane], b = ((const float4 *)(x + blk * 256))[2 * lane + 1];
+    const uint64_t step = (uint64_t)gridDim.y * sq.ctas * warps;
+    for (uint64_t blk = ((uint64_t)blockIdx.y * sq.ctas + blockIdx.x) * warps + threadIdx.x / 32; blk < sq.nblk; blk += step) {
+      const float4 a = ((const float4 *)(x + blk * 256))[2 * lane], b = ((const float4 *)(x + blk * 256))[2 * lane + 1];
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-      if (!sq.job[j].q) continue;
-      if (sq.job[j].q8k)
-        quantize_store<true>(a, b, blk, lane, sq.job[j]);
-      else
-        quantize_store<false>(a, b, blk, lane, sq.job[j]);
+      for (int j = 0; j < 2; j++) {
+        if (!sq.job[j].q) continue;
+        if (sq.job[j].q8k)
+          quantize_store<true>(a, b, blk, lane, sq.job[j]);
+        else
+          quantize_store<false>(a, b, blk, lane, sq.job[j]);
+      }
     }
     return;
   }
