@@ -9,30 +9,32 @@
 namespace moe {
 
 template <int QT, int NMAT, int MOST>
-static cudaError_t launch_mma_one(ExpertMmaArgs a, uint32_t max_entries, const LaunchCtx &ctx, cudaStream_t st) {
+static cudaError_t launch_mma_one(const ExpertMmaArgs &a, uint32_t max_entries, const LaunchCtx &ctx, cudaStream_t st) {
   auto kernel = k_expert_mma<QT, NMAT, MOST>;
-  const size_t smem = mma_smem(QT, 8 * MOST, a.K);
-  if (smem > 48 * 1024) {
-    static std::atomic<uint32_t> attr_done{0};
-    const cudaError_t e = ensure_dynamic_smem(kernel, kMmaMaxSmem, attr_done, ctx.device);
-    if (e != cudaSuccess) return e;
-  }
-  // Slabs a CTA: rows are staged, and a codebook with them, once for all of them. Groups of up to eight rows come in their
-  // hundreds: four slabs where that leaves an SM more CTAs than it runs at once (100 rows of Q8_0: 452 us with one slab
-  // of gate and up and two of down, 410 with four). The list of short tiles, which holds a fraction of max_entries when
-  // the routing is skewed, is cut finer, so that few experts still spread over the SMs (256 rows, skewed: 243 -> 200 us).
-  const uint64_t ctas = (uint64_t)(a.R / kMmaCtaRows) * max_entries;
-  a.slabs = MOST > 1 ? (NMAT == 2 ? 1 : 2) : ctas >= 16ull * ctx.sms ? 4 : ctas >= 8ull * ctx.sms ? 2 : 1;
-  // The lists' lengths are the device's, often a fraction of max_entries: no more CTAs than four rounds of them, which then
-  // take the entries in turn (CTAs that find their list ended cost some 3 ns each: 4,096 of them 10 us).
-  const uint32_t gx = (a.R / kMmaCtaRows + a.slabs - 1) / a.slabs, most = std::max(1u, 8 * ctx.sms / gx);
-  const dim3 grid(gx, std::min(max_entries, most));
-  return launch_kernel(ctx.pdl, kernel, grid, dim3(256), smem, st, a);
+  static std::atomic<uint32_t> attr_done{0};
+  constexpr size_t kSmSmem = 228 * 1024, kMost = 227 * 1024;  // an SM's shared memory, 1 KB of it kept for every CTA; what a CTA can have
+  const cudaError_t e = ensure_dynamic_smem(kernel, kMost, attr_done, ctx.device);
+  if (e != cudaSuccess) return e;
+  auto smem_of = [&](uint32_t warps) {
+    return (size_t)mma_smem(QT, 8 * MOST, a.K) + (size_t)warps * mma_stages(QT, MOST) * Frag<QT>::kStage;
+  };
+  // Sixteen warps an SM, in two CTAs; in one where two CTAs' rows do not fit (32 rows of 2,560 values).
+  uint32_t warps = 8, per_sm = MOST == 1 && grid_words(QT) ? 3 : 2;
+  while (per_sm > 1 && per_sm * (smem_of(8) + 1024) > kSmSmem) per_sm--;
+  if (per_sm == 1 && 32 * 16 <= mma_threads(MOST) && smem_of(16) <= kMost) warps = 16;
+  // Gate and up: an item is some 16 to 32 stages a warp, so CTAs of one item each, up to eight rounds of them, are shared out by
+  // the SMs as they come free. A down item is a stage or four: one round of CTAs, each with runs of items. (One round and eight,
+  // layer: Q8_0 60 rows 301 and 274 us, Q4_K 777 rows 384 and 377 for gate and up; 100 rows of Q4_K 242 and 252 for down.) CTAs past
+  // the items cost some 4 us a thousand: sixteen rounds lose that again (Q4_K 32 rows 168 -> 188).
+  constexpr uint32_t kRounds = NMAT == 1 ? 1 : 8;
+  const uint64_t items = (uint64_t)(a.R / (16 * warps)) * max_entries;
+  const dim3 grid((unsigned)std::min<uint64_t>(items, (uint64_t)kRounds * per_sm * ctx.sms));
+  return launch_kernel(ctx.pdl, kernel, grid, dim3(32 * warps), smem_of(warps), st, a);
 }
 
 template <int QT, int NMAT>
 cudaError_t launch_expert_mma(const ExpertMmaArgs &a, uint32_t most_rows, uint32_t max_entries, const LaunchCtx &ctx, cudaStream_t st) {
-  if (!mma_takes(QT, a.K, most_rows <= 8 ? 8 : kMmaRows) || a.R % kMmaCtaRows || most_rows > kMmaRows || max_entries == 0) return cudaErrorInvalidValue;
+  if (!mma_takes(QT, a.K, most_rows <= 8 ? 8 : kMmaRows) || a.R % kMmaRowsUnit || most_rows > kMmaRows || max_entries == 0) return cudaErrorInvalidValue;
   return most_rows <= 8 ? launch_mma_one<QT, NMAT, 1>(a, max_entries, ctx, st) : launch_mma_one<QT, NMAT, 4>(a, max_entries, ctx, st);
 }
 

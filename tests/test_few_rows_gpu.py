@@ -98,3 +98,14 @@ def test_a_layer_kept_off_the_tensor_cores_keeps_its_integer_dots(t, n_embd, n_f
         assert np.array_equal(check(layer, gpu, x[:T], INT_PATH_REL)[:16], few), T
         assert gpu.groups()[:, 2].max() > 4
     gpu.close()
+
+
+@pytest.mark.parametrize("t", TYPES)
+def test_entries_whose_rows_leave_room_for_one_cta(t):
+    """Rows of which two CTAs' 32 do not fit an SM: one CTA of sixteen warps takes them; with entries of 1 to 32 rows, and a
+    down product of more items than CTAs, each of which then takes runs of several entries."""
+    layer = synth.make_layer(n_embd=2560, n_ff=512, n_experts=96, n_used=4, gate_type=t, seed=t + 7)
+    gpu = MoELayer(layer, max_tokens=350)
+    check(layer, gpu, synth.make_input(350, 2560, seed=5))
+    assert len(gpu.groups()) == 0
+    gpu.close()
