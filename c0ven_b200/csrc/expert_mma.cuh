@@ -330,12 +330,6 @@ struct Frag<QT_Q6_K> {
 // lane's share is four bytes, looked up in the order their nibbles have (values v, 16 + v, v + 1, 17 + v of a word): the rows' codes
 // are staged in that order too (mma_stage_acts), so nothing parts low nibbles from high ones.
 __host__ __device__ constexpr bool mma_paired(uint32_t qt) { return qt == QT_IQ4_XS || qt == QT_IQ4_NL; }
-__device__ __forceinline__ uint2 iq4_pairs(uint32_t q) {
-  constexpr uint32_t T0 = iq4_table_word(0), T1 = iq4_table_word(1), T2 = iq4_table_word(2), T3 = iq4_table_word(3);
-  const uint32_t e = q & 0x77777777u, half = (q >> 1 & 0x44444444u) | 0x32103210u;
-  return make_uint2(__byte_perm(__byte_perm(T0, T1, e), __byte_perm(T2, T3, e), half),
-                    __byte_perm(__byte_perm(T0, T1, e >> 16), __byte_perm(T2, T3, e >> 16), half >> 16));
-}
 // y = d * (ls - 32) * table[q], a 6-bit ls a sub-block.
 template <>
 struct Frag<QT_IQ4_XS> {
@@ -371,7 +365,7 @@ struct Frag<QT_IQ4_XS> {
     for (int t = 0; t < NT; t++) sum[t][0] = sum[t][1] = sum[t][2] = sum[t][3] = 0;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-      const uint2 ax = iq4_pairs(x.q[i]), ay = iq4_pairs(y.q[i]);
+      const uint2 ax = iq4_pairs<0>(x.q[i]), ay = iq4_pairs<0>(y.q[i]);
       const int sx = (int)(((x.sl >> (4 * i)) & 0xF) | (((x.sh >> (2 * i)) & 3) << 4)) - 32, sy = (int)(((y.sl >> (4 * i)) & 0xF) | (((y.sh >> (2 * i)) & 3) << 4)) - 32;
 #pragma unroll
       for (int t = 0; t < NT; t++) {
@@ -416,7 +410,7 @@ struct Frag<QT_IQ4_NL> {
   __device__ static __forceinline__ void block(const Row &x, const Row &y, uint32_t b, uint32_t g, uint32_t j, const MmaActs &acts, float (&f)[NT][4]) {
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-      const uint2 ax = iq4_pairs(x.q[i]), ay = iq4_pairs(y.q[i]);
+      const uint2 ax = iq4_pairs<0>(x.q[i]), ay = iq4_pairs<0>(y.q[i]);
       const float dx = scale(x.d, i), dy = scale(y.d, i);
 #pragma unroll
       for (int t = 0; t < NT; t++) {

@@ -456,6 +456,19 @@ __device__ __forceinline__ void iq4_lookup8(uint32_t q, uint32_t &lo, uint32_t &
   lo = __byte_perm(r0, r1, 0x6420u), hi = __byte_perm(r0, r1, 0x7531u);
 }
 
+// Table values of q's eight nibbles in the order the nibbles have: .x those of its low two bytes (low nibble, high nibble, low,
+// high), .y of its high two; each byte plus BIAS. Where both operands of a dot or a later permute agree on that order, the
+// parting permutes of iq4_lookup8 are saved.
+template <int BIAS>
+__device__ __forceinline__ uint2 iq4_pairs(uint32_t q) {
+  constexpr uint32_t B = 0x01010101u * BIAS;  // 0 or 128: the sign bits flipped
+  constexpr uint32_t T0 = iq4_table_word(0) ^ B, T1 = iq4_table_word(1) ^ B, T2 = iq4_table_word(2) ^ B, T3 = iq4_table_word(3) ^ B;
+  static_assert(BIAS == 0 || BIAS == 128, "an exclusive-or adds nothing else");
+  const uint32_t e = q & 0x77777777u, half = (q >> 1 & 0x44444444u) | 0x32103210u;
+  return make_uint2(__byte_perm(__byte_perm(T0, T1, e), __byte_perm(T2, T3, e), half),
+                    __byte_perm(__byte_perm(T0, T1, e >> 16), __byte_perm(T2, T3, e >> 16), half >> 16));
+}
+
 // Sixteen 2-bit codes (a word's low or high half: 4 bytes of 4 codes) as 16 signed bytes q - 1 in four words. A byte's
 // four codes are spread to the digits of a permute selector, whose table is the bytes -1, 0, 1, 2.
 __device__ __forceinline__ uint32_t q2_bytes(uint32_t c) {  // c: one byte, four codes

@@ -294,9 +294,8 @@ __device__ __forceinline__ __half2 small_h2(uint32_t v) { return __hsub2(as_h2(0
 // a unit ahead of the decode. A load whose lanes each read a row of their own costs the load pipe a wavefront a lane,
 // whatever its width, so a unit is as much of a row as one round of wide loads brings: half a block of 256 values (two
 // stages), whose codes, signs, high bits and scales are then 3 to 8 loads. (Fetched a stage at a time, in halves of 32,
-// the same 128 values were 8 to 28 loads: 28 for Q6_K, 20 for IQ2_S and IQ3_S.) The unit of Q8_0, IQ4_NL and IQ4_XS is
-// one stage: two units of two in flight spill registers there, which cost more than the loads (IQ4_XS and IQ4_NL, 4,352
-// rows of the benchmark's layer: 1.01 ms against 0.97). Gate and up of IQ3_S and Q6_K spill too, 188 and 788 bytes of loads
+// the same 128 values were 8 to 28 loads: 28 for Q6_K, 20 for IQ2_S and IQ3_S.) The unit of Q8_0 is one stage: two units of
+// two in flight spill registers there, which cost more than the loads. Gate and up of IQ3_S and Q6_K spill too, 188 and 788 bytes of loads
 // a thread, and gain all the same: the layer's time at 4,352 rows is 0.90 and 0.63 of what it was with halves.
 template <int QT>
 struct Decoder;
@@ -605,13 +604,23 @@ __device__ __forceinline__ void int8x16_to_f16(const uint32_t (&w)[4], __half2 d
   }
 }
 // A block or sub-block of 32 four-bit codes (16 bytes: values 0 .. 15 in the low nibbles, 16 .. 31 in the high ones)
-// through the table, times d2, into chunks 4 h .. 4 h + 3 of the row.
+// through the table, times d2, into chunks 4 h .. 4 h + 3 of the row. The permutes that put the exponent byte beside two of the
+// looked-up bytes take every other one, so they part low nibbles from high ones too.
 __device__ __forceinline__ void iq4_store32(const uint4 &q, __half2 d2, uint8_t *tile, uint32_t m, uint32_t h) {
-  uint32_t lo[4], hi[4], o[16];
-  iq4_lookup8(q.x, lo[0], hi[0]), iq4_lookup8(q.y, lo[1], hi[1]), iq4_lookup8(q.z, lo[2], hi[2]), iq4_lookup8(q.w, lo[3], hi[3]);
-  int8x16_to_f16(lo, d2, o), int8x16_to_f16(hi, d2, o + 8);
+  const __half2 off = as_h2(0x64806480u);  // 1152 = 1024 + 128
+  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+  uint32_t lo[8], hi[8];
 #pragma unroll
-  for (int c = 0; c < 4; c++) store_chunk(tile, m, 4 * h + c, make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]));
+  for (int i = 0; i < 4; i++) {
+    const uint2 v = iq4_pairs<128>(w[i]);
+    lo[2 * i] = as_u32(__hmul2(__hsub2(as_h2(bias_h2(v.x, 0x4240)), off), d2)), lo[2 * i + 1] = as_u32(__hmul2(__hsub2(as_h2(bias_h2(v.y, 0x4240)), off), d2));
+    hi[2 * i] = as_u32(__hmul2(__hsub2(as_h2(bias_h2(v.x, 0x4341)), off), d2)), hi[2 * i + 1] = as_u32(__hmul2(__hsub2(as_h2(bias_h2(v.y, 0x4341)), off), d2));
+  }
+#pragma unroll
+  for (int c = 0; c < 2; c++) {
+    store_chunk(tile, m, 4 * h + c, make_uint4(lo[4 * c], lo[4 * c + 1], lo[4 * c + 2], lo[4 * c + 3]));
+    store_chunk(tile, m, 4 * h + 2 + c, make_uint4(hi[4 * c], hi[4 * c + 1], hi[4 * c + 2], hi[4 * c + 3]));
+  }
 }
 
 // Q2_0: w = (q - 1) * d. A stage is one block of 64, 16 bytes.
@@ -646,57 +655,48 @@ struct Decoder<QT_Q2_0> {
   }
 };
 
-// IQ4_NL: w = d * table[q]. A half is one block of 32.
+// IQ4_NL: w = d * table[q], blocks of 32 with a scale each; a header is the eight scales of 256 values.
 template <>
 struct Decoder<QT_IQ4_NL> {
   static constexpr uint32_t kUnitStages = 1;
-  static constexpr uint32_t kUnitBytes = 32;  // of the main quants run
-  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint32_t K, uint32_t r, uint32_t u) { return s + (uint64_t)r * (K / 2) + 32 * u; }
-  struct Raw {
-    uint4 q[2];
-    __half2 d;
+  struct Hdr {
+    uint4 d;
   };
-  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t u) {
-    Raw x;
-    const uint8_t *q = quants_at(s, K, r, u);
-    x.q[0] = ldg16(q), x.q[1] = ldg16(q + 16);
-    x.d = __ldg((const __half2 *)((const __half *)(s + 16 * nblk) + (uint64_t)r * (K / 32) + 2 * u));
-    return x;
+  struct Raw {
+    uint4 q;
+  };
+  __device__ static __forceinline__ Hdr fetch_hdr(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t k0) {
+    return Hdr{__ldg((const uint4 *)((const __half *)(s + 16 * nblk) + (uint64_t)r * (K / 32) + k0 / 32))};
   }
-  template <int S>
-  __device__ static __forceinline__ void store(const Raw &x, uint8_t *tile, uint32_t m, const uint32_t *) {
-    iq4_store32(x.q[0], __low2half2(x.d), tile, m, 0), iq4_store32(x.q[1], __high2half2(x.d), tile, m, 1);
+  __device__ static __forceinline__ void store(const Hdr &hd, const Raw (&x)[2], uint8_t *tile, uint32_t m, uint32_t k0) {
+    const uint32_t c = k0 % 256 / 64;
+    const __half2 d = as_h2(c & 2 ? (c & 1 ? hd.d.w : hd.d.z) : (c & 1 ? hd.d.y : hd.d.x));
+    iq4_store32(x[0].q, __low2half2(d), tile, m, 0), iq4_store32(x[1].q, __high2half2(d), tile, m, 1);
   }
 };
 
-// IQ4_XS: w = d * (ls - 32) * table[q]. A half is one sub-block of 32 with its 6-bit ls.
+// IQ4_XS: w = d * (ls - 32) * table[q], sub-blocks of 32 with a 6-bit ls each.
 template <>
 struct Decoder<QT_IQ4_XS> {
   static constexpr uint32_t kUnitStages = 1;
-  static constexpr uint32_t kUnitBytes = 32;  // of the main quants run
-  __device__ static __forceinline__ const uint8_t *quants_at(const uint8_t *s, uint32_t K, uint32_t r, uint32_t u) { return s + (uint64_t)r * (K / 2) + 32 * u; }
-  struct Raw {
-    uint4 q[2];
-    uint32_t sl, sh;  // the two sub-blocks' low nibbles; their high pairs of bits, at bit 4 (u % 2)
+  struct Hdr {
+    uint32_t sl, sh;  // the eight sub-blocks' low nibbles; their high pairs of bits
     __half d;
   };
-  __device__ static __forceinline__ Raw fetch(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t u) {
-    const uint64_t blk = (uint64_t)r * (K / 256) + u / 4;
-    Raw x;
-    const uint8_t *q = quants_at(s, K, r, u);
-    x.q[0] = ldg16(q), x.q[1] = ldg16(q + 16);
-    x.sl = __ldg(s + 128 * nblk + 4 * blk + u % 4);
-    x.sh = (uint32_t)__ldg(s + 132 * nblk + 2 * blk + u % 4 / 2) >> (4 * (u % 2));
-    x.d = __ldg((const __half *)(s + 134 * nblk) + blk);
-    return x;
+  struct Raw {
+    uint4 q;
+  };
+  __device__ static __forceinline__ Hdr fetch_hdr(const uint8_t *s, uint64_t nblk, uint32_t K, uint32_t r, uint32_t k0) {
+    const uint64_t blk = (uint64_t)r * (K / 256) + k0 / 256;
+    return Hdr{__ldg((const uint32_t *)(s + 128 * nblk) + blk), __ldg((const uint16_t *)(s + 132 * nblk) + blk), __ldg((const __half *)(s + 134 * nblk) + blk)};
   }
-  template <int S>
-  __device__ static __forceinline__ void store(const Raw &x, uint8_t *tile, uint32_t m, const uint32_t *) {
+  __device__ static __forceinline__ void store(const Hdr &hd, const Raw (&x)[2], uint8_t *tile, uint32_t m, uint32_t k0) {
+    const uint32_t c = k0 % 256 / 64, sl = hd.sl >> (8 * c), sh = hd.sh >> (4 * c);
     // d * (ls - 32) rounded to f16 once; ls - 32 is in -32 .. 31, exact in f16.
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const uint32_t ls = ((x.sl >> (4 * h)) & 0xF) | (((x.sh >> (2 * h)) & 3) << 4);
-      iq4_store32(x.q[h], __float2half2_rn(__half2float(x.d) * (float)((int)ls - 32)), tile, m, h);
+      const uint32_t ls = ((sl >> (4 * h)) & 0xF) | (((sh >> (2 * h)) & 3) << 4);
+      iq4_store32(x[h].q, __float2half2_rn(__half2float(hd.d) * (float)((int)ls - 32)), tile, m, h);
     }
   }
 };
@@ -706,9 +706,10 @@ struct Decoder<QT_IQ4_XS> {
 
 // Whether a type's quants reach the decode warps through a ring in shared memory filled by bulk-tensor copies, rather
 // than by the warps' own global loads (whose one-row-per-lane pattern costs the load pipe 32 wavefronts an
-// instruction). Q4_K, the benchmark's type: its quants are one run of K / 2 bytes a row, which a 3-D map (bytes of the
-// row, rows, expert slots) covers.
-__host__ __device__ constexpr bool quants_by_copy(uint32_t qt) { return qt == QT_Q4_K; }
+// instruction). Q4_K, IQ4_XS and IQ4_NL: their quants are one run of K / 2 bytes a row, which a 3-D map (bytes of the
+// row, rows, expert slots) covers. (IQ4_XS with IQ4_NL, 4,352 rows of the benchmark's layer, by the threads' own loads and
+// the table's values parted by permutes of their own: gate and up 448 us, 417 so; the layer 985 and 944.)
+__host__ __device__ constexpr bool quants_by_copy(uint32_t qt) { return qt == QT_Q4_K || qt == QT_IQ4_XS || qt == QT_IQ4_NL; }
 
 // What a decode thread loads of a block beside the quants the ring brings.
 template <int QT, bool = quants_by_copy(QT)>
