@@ -31,8 +31,10 @@ constexpr uint32_t kTileM = 128;   // weight rows a CTA takes
 constexpr uint32_t kTileN = 256;   // activation rows at most
 constexpr uint32_t kTileK = 64;    // values of the contraction a stage holds
 constexpr uint32_t kTileDecoders = 512;  // threads that decode weights: 16 warps, enough of them to hide their loads' latency
-constexpr uint32_t kTileEpilogue = 128;  // threads that turn accumulators into results: a warp per quarter of the weight rows
-constexpr uint32_t kTileThreads = kTileDecoders + kTileEpilogue + 96;  // and the rows' copy warp, the MMA warp, the quants' copy warp
+// Threads that turn accumulators into results: a warp per quarter of the weight rows, two for the down product, whose items are
+// a quarter as long as gate's and up's for twice the results (32,768 rows, the layer: 3,715 us with one, 3,461 with two).
+__host__ __device__ constexpr uint32_t tile_epilogue(int nmat) { return nmat == 1 ? 256 : 128; }
+__host__ __device__ constexpr uint32_t tile_threads(int nmat) { return kTileDecoders + tile_epilogue(nmat) + 96; }  // and the rows' copy warp, the MMA warp, the quants' copy warp
 constexpr uint32_t kTileBoxRows = 64;    // rows one bulk-tensor copy brings (the tensor map's box: 64 values x 64 rows)
 
 struct ExpertTilesArgs {
@@ -103,6 +105,29 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
       return false;
     }
   }
+}
+// mbar_wait by a whole warp: every lane leaves it together, with the same answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t *abort, uint32_t *error) {
+  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+  const long long t0 = clock64();
+  for (;;) {
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity, 20000))) return true;
+    const bool late = clock64() - t0 > 2000000000ll;
+    if (__any_sync(0xffffffffu, late || *abort)) {
+      if (late && !*abort) *abort = 1, atomicExch(error, 1u);
+      return false;
+    }
+  }
+}
+// One lane of the warp, the same one every time.
+__device__ __forceinline__ uint32_t elect_leader() {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(r));
+  return r;
 }
 // One arrival that also tells the barrier to expect `bytes` of bulk copies before its phase completes.
 __device__ __forceinline__ void mbar_arrive_expect(uint32_t bar, uint32_t bytes) {
@@ -179,19 +204,28 @@ __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncol
 __device__ __forceinline__ void tmem_free_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
+// MMAs and commits are issued by one lane, `leader`, in code that the whole warp runs together: the instruction takes its
+// descriptors from uniform registers, which the compiler can keep them in only where no lane goes its own way. (In a branch
+// for lane 0 each was worked out in that lane's registers and moved over, some twenty instructions an MMA at the ten clocks
+// each that a scheduler's six warps leave: 173 clocks an MMA of 96 rows and 200 of 256, for 48 and 128 of the tensor core's.)
 // The pair's commit: one arrival on the barrier at this place in each CTA of the mask.
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar, uint32_t cta_mask) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)cta_mask)
-               : "memory");
+__device__ __forceinline__ void mma_commit_pair(uint32_t leader, uint32_t bar, uint32_t cta_mask) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+      ::"r"(bar), "h"((uint16_t)cta_mask), "r"(leader)
+      : "memory");
 }
 // D[tmem of both CTAs] (+)= A[256 rows: 128 in each CTA's shared memory] * B[n rows: half in each CTA's]^T, issued by
 // one thread of the pair's first CTA; the descriptors name the same places in both.
-__device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16_pair(uint32_t leader, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(leader)
       : "memory");
 }
 
@@ -207,16 +241,22 @@ __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
 __device__ __forceinline__ void tmem_free(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ void mma_commit(uint32_t leader, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(bar), "r"(leader)
+      : "memory");
 }
 // D[tmem] (+)= A[smem] * B[smem]^T, f16 operands, f32 accumulate, M 128, K 16.
-__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16(uint32_t leader, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *v) {
@@ -787,7 +827,7 @@ __device__ __forceinline__ ItemTile item_tile(const ExpertTilesArgs &a, uint32_t
 // NMAT 2: out = swiglu(gate x, up x); NMAT 1: out = down h. Persistent: the grid is one CTA per SM (fewer when there is
 // less work), single or in pairs (PAIR, below); a unit (a CTA or a pair) takes the work items dealt to it round by
 // round; item i is weight-row tile (or pair of tiles) i % RTU of big tile i / RTU, so neighbouring units share a tile's
-// activations in L2. Five roles: 16 decode warps (quants to f16 weights in shared memory), 4 epilogue warps
+// activations in L2. Five roles: 16 decode warps (quants to f16 weights in shared memory), 4 or 8 epilogue warps
 // (accumulators to the result), a warp whose first lane issues the bulk-tensor copies of the rows' activations (the
 // whole warp when the rows are gathered by index), the warp that owns tensor memory and whose first lane issues the
 // MMAs, and a warp whose first lane issues the copies of the quants for types that take them through the ring. A warp
@@ -799,7 +839,7 @@ __device__ __forceinline__ ItemTile item_tile(const ExpertTilesArgs &a, uint32_t
 // wait for its epilogue, and to keep that short the decode warps join the epilogue warps for it.
 // Dynamic shared memory TileSmem::kBytes.
 template <int QT, int NMAT, bool PAIR>
-__global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_constant__ ExpertTilesArgs a,
+__global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __grid_constant__ ExpertTilesArgs a,
                                                                   const __grid_constant__ CUtensorMap act_map,
                                                                   const uint32_t *__restrict__ grid_global) {
   using namespace tc;
@@ -807,7 +847,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
   using Dec = Decoder<QT>;
   using Raw = typename Dec::Raw;
   constexpr uint32_t S = SM::kStages, kCols = 512;
-  constexpr uint32_t kDW = kTileDecoders / 32, kEW = kTileEpilogue / 32, kCopyWarp = kDW + kEW, kMmaWarp = kCopyWarp + 1, kQuantWarp = kMmaWarp + 1;
+  constexpr uint32_t kDW = kTileDecoders / 32, kEW = tile_epilogue(NMAT) / 32, kCopyWarp = kDW + kEW, kMmaWarp = kCopyWarp + 1, kQuantWarp = kMmaWarp + 1;
   // A decode thread takes a whole row of a stage, 64 values as two halves of 32, so that what a stage costs a thread
   // beside the arithmetic (the barrier round trip, the addresses, the block's scales) is paid once per 64 values. A
   // stage's NMAT * 128 rows are one group of threads; the 512 decode threads form 2 groups (two matrices) or 4 (one),
@@ -828,6 +868,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
   const uint32_t unit = PAIR ? blockIdx.x / 2 : blockIdx.x, nunits = PAIR ? gridDim.x / 2 : gridDim.x;
   const uint32_t RTU = PAIR ? RT / 2 : RT;  // a big tile's items
   const uint32_t nitems = ntiles * RTU;
+  // Item / RTU without a division: exact while item * RTU stays below 2^32.
+  const uint32_t magic = RTU > 1 ? 0xFFFFFFFFu / RTU + 1 : 0;
+  auto tile_of_item = [&](uint32_t item) { return RTU > 1 ? __umulhi(item, magic) : item; };
   if (unit >= nitems) return;  // both CTAs of a pair alike
   const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   uint64_t *bars = (uint64_t *)(smem + SM::kBarriers);
@@ -883,7 +926,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
       mbar_arrive(own_bar);
   };
   // The weight rows of an item that this CTA decodes and drains.
-  auto item_rows0 = [&](uint32_t item) { return ((item % RTU) * (PAIR ? 2u : 1u) + rank) * kTileM; };
+  auto item_rows0 = [&](uint32_t item) { return ((item - tile_of_item(item) * RTU) * (PAIR ? 2u : 1u) + rank) * kTileM; };
 
   // CTA b's item of round r: the items come expert by expert for the experts with full tiles, then the short tiles of
   // the others by falling row count, and the rounds deal them boustrophedon (b, then G - 1 - b, ...), so that every CTA
@@ -936,14 +979,14 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
       }
       const uint64_t at = (uint64_t)(t.start + W * c) * a.out_stride + r;
       if (a.out_f16) {
-        __half *p = (__half *)a.out + at;
-        if (left >= (uint32_t)W) {
+        // Two lanes that hold neighbouring weight rows share out two result rows: the even one stores both values of the first,
+        // the odd one of the second, four bytes each.
+        const uint32_t odd = lane & 1, sel = odd ? 0x3276u : 0x5410u;
+        uint32_t *p = (uint32_t *)((__half *)a.out + at + (uint64_t)odd * a.out_stride - odd);
 #pragma unroll
-          for (int j = 0; j < W; j++) p[(uint64_t)j * a.out_stride] = __float2half_rn(v[j]);
-        } else {
-#pragma unroll
-          for (int j = 0; j < W; j++)
-            if ((uint32_t)j < left) p[(uint64_t)j * a.out_stride] = __float2half_rn(v[j]);
+        for (int j = 0; j < W; j += 2, p += a.out_stride) {
+          const uint32_t mine = as_u32(__floats2half2_rn(v[j], v[j + 1])), theirs = __shfl_xor_sync(0xffffffffu, mine, 1);
+          if (left >= (uint32_t)W || j + odd < left) *p = __byte_perm(mine, theirs, sel);
         }
       } else {
         float *p = (float *)a.out + at;
@@ -989,19 +1032,19 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
     if constexpr (quants_by_copy(QT)) {
       const uint32_t i0 = item_at(0);
       if (i0 != kNoItem && first < KT) {
-        const ItemTile t0 = item_tile(a, i0 / RTU);
+        const ItemTile t0 = item_tile(a, tile_of_item(i0));
         hdr_ahead = Dec::fetch_hdr((mat == 0 ? a.w0 : a.w1) + (uint64_t)t0.slot * a.slice_bytes, nblk, K, item_rows0(i0) + m,
                                    (first * kTileK) & ~255u);
       }
     }
     for (uint32_t rnd = 0, item; (item = item_at(rnd)) != kNoItem && ok; rnd++, li++) {
-      const ItemTile t = item_tile(a, item / RTU);
+      const ItemTile t = item_tile(a, tile_of_item(item));
       const uint32_t r0 = item_rows0(item);
       const uint8_t *wm = (mat == 0 ? a.w0 : a.w1) + (uint64_t)t.slot * a.slice_bytes;
       // The next item's weights and rows, known early: its first header is asked for at this item's last stage.
       const uint32_t item_after = quants_by_copy(QT) ? item_at(rnd + 1) : kNoItem;
       ItemTile t_after{0, 0, 0};
-      if (item_after != kNoItem) t_after = item_tile(a, item_after / RTU);
+      if (item_after != kNoItem) t_after = item_tile(a, tile_of_item(item_after));
       auto stage_begin = [&](uint32_t it, uint32_t &s) {
         const uint32_t g = li * KT + it, use_s = g / S;
         s = g % S;
@@ -1090,7 +1133,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
         // The first lines of a row's quants are asked for an item ahead, so that an item does not begin by waiting for HBM.
         const uint32_t item_next = item_at(rnd + 1);
         if (first == 0 && item_next != kNoItem) {
-          const ItemTile tn = item_tile(a, item_next / RTU);
+          const ItemTile tn = item_tile(a, tile_of_item(item_next));
           const uint8_t *wn = (mat == 0 ? a.w0 : a.w1) + (uint64_t)tn.slot * a.slice_bytes;
           for (uint32_t u = 0; u < units && u < 3 * kDecGroups; u += 128 / Dec::kUnitBytes) prefetch_l2(Dec::quants_at(wn, K, item_rows0(item_next) + m, u));
         }
@@ -1124,7 +1167,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
     // Epilogue warps: warp w reads TMEM lanes 32 (w % 4) .., its quarter of the weight rows.
     uint32_t li = 0;
     for (uint32_t rnd = 0, item; (item = item_at(rnd)) != kNoItem && ok; rnd++, li++) {
-      const ItemTile t = item_tile(a, item / RTU);
+      const ItemTile t = item_tile(a, tile_of_item(item));
       const uint32_t r0 = item_rows0(item);
       if (is_wide(t.count)) {
         if (ok) ok = mbar_wait(acc_full(0), use0 & 1, abort, a.error);
@@ -1141,7 +1184,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
         ok = mbar_wait(acc_full(b), use_of(b) & 1, abort, a.error);
         if (!ok) break;
         tc_fence_after();
-        drain(t, r0, b * kTileN, b * kTileN + kTileN / 2, 0, 1);
+        drain(t, r0, b * kTileN, b * kTileN + kTileN / 2, (warp - kDW) / 4, kEW / 4);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) arrive_lead(acc_empty_lead(b), acc_empty(b));
@@ -1157,7 +1200,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
       constexpr uint32_t kPerLane = PAIR ? 1 : 2;
       uint32_t li = 0;
       for (uint32_t rnd = 0, item; (item = item_at(rnd)) != kNoItem && ok; rnd++, li++) {
-        const ItemTile t = item_tile(a, item / RTU);
+        const ItemTile t = item_tile(a, tile_of_item(item));
         const uint32_t half = ((t.count + 15) & ~15u) / 2;
         const uint32_t mine = PAIR ? half : t.count, first_row = PAIR ? rank * half : 0;
         const uint32_t ncopies = (mine + 3) / 4;
@@ -1205,7 +1248,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
       // run past the tile's rows into the next expert's, or past the tensor (zeros): those columns of the result are dropped.
       uint32_t li = 0;
       for (uint32_t rnd = 0, item; (item = item_at(rnd)) != kNoItem && ok; rnd++, li++) {
-        const ItemTile t = item_tile(a, item / RTU);
+        const ItemTile t = item_tile(a, tile_of_item(item));
         // A CTA of a pair brings its half of the rows the instruction takes (the rows rounded up to 16): the first
         // CTA the first half.
         const uint32_t half = ((t.count + 15) & ~15u) / 2;
@@ -1240,7 +1283,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
     // as the decode warps have read the slot's last contents; it runs ahead of the stages by the ring's two slots.
     uint32_t li = 0;
     for (uint32_t rnd = 0, item; (item = item_at(rnd)) != kNoItem && ok; rnd++, li++) {
-      const ItemTile t = item_tile(a, item / RTU);
+      const ItemTile t = item_tile(a, tile_of_item(item));
       for (uint32_t j = 0; j < KT / kDecGroups && ok; j++) {
         const uint32_t qn = li * (KT / kDecGroups) + j, qb = qn % SM::kQSlots, use_q = qn / SM::kQSlots;
         if (use_q > 0) ok = mbar_wait(q_empty(qb), (use_q - 1) & 1, abort, a.error);
@@ -1257,29 +1300,31 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
       }
     }
     }
-  } else if (lane == 0 && rank == 0) {
-    // The MMA thread (of a pair's first CTA): per stage, four K steps of 16 for each matrix; the commit frees the stage
-    // when they are done, in both CTAs of a pair.
-    auto wait_lead = [&](uint32_t bar, uint32_t parity) { return mbar_wait(bar, parity, abort, a.error); };
+  } else if (rank == 0) {
+    // The MMA warp (of a pair's first CTA), one lane of which issues: per stage, four K steps of 16 for each matrix; the
+    // commit frees the stage when they are done, in both CTAs of a pair.
+    const uint32_t leader = elect_leader();
+    auto wait_lead = [&](uint32_t bar, uint32_t parity) { return mbar_wait_warp(bar, parity, abort, a.error); };
     auto mma = [&](uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
       if constexpr (PAIR)
-        mma_f16_pair(d, da, db, idesc, acc);
+        mma_f16_pair(leader, d, da, db, idesc, acc);
       else
-        mma_f16(d, da, db, idesc, acc);
+        mma_f16(leader, d, da, db, idesc, acc);
     };
     auto commit = [&](uint32_t bar) {
       if constexpr (PAIR)
-        mma_commit_pair(bar, 3);
+        mma_commit_pair(leader, bar, 3);
       else
-        mma_commit(bar);
+        mma_commit(leader, bar);
     };
-    uint32_t li = 0;
+    const uint32_t stages = smem_u32(smem);
+    uint32_t s = 0, phase = 0;
     bool after_wide = false;
-    for (uint32_t rnd = 0, item; (item = item_at(rnd)) != kNoItem && ok; rnd++, li++) {
-      const ItemTile t = item_tile(a, item / RTU);
+    for (uint32_t rnd = 0, item; (item = item_at(rnd)) != kNoItem && ok; rnd++) {
+      const ItemTile t = item_tile(a, tile_of_item(item));
       const uint32_t idesc = instr_desc((t.count + 15) & ~15u, PAIR ? 2 * kTileM : kTileM);
       const bool wide = is_wide(t.count);
-      const uint32_t b = next_buf, colg = wide ? 0 : b * kTileN, colu = wide ? kTileN : colg + kTileN / 2;
+      const uint32_t b = next_buf, colg = tmem_base + (wide ? 0 : b * kTileN), colu = colg + (wide ? kTileN : kTileN / 2);
       // The buffers this item writes must have been read: by the epilogue warps, and after a two-buffer item by the
       // decode warps too.
       if (after_wide) ok = wait_lead(acc_empty_wide, (wides - 1) & 1);
@@ -1287,18 +1332,18 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_expert_tiles(const __grid_c
       for (uint32_t bb = 0; bb < 2 && ok; bb++)
         if ((wide || bb == b) && use_of(bb) > 0) ok = wait_lead(acc_empty(bb), (use_of(bb) - 1) & 1);
       for (uint32_t it = 0; it < KT && ok; it++) {
-        const uint32_t g = li * KT + it, s = g % S;
-        ok = wait_lead(full_bar(s), (g / S) & 1);
+        ok = wait_lead(full_bar(s), phase);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t stage = smem_u32(smem + s * SM::kStageBytes), xt = stage + NMAT * SM::kWBytes;
+        const uint32_t stage = stages + s * SM::kStageBytes, xt = stage + NMAT * SM::kWBytes;
 #pragma unroll
         for (uint32_t k = 0; k < kTileK / 16; k++) {
           const uint64_t db = smem_desc_sw128(xt + 32 * k);
-          mma(tmem_base + colg, smem_desc(stage + 2 * k * kLbo), db, idesc, (it | k) != 0);
-          if constexpr (NMAT == 2) mma(tmem_base + colu, smem_desc(stage + SM::kWBytes + 2 * k * kLbo), db, idesc, (it | k) != 0);
+          mma(colg, smem_desc(stage + 2 * k * kLbo), db, idesc, (it | k) != 0);
+          if constexpr (NMAT == 2) mma(colu, smem_desc(stage + SM::kWBytes + 2 * k * kLbo), db, idesc, (it | k) != 0);
         }
         commit(empty_bar(s));
+        if (++s == S) s = 0, phase ^= 1;
       }
       if (!ok) break;
       if (wide) {

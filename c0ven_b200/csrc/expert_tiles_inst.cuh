@@ -11,7 +11,7 @@ namespace moe {
 
 // Pairs of CTAs the GPU runs at once for kernel (one CTA an SM, so at most one pair a TPC), asked once per device.
 template <class Kernel>
-static cudaError_t max_pairs(Kernel kernel, size_t smem, int device, uint32_t &pairs) {
+static cudaError_t max_pairs(Kernel kernel, uint32_t threads, size_t smem, int device, uint32_t &pairs) {
   static std::atomic<uint32_t> known[64];
   if (device < 0 || device >= 64) return cudaErrorInvalidValue;
   pairs = known[device].load(std::memory_order_acquire);
@@ -20,7 +20,7 @@ static cudaError_t max_pairs(Kernel kernel, size_t smem, int device, uint32_t &p
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeClusterDimension;
   at.val.clusterDim.x = 2, at.val.clusterDim.y = 1, at.val.clusterDim.z = 1;
-  cfg.gridDim = dim3(2), cfg.blockDim = dim3(kTileThreads), cfg.dynamicSmemBytes = smem, cfg.attrs = &at, cfg.numAttrs = 1;
+  cfg.gridDim = dim3(2), cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem, cfg.attrs = &at, cfg.numAttrs = 1;
   int n = 0;
   const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
   if (e != cudaSuccess) return e;
@@ -43,14 +43,14 @@ cudaError_t launch_expert_tiles(const ExpertTilesArgs &a, const CUtensorMap &act
     cudaError_t e = ensure_dynamic_smem(kernel, smem, attr_done, ctx.device);
     if (e != cudaSuccess) return e;
     uint32_t pairs = 0;
-    e = max_pairs(kernel, smem, ctx.device, pairs);
+    e = max_pairs(kernel, tile_threads(NMAT), smem, ctx.device, pairs);
     if (e != cudaSuccess) return e;
     const uint64_t items = (uint64_t)max_tiles * (RT / 2);
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = 2, at.val.clusterDim.y = 1, at.val.clusterDim.z = 1;
-    cfg.gridDim = dim3(2 * (unsigned)std::min<uint64_t>(items, pairs)), cfg.blockDim = dim3(kTileThreads);
+    cfg.gridDim = dim3(2 * (unsigned)std::min<uint64_t>(items, pairs)), cfg.blockDim = dim3(tile_threads(NMAT));
     cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = &at, cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, a, act_map, grid_global);
   }
@@ -60,7 +60,7 @@ cudaError_t launch_expert_tiles(const ExpertTilesArgs &a, const CUtensorMap &act
   const cudaError_t e = ensure_dynamic_smem(kernel, smem, attr_done, ctx.device);
   if (e != cudaSuccess) return e;
   const uint64_t items = (uint64_t)max_tiles * RT;
-  kernel<<<(unsigned)std::min<uint64_t>(items, (uint64_t)ctx.sms), kTileThreads, smem, st>>>(a, act_map, grid_global);
+  kernel<<<(unsigned)std::min<uint64_t>(items, (uint64_t)ctx.sms), tile_threads(NMAT), smem, st>>>(a, act_map, grid_global);
   return cudaGetLastError();
 }
 

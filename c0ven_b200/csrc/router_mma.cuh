@@ -98,31 +98,29 @@ static __global__ void __launch_bounds__(kRouterThreads, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | ((ne_tile >> 3) << 17) | ((kRouterTileRows >> 4) << 24);
-      uint32_t li = 0;
-      for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x, li++) {
-        const uint32_t b = li & 1, use_b = li / 2;
-        if (use_b > 0) ok = mbar_wait(acc_empty(b), (use_b - 1) & 1, abort, a.error);
-        for (uint32_t it = 0; it < KT && ok; it++) {
-          const uint32_t g = li * KT + it, s = g % S;
-          ok = mbar_wait(full_bar(s), (g / S) & 1, abort, a.error);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t st = smem_u32(smem + s * kRouterStageBytes);
-          const uint32_t xh = st, xl = st + kRouterABytes, wh = st + 2 * kRouterABytes, wl = wh + kRouterBBytes;
-          const uint32_t d = tmem_base + b * kRouterTileExperts;
+    // The MMA warp, one lane of which issues (tc::mma_f16).
+    const uint32_t leader = elect_leader(), idesc = (1u << 4) | ((ne_tile >> 3) << 17) | ((kRouterTileRows >> 4) << 24), stages = smem_u32(smem);
+    uint32_t li = 0, s = 0, phase = 0;
+    for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x, li++) {
+      const uint32_t b = li & 1, use_b = li / 2;
+      if (use_b > 0) ok = mbar_wait_warp(acc_empty(b), (use_b - 1) & 1, abort, a.error);
+      for (uint32_t it = 0; it < KT && ok; it++) {
+        ok = mbar_wait_warp(full_bar(s), phase, abort, a.error);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t xh = stages + s * kRouterStageBytes, xl = xh + kRouterABytes, wh = xl + kRouterABytes, wl = wh + kRouterBBytes;
+        const uint32_t d = tmem_base + b * kRouterTileExperts;
 #pragma unroll
-          for (uint32_t k = 0; k < kRouterTileK / 16; k++) {
-            const uint64_t dxh = smem_desc_sw128(xh + 32 * k), dwh = smem_desc_sw128(wh + 32 * k);
-            mma_f16(d, dxh, dwh, idesc, (it | k) != 0);
-            mma_f16(d, dxh, smem_desc_sw128(wl + 32 * k), idesc, 1);
-            mma_f16(d, smem_desc_sw128(xl + 32 * k), dwh, idesc, 1);
-          }
-          mma_commit(empty_bar(s));
+        for (uint32_t k = 0; k < kRouterTileK / 16; k++) {
+          const uint64_t dxh = smem_desc_sw128(xh + 32 * k), dwh = smem_desc_sw128(wh + 32 * k);
+          mma_f16(leader, d, dxh, dwh, idesc, (it | k) != 0);
+          mma_f16(leader, d, dxh, smem_desc_sw128(wl + 32 * k), idesc, 1);
+          mma_f16(leader, d, smem_desc_sw128(xl + 32 * k), dwh, idesc, 1);
         }
-        if (ok) mma_commit(acc_full(b));
+        mma_commit(leader, empty_bar(s));
+        if (++s == S) s = 0, phase ^= 1;
       }
+      if (ok) mma_commit(leader, acc_full(b));
     }
   } else {
     // Epilogue warps: warp w reads TMEM lanes 32 (w % 4) .., a quarter of the item's rows; a lane is a row, and writes
