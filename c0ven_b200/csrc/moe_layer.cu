@@ -544,17 +544,22 @@ uint32_t few_rows_for(const moe_layer *l, uint64_t R, uint32_t nexp) {
 }
 
 // Whether groups of at most M rows, in a call of R expert rows, go to the few-rows kernel: with more than two rows its eight columns are worth their
-// instructions whatever the type (200 rows of IQ3_S: 1085 -> 491 us); with one or two, where the integer-dot kernel's
-// decode is long and runs once a row (32 rows, even routing: Q4_K 309 -> 215 us, Q4_K with Q6_K 326 -> 251, IQ4_XS with
-// IQ4_NL 315 -> 276), not where it is nothing or a codebook's (Q8_0 246 -> 256, IQ3_S 272 -> 305, IQ2_S 281 -> 293), nor in
-// steps of so few rows that the kernel's warps, of 16 weight rows, are few (5 rows over 256 experts in Q4_K and Q6_K: 51 ->
-// 61 us for the experts' stage; 40 rows 92 either way). Never
+// instructions whatever the type (200 rows of IQ3_S: 1085 -> 491 us); with one or two it depends on how much work there is to
+// spread over its warps, of 16 weight rows, and on what it replaces. From 32 assignments on where the integer-dot kernel's decode is
+// long and runs once a row (32 rows, even routing: Q4_K 309 -> 168 us, IQ4_XS with IQ4_NL 315 -> 236) or where it finds a row's
+// units at run time (14 rows of 2,560 values: Q8_0 219 -> 152, IQ3_S 242 -> 160; 12 rows of 1,024 in IQ3_S 68 -> 57). Of the
+// rest from 200 on (Q8_0 9 rows 123 and 137, 20 rows 182 and 178, 50 rows 297 and 264; IQ2_S with Q2_0 32 rows 262 and 221), but not
+// IQ3_S, whose two kernels decode at the same rate (13 rows 141 and 160, 32 rows 246 and 248). Never
 // in a layer kept off the tensor cores (MOE_FLAG_NO_TENSOR), whose products are the integer-dot kernels' whatever the rows.
 bool groups_take_mma(const moe_layer *l, int M, uint64_t R) {
-  if (!l->can_tensor) return false;
+  if (!l->can_tensor || M < 2) return false;
   const uint32_t g = l->cfg.gate_type, d = l->cfg.down_type;
+  if (!mma_takes(g, l->E, kGroupMax) || !mma_takes(d, l->F, kGroupMax)) return false;
   auto heavy = [](uint32_t t) { return t == QT_Q4_K || t == QT_Q6_K || t == QT_IQ4_XS || t == QT_IQ4_NL; };
-  return (M > 2 || (M == 2 && R >= 32 && heavy(g) && heavy(d))) && mma_takes(g, l->E, kGroupMax) && mma_takes(d, l->F, kGroupMax);
+  auto specialised = [](uint32_t K) { return K == 2048 || K == 512 || K == 256; };  // launch_shape
+  if (M > 2) return true;
+  if ((heavy(g) && heavy(d)) || !specialised(l->E) || !specialised(l->F)) return R >= 32;
+  return R >= 200 && g != QT_IQ3_S;
 }
 
 // Shared memory of the exact router's CTA: tm rows of x, each in padded pieces.
