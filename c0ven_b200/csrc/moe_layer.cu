@@ -433,25 +433,37 @@ void create(moe_layer *l, const moe_layer_config &c, const moe_layer_weights &w)
 //
 // The bound. An approximate logit differs from the fp32 sum in the exact order by (a) the dropped lo * lo products and
 // the rounding of the lo parts, at most 2^-20 of sum |x_i w_i|; (b) the roundings of the accumulations, each taken as
-// at most 2^-23 of the running sum, one per MMA of 16 values and three MMAs a step: 3 E / 16 of them; (c) the exact
-// order's own roundings: chains of E / 8 fused multiply-adds at 2^-24 of the running sum each, then eight additions, and
-// the up to three that put a split product's pieces together.
-// sum |x_i w_i| <= |x| |w_e| (Cauchy-Schwarz), so eps = eps_rel |x| max_e |w_e| with eps_rel = (3 E / 16 + E / 8 + 16) 2^-23
-// (2^-13.6 at E = 2048) covers all three in the worst case, where every rounding falls the same way; measured errors
-// are some hundred times smaller, and the GPU tests hold them under a quarter of the bound. The bias adds one rounding
-// of the biased logit, covered by eps_abs.
+// at most 2^-23 of the running sum, one per MMA of 16 values and three MMAs a step; (c) the exact order's own roundings:
+// eight chains of E / 8 fused multiply-adds at 2^-24 of the running sum each, then eight additions, and the up to three that put
+// a split product's pieces together.
+// sum |x_i w_i| <= |x| |w_e| (Cauchy-Schwarz), and a running sum over the first i values is at most |x| |w_e's first i values|,
+// whose norms are known here: (b) is at most 3 * 2^-23 |x| times their sum over the E / 16 steps, (c)'s chains at most
+// 2^-24 |x| times the root of the sum over the chains of (the sum of the chain's prefix norms) squared, whatever way the row's
+// norm falls to the chains. So eps = eps_rel |x| with eps_rel the largest over the experts of 2^-23 (3 * steps + chains / 2 +
+// 16 |w_e|), a hundredth more for the roundings of roundings, covers all three in the worst case, where every rounding falls the
+// same way (some 2^-14.5 |w_e| at E = 2048; with |w_e| for every prefix it was 2^-13.6, and the top-k, which then recomputed more
+// logits and copied four rows whatever their number, took 193 us for 32,768 rows, 170 now); measured errors are some fifty times
+// smaller, and the GPU tests hold them under a quarter of the bound. The bias adds one rounding of the biased logit, covered by eps_abs.
 void setup_router_tensor(moe_layer *l, const float *router, const float *bias, cudaStream_t st) {
   const uint32_t E = l->E, NE = l->NE, T = l->Tmax;
   const uint64_t wrows = std::max<uint32_t>(NE, kRouterTileExperts), xrows = std::max<uint32_t>(T, kRouterTileRows);
   std::vector<__half> hi(wrows * E, __float2half_rn(0.0f)), lo(wrows * E, __float2half_rn(0.0f));
   std::vector<float> unscale(NE, 1.0f);
-  double wn_max = 0.0;
+  double eps = 0.0;
   for (uint32_t e = 0; e < NE; e++) {
     const float *w = router + (size_t)e * E;
     float m = 0.0f;
-    double n2 = 0.0;
-    for (uint32_t i = 0; i < E; i++) m = std::max(m, std::fabs(w[i])), n2 += (double)w[i] * w[i];
-    wn_max = std::max(wn_max, std::sqrt(n2));
+    double n2 = 0.0, steps = 0.0, chains2 = 0.0;
+    for (uint32_t p = 0; p < kRouterPieces; p++) {
+      double piece2 = 0.0, chain = 0.0;
+      for (uint32_t i = p * (E / kRouterPieces); i < (p + 1) * (E / kRouterPieces); i++) {
+        m = std::max(m, std::fabs(w[i])), n2 += (double)w[i] * w[i], piece2 += (double)w[i] * w[i];
+        chain += std::sqrt(piece2);
+        if (i % 16 == 15) steps += std::sqrt(n2);
+      }
+      chains2 += chain * chain;
+    }
+    eps = std::max(eps, 1.01 * (3.0 * steps + 0.5 * std::sqrt(chains2)) + 16.0 * std::sqrt(n2));
     int ex = 0;
     if (m > 0.0f && std::isfinite(m)) std::frexp(m, &ex);
     ex = std::min(std::max(ex, -100), 100);
@@ -466,7 +478,7 @@ void setup_router_tensor(moe_layer *l, const float *router, const float *bias, c
   }
   float bias_max = 0.0f;
   for (uint32_t e = 0; bias && e < NE; e++) bias_max = std::max(bias_max, std::fabs(bias[e]));
-  l->router_eps_rel = (float)(std::ldexp(3.0 * E / 16 + E / 8 + 16, -23) * wn_max);
+  l->router_eps_rel = (float)std::ldexp(eps, -23);
   l->router_eps_abs = std::ldexp(1.0f + bias_max, -20);
   l->rw_hi.alloc(hi.size()), l->rw_lo.alloc(lo.size()), l->rw_unscale.alloc(NE);
   CUDA_OK(cudaMemcpyAsync(l->rw_hi.get(), hi.data(), hi.size() * sizeof(__half), cudaMemcpyHostToDevice, st));

@@ -85,8 +85,9 @@ constexpr uint32_t kExWarpBytes = 2 * kExBuf;            // two chunks: 11,520 b
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
 }
+// With fewer than four experts (n) only their rows are copied; the other lanes' sums are nobody's.
 __device__ __forceinline__ float exact_logits4_staged(const float *x, const float *__restrict__ W, const float *__restrict__ bias,
-                                                      uint32_t E, uint32_t e, uint32_t lane, uint8_t *buf) {
+                                                      uint32_t E, uint32_t e, uint32_t n, uint32_t lane, uint8_t *buf) {
   const uint32_t piece = E / kRouterPieces, nch = piece / kExChunk, s = lane % 8, g = lane / 8;
   const uint32_t buf32 = (uint32_t)__cvta_generic_to_shared(buf);
   // The four experts of the pass, known to every lane.
@@ -102,7 +103,8 @@ __device__ __forceinline__ float exact_logits4_staged(const float *x, const floa
       const uint32_t dst = buf32 + b * kExBuf + pc * kExPiece + j * 16;
       cp_async16(dst, x + off);
 #pragma unroll
-      for (int r = 0; r < 4; r++) cp_async16(dst + (1 + r) * kExRow, W + (uint64_t)ex[r] * E + off);
+      for (int r = 0; r < 4; r++)
+        if ((uint32_t)r < n) cp_async16(dst + (1 + r) * kExRow, W + (uint64_t)ex[r] * E + off);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -150,8 +152,8 @@ __device__ __forceinline__ float exact_logits4_staged(const float *x, const floa
 __device__ __forceinline__ void router_topk_row(uint32_t t, const float *rl, const RouterApprox &ap, const float *__restrict__ bias,
                                                 uint32_t NE, uint32_t K, int32_t *__restrict__ ids, float *__restrict__ w,
                                                 float *__restrict__ gs, uint32_t *hist, int32_t *s_ids, uint8_t *ex_buf) {
-  auto exact4 = [&](const float *xr, uint32_t e, uint32_t ln) {
-    return ex_buf ? exact_logits4_staged(xr, ap.W, bias, ap.E, e, ln, ex_buf) : exact_logits4(xr, ap.W, bias, ap.E, e, ln);
+  auto exact4 = [&](const float *xr, uint32_t e, uint32_t n, uint32_t ln) {
+    return ex_buf ? exact_logits4_staged(xr, ap.W, bias, ap.E, e, n, ln, ex_buf) : exact_logits4(xr, ap.W, bias, ap.E, e, ln);
   };
   const uint32_t lane = threadIdx.x % 32, per = NE / 32;
   uint32_t key[kMaxPerLane];
@@ -210,7 +212,7 @@ __device__ __forceinline__ void router_topk_row(uint32_t t, const float *rl, con
       // Every logit exactly, four experts a pass: for rows the approximate ones cannot serve.
       mx = -INFINITY;
       for (uint32_t e0 = 0; e0 < NE; e0 += 4) {
-        const float v = exact4(ap.x + (uint64_t)t * ap.E, e0 + lane / 8, lane);
+        const float v = exact4(ap.x + (uint64_t)t * ap.E, e0 + lane / 8, 4, lane);
 #pragma unroll
         for (int q = 0; q < 4; q++) {
           const float vq = __shfl_sync(0xffffffffu, v, 8 * q);
@@ -276,6 +278,7 @@ __device__ __forceinline__ void router_topk_row(uint32_t t, const float *rl, con
     const bool need = lane < ncand && ((lane > 0 && up - my_v <= eps2) || (lane + 1 < ncand && my_v - down <= eps2));
     uint32_t todo = __ballot_sync(0xffffffffu, need);
     while (todo) {
+      const uint32_t n = min(4u, (uint32_t)__popc(todo));
       uint32_t c[4];
 #pragma unroll
       for (int q = 0; q < 4; q++) {
@@ -284,7 +287,7 @@ __device__ __forceinline__ void router_topk_row(uint32_t t, const float *rl, con
       }
       const uint32_t g8 = lane / 8, mine = g8 == 0 ? c[0] : g8 == 1 ? c[1] : g8 == 2 ? c[2] : c[3];
       const uint32_t e = __shfl_sync(0xffffffffu, my_id, mine == 0xFFFFFFFFu ? 0 : mine);
-      const float v = exact4(ap.x + (uint64_t)t * ap.E, e, lane);
+      const float v = exact4(ap.x + (uint64_t)t * ap.E, e, n, lane);
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         const float vq = __shfl_sync(0xffffffffu, v, 8 * q);
