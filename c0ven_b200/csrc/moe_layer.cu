@@ -308,7 +308,6 @@ void check_config(const moe_layer_config &c, const moe_layer_weights &w) {
     bad("a shared expert needs its gate vector and three matrices");
 }
 
-uint32_t router_rows_cta(uint32_t T, uint32_t E);
 void setup_router_tensor(moe_layer *l, const float *router, const float *bias, cudaStream_t st);
 
 void create(moe_layer *l, const moe_layer_config &c, const moe_layer_weights &w) {
@@ -350,7 +349,7 @@ void create(moe_layer *l, const moe_layer_config &c, const moe_layer_weights &w)
     if (routed > 65535 || dense > 65535)
       throw BadArgument("max_tokens (or max_expert_rows) is too large for the integer-dot kernels' grid: lower it, or leave the tensor-core kernels on");
     // The exact router's passes over a step's rows are its grid's second extent.
-    if (!l->can_tensor && (T + router_rows_cta(T, E) - 1) / router_rows_cta(T, E) > 65535)
+    if (!l->can_tensor && (T + kRouterRows - 1) / kRouterRows > 65535)
       throw BadArgument("max_tokens is too large for the exact router's grid: lower it, or leave the tensor-core kernels on");
   }
 
@@ -574,50 +573,41 @@ bool groups_take_mma(const moe_layer *l, int M, uint64_t R) {
   return R >= 200 && g != QT_IQ3_S;
 }
 
-// Shared memory of the exact router's CTA: tm rows of x, each in padded pieces.
-size_t router_rows_smem(uint32_t tm, uint32_t E) { return (size_t)tm * kRouterPieces * (E / kRouterPieces + 4) * sizeof(float); }
-constexpr size_t kRouterRowsMaxSmem = 227 * 1024;  // what a CTA can have
-
-// Rows of x a CTA of the exact router takes. The fewer, the more CTAs share the step's multiply-adds and the shorter a lane's
-// chain of them, for one more reading of the router's 4 MB out of L2 a pass: 2 rows in steps of up to 32 (13 rows: 35 -> 12.6
-// us against 8, ncu, cold; 32 rows by fours, whose registers leave no room for sixteen loads in flight, 27); 8 in longer
-// ones, where the readings count (the layer in Q8_0, by 2 and by 8 rows: 40 rows 277 and 266 us, 48 rows 305 and 293; at
-// 32 it depends on the layer: 235 and 229 of 512 experts, 242 and 255 of 128), as long as 8 fit a CTA (7,232 values a row).
-constexpr uint32_t kRouterTwoRows = 32;
-uint32_t router_rows_cta(uint32_t T, uint32_t E) { return T == 1 ? 1 : T <= kRouterTwoRows || router_rows_smem(8, E) > kRouterRowsMaxSmem ? 2 : 8; }
-
-template <int TM, int D>
-cudaError_t launch_router_form(moe_layer *l, const float *x, uint32_t T, dim3 grid, uint32_t threads, const StepQuant &sq, cudaStream_t st) {
-  const size_t smem = router_rows_smem(TM, l->E);
-  if (smem > 48 * 1024) {
-    // Set once per device, to the most that any layer's rows take: layers of several sizes share the kernel.
-    static std::atomic<uint32_t> attr_done{0};
-    const cudaError_t e = ensure_dynamic_smem(k_router_logits_rows<TM, D>, std::min(kRouterRowsMaxSmem, router_rows_smem(TM, kRowsMaxK)), attr_done, l->cfg.device);
-    if (e != cudaSuccess) return e;
-  }
-  return launch_kernel(l->ctx.pdl, k_router_logits_rows<TM, D>, grid, dim3(threads), smem, st, x, T, l->E, l->router.get(), l->N, l->bias.get(), l->NE,
-                       l->rl.get(), sq);
-}
-
 // The exact fp32 router product of a step's rows, its x quantised by the same launch.
-void launch_router_rows(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
-  const uint32_t E = l->E, N = l->N;
-  const uint32_t tm = router_rows_cta(T, E), warps = T <= 4 ? 1 : tm == 2 ? 4 : 8;
-  const uint32_t passes = (T + tm - 1) / tm;
+template <uint32_t ROWS>
+void launch_router_form(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
+  const uint32_t E = l->E, N = l->N, passes = (T + ROWS - 1) / ROWS, router_ctas = (N + kRouterExperts - 1) / kRouterExperts;
   StepQuant sq{};
   sq.job[0] = l->xq_routed.job();
   if (l->has_shared && !l->shared_x_same) sq.job[1] = l->xq_shared.job();
   sq.nblk = (uint64_t)T * (E / 256);
-  // CTAs of eight rows: the quantisers get those SMs that the router's CTAs leave, one CTA a pass at least. With a CTA for every
-  // eight blocks they made 200 CTAs of 64 rows, and so SMs with two of the router's (42 us by ncu, cold; a rank of two
-  // routing 64 rows 86 us, 72 now; the layer in Q8_0 5 % less).
-  const uint32_t router_ctas = (N + 4 * warps - 1) / (4 * warps), most = (uint32_t)((sq.nblk + (uint64_t)warps * passes - 1) / (warps * passes));
-  sq.ctas = tm < 8 ? most : std::min(most, std::max(1u, l->sms / passes > router_ctas ? l->sms / passes - router_ctas : 1));
-  const dim3 grid(sq.ctas + router_ctas, passes);
-  const bool deep = (E / kRouterPieces) % 64 == 0;  // sixteen loads in flight a lane: a step of one row is all latency
-  auto launch = tm == 1 ? (deep ? launch_router_form<1, 16> : launch_router_form<1, 8>)
-                        : tm == 2 ? (deep ? launch_router_form<2, 16> : launch_router_form<2, 8>) : launch_router_form<8, 8>;
-  launched(l, launch(l, x, T, grid, 32 * warps, sq, st), "router logits");
+  // The quantisers get the places that the router's CTAs, two an SM, leave of one round, one CTA a pass at least.
+  const uint32_t most = (uint32_t)((sq.nblk + (uint64_t)kRouterPieces * passes - 1) / (kRouterPieces * passes)), places = 2 * l->sms / passes;
+  sq.ctas = std::min(most, places > router_ctas ? places - router_ctas : 1);
+  constexpr uint32_t smem = router_rows_smem(ROWS);
+  static std::atomic<uint32_t> attr_done{0};
+  CUDA_OK(ensure_dynamic_smem(k_router_logits_rows<ROWS>, smem, attr_done, l->cfg.device));
+  launched(l, launch_kernel(l->ctx.pdl, k_router_logits_rows<ROWS>, dim3(sq.ctas + router_ctas, passes), dim3(32 * kRouterPieces), smem, st, x, T, E,
+                            l->router.get(), N, l->bias.get(), l->NE, l->rl.get(), sq),
+           "router logits");
+}
+template <int D>
+void launch_router_one(moe_layer *l, const float *x, cudaStream_t st) {
+  const uint32_t E = l->E, N = l->N;
+  StepQuant sq{};
+  sq.job[0] = l->xq_routed.job();
+  if (l->has_shared && !l->shared_x_same) sq.job[1] = l->xq_shared.job();
+  sq.nblk = E / 256, sq.ctas = E / 256;
+  const size_t smem = (E + 4 * kRouterPieces) * sizeof(float);
+  static std::atomic<uint32_t> attr_done{0};  // set once per device, to the most that any layer's row takes
+  CUDA_OK(ensure_dynamic_smem(k_router_logits_one<D>, (kRowsMaxK + 4 * kRouterPieces) * sizeof(float), attr_done, l->cfg.device));
+  launched(l, launch_kernel(l->ctx.pdl, k_router_logits_one<D>, dim3(sq.ctas + (N + 3) / 4), dim3(32), smem, st, x, E, l->router.get(), N, l->bias.get(), l->NE,
+                            l->rl.get(), sq),
+           "router logits");
+}
+void launch_router_rows(moe_layer *l, const float *x, uint32_t T, cudaStream_t st) {
+  if (T == 1) return l->E / kRouterPieces % 64 == 0 ? launch_router_one<16>(l, x, st) : launch_router_one<8>(l, x, st);
+  T <= kRouterFewRows ? launch_router_form<kRouterFewRows>(l, x, T, st) : launch_router_form<kRouterRows>(l, x, T, st);
 }
 
 // Steps of up to this many rows take the top-k and the pack in one launch. One CTA's warps share an SM's issue slots: with

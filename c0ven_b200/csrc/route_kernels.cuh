@@ -82,9 +82,15 @@ static __global__ void __launch_bounds__(256) k_quant(const float *x, uint64_t n
 // order, the pieces then added in order, and an expert's bias last. Both kernels and the CPU oracle keep this one
 // order, so that the logits, and with them the chosen experts, agree bit for bit whatever the row count.
 
-// Few rows (up to TM per CTA pass): a warp takes 4 weight rows, 8 lanes a row, lane s taking piece s; D loads of 16 bytes
-// in flight per lane (a piece is a multiple of 4 D values: 8 always, 16 when the piece is a multiple of 64 values). A CTA
-// is 1 to 8 warps, by the step's rows (launch_router_rows).
+// A CTA takes four of the router's rows and up to ROWS rows of x: a warp a piece, its lanes the pairs of a row of x and one of the
+// router's (8 rows: a chain a lane) or a row of x each (32 rows: four chains a lane). Both come through a ring in shared memory by
+// 16-byte asynchronous copies, 16 values of every piece a stage, so that each of the router's rows is read from HBM once. What bounds
+// it is the way of x out of L2, 256 KB a CTA at 32 rows of 2,048 values, and the chains, of E / 8 multiply-adds. (A lane walking its
+// piece of a weight row itself for two rows of x a CTA, the router's 4 MB read out of L2 again for every two rows: 33 us at 32
+// rows by ncu, cold, 17.6 now; two layers of 32 rows of IQ3_S 493 us and 464, 64 rows of Q8_0 377 and 272 together with the groups'
+// other kernel, four rows of Q4_K with Q6_K 70 and 64.)
+// One row has a kernel of its own, k_router_logits_one: by the form for 8 rows, of a ring of 43 to 104 KB, which keeps the next
+// kernel's waiting CTAs off the SM, the layer in Q8_0 took 27.5 to 28.8 us, 26.7 so.
 // The step's quantisers ride along: the first sq.ctas CTAs of every grid row share out the blocks of x among their warps,
 // so that quantising x is neither a launch of its own in front of the router nor behind it. A warp takes as many blocks as
 // that leaves it.
@@ -93,48 +99,126 @@ struct StepQuant {
   uint64_t nblk;
   uint32_t ctas;    // in the grid's first extent; 0: x is quantised elsewhere
 };
-template <int TM, int D = 8>
-static __global__ void __launch_bounds__(256) k_router_logits_rows(const float *x, uint32_t T, uint32_t E,
+__device__ __forceinline__ void quantize_share(const float *x, const StepQuant &sq) {
+  wait_for_predecessors();
+  const uint32_t lane = threadIdx.x % 32, warps = blockDim.x / 32;
+  const uint64_t step = (uint64_t)gridDim.y * sq.ctas * warps;
+  for (uint64_t blk = ((uint64_t)blockIdx.y * sq.ctas + blockIdx.x) * warps + threadIdx.x / 32; blk < sq.nblk; blk += step) {
+    const float4 a = ((const float4 *)(x + blk * 256))[2 * lane], b = ((const float4 *)(x + blk * 256))[2 * lane + 1];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      if (!sq.job[j].q) continue;
+      if (sq.job[j].q8k)
+        quantize_store<true>(a, b, blk, lane, sq.job[j]);
+      else
+        quantize_store<false>(a, b, blk, lane, sq.job[j]);
+    }
+  }
+}
+constexpr uint32_t kRouterExperts = 4;                     // the router's rows a CTA takes
+constexpr uint32_t kRouterFewRows = 8, kRouterRows = 32;   // rows of x a CTA takes: the two forms
+constexpr uint32_t kRouterChunk = 16;                      // values of a piece a stage holds
+constexpr uint32_t kRouterXRow = kRouterChunk * 4 + 16;    // bytes from a row's chunk to the next: spreads a quarter-warp over the banks
+constexpr uint32_t kRouterWBytes = kRouterExperts * kRouterPieces * kRouterChunk * 4;
+__host__ __device__ constexpr uint32_t router_ring(uint32_t rows) { return rows == kRouterFewRows ? 6 : 4; }
+__host__ __device__ constexpr uint32_t router_x_bytes(uint32_t rows) { return kRouterPieces * rows * kRouterXRow; }
+__host__ __device__ constexpr uint32_t router_rows_smem(uint32_t rows) { return router_ring(rows) * (router_x_bytes(rows) + kRouterWBytes); }  // 42, 88 KB
+template <uint32_t ROWS>
+static __global__ void __launch_bounds__(32 * kRouterPieces) k_router_logits_rows(const float *x, uint32_t T, uint32_t E,
                                                           const float *__restrict__ W, uint32_t N,
                                                           const float *__restrict__ bias, uint32_t NE,
                                                           float *__restrict__ rl, const StepQuant sq) {
-  extern __shared__ __align__(16) float xs[];  // TM rows, each piece padded by 4 floats to spread the banks
+  extern __shared__ __align__(16) uint8_t smem[];
   dependents_may_launch();
-  if (blockIdx.x < sq.ctas) {
-    wait_for_predecessors();
-    const uint32_t lane = threadIdx.x % 32, warps = blockDim.x / 32;
-    const uint64_t step = (uint64_t)gridDim.y * sq.ctas * warps;
-    for (uint64_t blk = ((uint64_t)blockIdx.y * sq.ctas + blockIdx.x) * warps + threadIdx.x / 32; blk < sq.nblk; blk += step) {
-      const float4 a = ((const float4 *)(x + blk * 256))[2 * lane], b = ((const float4 *)(x + blk * 256))[2 * lane + 1];
+  const uint32_t tid = threadIdx.x, lane = tid % 32, piece_of = tid / 32;
+  if (blockIdx.x < sq.ctas) return quantize_share(x, sq);
+  constexpr uint32_t S = router_ring(ROWS), C = kRouterChunk, kXBytes = router_x_bytes(ROWS), kStage = kXBytes + kRouterWBytes;
+  constexpr uint32_t CHAINS = kRouterExperts * ROWS / 32;  // a lane's
+  const uint32_t piece = E / kRouterPieces, nch = piece / C;
+  const uint32_t t0 = blockIdx.y * ROWS, tn = min(ROWS, T - t0), e0 = (blockIdx.x - sq.ctas) * kRouterExperts;
+  const uint32_t smem32 = (uint32_t)__cvta_generic_to_shared(smem);
+  // Four neighbouring threads bring a piece's 64 bytes of a row: the router's rows by half of the threads, x's by all of them.
+  const uint32_t part = tid % 4, pc = tid / 4 % kRouterPieces, first = tid / 32;
+  auto ask_w = [&](uint32_t c) {
+    if (first < kRouterExperts)
+      cp_async16(smem32 + c % S * kStage + kXBytes + (first * kRouterPieces + pc) * (C * 4) + part * 16,
+                 W + (uint64_t)min(e0 + first, N - 1) * E + pc * piece + c * C + part * 4);
+  };
+  auto ask_x = [&](uint32_t c) {
+    for (uint32_t t = first; t < tn; t += 8)
+      cp_async16(smem32 + c % S * kStage + (pc * ROWS + t) * kRouterXRow + part * 16, x + (uint64_t)(t0 + t) * E + pc * piece + c * C + part * 4);
+  };
+  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+  // The first weights are on their way before the rows are there: they are nobody's output.
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        if (!sq.job[j].q) continue;
-        if (sq.job[j].q8k)
-          quantize_store<true>(a, b, blk, lane, sq.job[j]);
-        else
-          quantize_store<false>(a, b, blk, lane, sq.job[j]);
+  for (uint32_t c = 0; c + 1 < S; c++)
+    if (c < nch) ask_w(c);
+  wait_for_predecessors();
+#pragma unroll
+  for (uint32_t c = 0; c + 1 < S; c++) {
+    if (c < nch) ask_x(c);
+    commit();
+  }
+  const uint32_t my_row = lane % ROWS, my_first = lane / ROWS;
+  float p[CHAINS];
+#pragma unroll
+  for (uint32_t e = 0; e < CHAINS; e++) p[e] = 0.0f;
+  for (uint32_t c = 0; c < nch; c++) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+    __syncthreads();  // every thread's copies of this chunk are there, and the stage asked for next has been read
+    if (c + S - 1 < nch) ask_w(c + S - 1), ask_x(c + S - 1);
+    commit();
+    const uint8_t *st = smem + c % S * kStage;
+    const float4 *xs = (const float4 *)(st + (piece_of * ROWS + my_row) * kRouterXRow);
+    const float4 *ws = (const float4 *)(st + kXBytes + (my_first * kRouterPieces + piece_of) * (C * 4));
+#pragma unroll
+    for (uint32_t i = 0; i < C / 4; i++) {
+      const float4 xv = xs[i];
+#pragma unroll
+      for (uint32_t e = 0; e < CHAINS; e++) {
+        const float4 wv = ws[e * kRouterPieces * (C / 4) + i];
+        p[e] = fmaf(xv.x, wv.x, p[e]);
+        p[e] = fmaf(xv.y, wv.y, p[e]);
+        p[e] = fmaf(xv.z, wv.z, p[e]);
+        p[e] = fmaf(xv.w, wv.w, p[e]);
       }
     }
-    return;
   }
-  const uint32_t piece = E / kRouterPieces, pstride = piece + 4, rstride = kRouterPieces * pstride;
-  const uint32_t t0 = blockIdx.y * TM, tn = min((uint32_t)TM, T - t0);
-  const uint32_t lane = threadIdx.x % 32, s = lane % 8, row = ((blockIdx.x - sq.ctas) * (blockDim.x / 32) + threadIdx.x / 32) * 4 + lane / 8;
-  // The first weights are on their way while the rows are staged (and before they are there: the weights are nobody's output).
+  // The pieces of a logit added in order, a thread a logit.
+  __syncthreads();
+  float *sum = (float *)smem;  // [expert][piece][row]
+#pragma unroll
+  for (uint32_t e = 0; e < CHAINS; e++) sum[((my_first + e) * kRouterPieces + piece_of) * ROWS + my_row] = p[e];
+  __syncthreads();
+  const uint32_t e = tid % kRouterExperts, t = tid / kRouterExperts, row = e0 + e;
+  if (t < tn && row < N) {
+    float tot = sum[e * kRouterPieces * ROWS + t];
+#pragma unroll
+    for (uint32_t j = 1; j < kRouterPieces; j++) tot = __fadd_rn(tot, sum[(e * kRouterPieces + j) * ROWS + t]);
+    if (bias && row < NE) tot = __fadd_rn(tot, bias[row]);
+    rl[(uint64_t)(t0 + t) * N + row] = tot;
+  }
+}
+
+// One row: a warp takes four of the router's rows, 8 lanes a row, lane s walking piece s of it with D loads of 16 bytes in flight (a
+// piece is a multiple of 4 D values: 8 always, 16 when the piece is a multiple of 64 values); x in shared memory. A CTA is a warp.
+template <int D>
+static __global__ void __launch_bounds__(32) k_router_logits_one(const float *x, uint32_t E, const float *__restrict__ W, uint32_t N,
+                                                         const float *__restrict__ bias, uint32_t NE, float *__restrict__ rl, const StepQuant sq) {
+  extern __shared__ __align__(16) float xs[];  // each piece padded by 4 floats to spread the banks
+  dependents_may_launch();
+  if (blockIdx.x < sq.ctas) return quantize_share(x, sq);
+  const uint32_t piece = E / kRouterPieces, pstride = piece + 4;
+  const uint32_t lane = threadIdx.x, s = lane % 8, row = (blockIdx.x - sq.ctas) * 4 + lane / 8;
+  // The first weights are on their way while the row is staged (and before it is there: the weights are nobody's output).
   const float4 *w = (const float4 *)(W + (uint64_t)min(row, N - 1) * E + s * piece);
   float4 wq[D];
 #pragma unroll
   for (int i = 0; i < D; i++) wq[i] = __ldg(w + i);
   wait_for_predecessors();
-  for (uint32_t i = threadIdx.x; i < TM * (E / 4); i += blockDim.x) {
-    const uint32_t t = i / (E / 4), k4 = i % (E / 4), k = 4 * k4;
-    const float4 v = t < tn ? ((const float4 *)(x + (uint64_t)(t0 + t) * E))[k4] : make_float4(0, 0, 0, 0);
-    *(float4 *)(xs + t * rstride + (k / piece) * pstride + k % piece) = v;
-  }
-  __syncthreads();
-  float p[TM];
-#pragma unroll
-  for (int t = 0; t < TM; t++) p[t] = 0.0f;
+  for (uint32_t k4 = lane; k4 < E / 4; k4 += 32) *(float4 *)(xs + 4 * k4 / piece * pstride + 4 * k4 % piece) = ((const float4 *)x)[k4];
+  __syncwarp();
+  float p = 0.0f;
   const float *xp = xs + s * pstride;
   for (uint32_t i0 = 0; i0 < piece / 4; i0 += D) {
     float4 cur[D];
@@ -146,25 +230,19 @@ static __global__ void __launch_bounds__(256) k_router_logits_rows(const float *
     }
 #pragma unroll
     for (int i = 0; i < D; i++) {
-#pragma unroll
-      for (int t = 0; t < TM; t++) {
-        const float4 xv = *(const float4 *)(xp + t * rstride + 4 * (i0 + i));
-        p[t] = fmaf(xv.x, cur[i].x, p[t]);
-        p[t] = fmaf(xv.y, cur[i].y, p[t]);
-        p[t] = fmaf(xv.z, cur[i].z, p[t]);
-        p[t] = fmaf(xv.w, cur[i].w, p[t]);
-      }
+      const float4 xv = *(const float4 *)(xp + 4 * (i0 + i));
+      p = fmaf(xv.x, cur[i].x, p);
+      p = fmaf(xv.y, cur[i].y, p);
+      p = fmaf(xv.z, cur[i].z, p);
+      p = fmaf(xv.w, cur[i].w, p);
     }
   }
+  float tot = __shfl_sync(0xffffffffu, p, lane & ~7u);
 #pragma unroll
-  for (int t = 0; t < TM; t++) {
-    float tot = __shfl_sync(0xffffffffu, p[t], lane & ~7u);
-#pragma unroll
-    for (int j = 1; j < (int)kRouterPieces; j++) tot = __fadd_rn(tot, __shfl_sync(0xffffffffu, p[t], (lane & ~7u) + j));
-    if (s == 0 && row < N && (uint32_t)t < tn) {
-      if (bias && row < NE) tot = __fadd_rn(tot, bias[row]);
-      rl[(uint64_t)(t0 + t) * N + row] = tot;
-    }
+  for (int j = 1; j < (int)kRouterPieces; j++) tot = __fadd_rn(tot, __shfl_sync(0xffffffffu, p, (lane & ~7u) + j));
+  if (s == 0 && row < N) {
+    if (bias && row < NE) tot = __fadd_rn(tot, bias[row]);
+    rl[row] = tot;
   }
 }
 

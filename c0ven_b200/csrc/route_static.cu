@@ -37,8 +37,7 @@ cudaError_t setup(int device, float **out) {
     float *p = nullptr;
     cudaError_t e = cudaGetSymbolAddress((void **)&p, g_route_scratch);
     if (e != cudaSuccess) return e;
-    const int smem = (int)((size_t)8 * kRouterPieces * (kStaticEmbd / kRouterPieces + 4) * sizeof(float));
-    e = cudaFuncSetAttribute(k_router_logits_rows<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = cudaFuncSetAttribute(k_router_logits_rows<kRouterRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)router_rows_smem(kRouterRows));
     if (e != cudaSuccess) return e;
     g_scratch_ptr[device] = p;
   }
@@ -83,8 +82,7 @@ MOE_API moe_status moe_route_rows_static(const float *x_dev, uint32_t T, uint32_
   uint32_t *hist = (uint32_t *)(scratch + kLogitFloats);
   // Both regions are written in full for the rows of this call before they are read (every logit of rows < T; every
   // expert's count of every chunk), so the last call's contents need no clearing.
-  const size_t smem = (size_t)8 * kRouterPieces * (n_embd / kRouterPieces + 4) * sizeof(float);
-  k_router_logits_rows<8><<<dim3((N + 3) / 4, (T + 7) / 8), 32, smem, st>>>(x_dev, T, n_embd, router_dev, N, bias_dev, n_experts, rl, StepQuant{});
+  k_router_logits_rows<kRouterRows><<<dim3((N + kRouterExperts - 1) / kRouterExperts, (T + kRouterRows - 1) / kRouterRows), 32 * kRouterPieces, router_rows_smem(kRouterRows), st>>>(x_dev, T, n_embd, router_dev, N, bias_dev, n_experts, rl, StepQuant{});
   const uint32_t nchunks = (T + kChunkTokens - 1) / kChunkTokens;
   k_router_topk<<<nchunks, 32 * kChunkTokens, 0, st>>>(rl, RouterApprox{}, nullptr, T, n_experts, n_used, ids_dev, w_dev, gate_dev, hist);
   e = cudaGetLastError();

@@ -93,3 +93,14 @@ def test_layers_of_several_row_lengths_in_turn():
             check(layer, gpu, synth.make_input(T, layer["n_embd"], seed=T))
     for gpu in gpus:
         gpu.close()
+
+
+@pytest.mark.parametrize("n_embd,n_experts", [(256, 32), (768, 96), (2304, 512)])
+def test_exact_router_at_the_edges_of_its_forms(n_embd, n_experts):
+    """One row, 8 and 32 rows a CTA and one more than each, the longest step; rows of one stage's length a piece and of lengths
+    whose stages the ring does not divide; the oracle's ids bit for bit (check)."""
+    layer = synth.make_layer(n_embd=n_embd, n_ff=256, n_experts=n_experts, n_used=4, gate_type=synth.Q8_0, seed=n_embd)
+    gpu = MoELayer(layer, max_tokens=64)
+    for T in (1, 2, 8, 9, 32, 33, 64):
+        check(layer, gpu, synth.make_input(T, n_embd, seed=T))
+    gpu.close()
