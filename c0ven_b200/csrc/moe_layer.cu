@@ -431,7 +431,8 @@ void create(moe_layer *l, const moe_layer_config &c, const moe_layer_weights &w)
 // are then normal f16 numbers for every weight within 2^-13 of the row's largest, and hi + lo holds 22 bits of w.
 //
 // The bound. An approximate logit differs from the fp32 sum in the exact order by (a) the dropped lo * lo products and
-// the rounding of the lo parts, at most 2^-20 of sum |x_i w_i|; (b) what the MMAs drop, three a step of 16 values; (c) the
+// the rounding of the lo parts, at most 2^-20 of sum |x_i w_i|, and 2^-25 |w_i| for a value of x whose lo part ends below the
+// smallest f16 number, 2^-24, as those under 2^-3 can (x is not scaled); (b) what the MMAs drop, three a step of 16 values; (c) the
 // exact order's own roundings: eight chains of E / 8 fused multiply-adds at 2^-24 of the running sum each, then eight
 // additions, and the up to three that put a split product's pieces together.
 // (b) rests on what the unit does, which tests/test_router_bound_gpu.py checks on it: an MMA aligns its 16 products and the sum
@@ -444,19 +445,20 @@ void create(moe_layer *l, const moe_layer_config &c, const moe_layer_weights &w)
 // the root of the sum over the runs of (the sum of the run's prefix norms) squared, whatever way x's norm falls to them: prefix_sums.
 // eps = eps_rel |x|, with eps_rel the largest over the experts of 2^-23 (15 steps + chains / 2 + 16 |w_e|), a hundredth more
 // for the roundings of roundings, covers all three where every rounding falls the same way (of |w_e|, at E = 2048 and in one, two and four
-// pieces: 2^-12.6, 2^-13.5, 2^-14.5); a random row's error is some hundredth of it. The bias adds one rounding of the biased logit,
-// covered by eps_abs.
+// pieces: 2^-12.6, 2^-13.5, 2^-14.5); a random row's error is some hundredth of it. eps_abs is the rest: 2^-25 of the largest sum of
+// an expert's |w_i|, and 2^-20 for the rounding of the biased logit.
 void setup_router_tensor(moe_layer *l, const float *router, const float *bias, cudaStream_t st) {
   const uint32_t E = l->E, NE = l->NE, T = l->Tmax;
   const uint64_t wrows = std::max<uint32_t>(NE, kRouterTileExperts), xrows = std::max<uint32_t>(T, kRouterTileRows);
   std::vector<__half> hi(wrows * E, __float2half_rn(0.0f)), lo(wrows * E, __float2half_rn(0.0f));
   std::vector<float> unscale(NE, 1.0f);
-  double eps[3] = {0.0, 0.0, 0.0};
+  double eps[3] = {0.0, 0.0, 0.0}, w_sum_max = 0.0;
   for (uint32_t e = 0; e < NE; e++) {
     const float *w = router + (size_t)e * E;
     float m = 0.0f;
-    double n2 = 0.0;
-    for (uint32_t i = 0; i < E; i++) m = std::max(m, std::fabs(w[i])), n2 += (double)w[i] * w[i];
+    double n2 = 0.0, w_sum = 0.0;
+    for (uint32_t i = 0; i < E; i++) m = std::max(m, std::fabs(w[i])), n2 += (double)w[i] * w[i], w_sum += std::fabs(w[i]);
+    w_sum_max = std::max(w_sum_max, w_sum);
     // The norms of each run's first values, every `step` of them, added up; of the runs' sums the norm.
     auto prefix_sums = [&](uint32_t runs, uint32_t step) {
       double all = 0.0;
@@ -487,7 +489,7 @@ void setup_router_tensor(moe_layer *l, const float *router, const float *bias, c
   float bias_max = 0.0f;
   for (uint32_t e = 0; bias && e < NE; e++) bias_max = std::max(bias_max, std::fabs(bias[e]));
   for (uint32_t j = 0; j < 3; j++) l->router_eps_rel[j] = (float)std::ldexp(eps[j], -23);
-  l->router_eps_abs = std::ldexp(1.0f + bias_max, -20);
+  l->router_eps_abs = std::ldexp(1.0f + bias_max, -20) + (float)std::ldexp(1.01 * w_sum_max, -25);
   l->rw_hi.alloc(hi.size()), l->rw_lo.alloc(lo.size()), l->rw_unscale.alloc(NE);
   CUDA_OK(cudaMemcpyAsync(l->rw_hi.get(), hi.data(), hi.size() * sizeof(__half), cudaMemcpyHostToDevice, st));
   CUDA_OK(cudaMemcpyAsync(l->rw_lo.get(), lo.data(), lo.size() * sizeof(__half), cudaMemcpyHostToDevice, st));

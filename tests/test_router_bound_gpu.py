@@ -100,3 +100,25 @@ def test_the_nearest_expert_by_the_fixed_order_is_the_one_taken():
     gpu.forward(x)
     assert np.array_equal(gpu.route(T)[0][:40], ids)
     gpu.close()
+
+
+def test_values_too_small_for_the_two_parts():
+    """A row of values just under half the smallest f16 number: both parts are zero, and all of the first expert's logit, summed
+    over the whole row, is error; the second expert's is a third less, from one value that f16 holds."""
+    E, T = 2048, ROWS[1]
+    W = np.zeros((NE, E), np.float32)
+    W[3, 1:] = np.where(np.arange(1, E) % 3 == 0, -1.0, 1.0)
+    x = np.zeros((T, E), np.float32)
+    x[:, 1:] = W[3, 1:] * np.float32(0.49 * 2.0 ** -24)
+    x[:, 0] = 2.0 ** -10
+    exact = O.router_logits(x[:1], W, np.zeros(E, np.float32), None)[0, 3]
+    W[1, 0] = exact * np.float32(2 / 3 * 2 ** 10)
+    exact = O.router_logits(x[:40], W, np.zeros(E, np.float32), None)
+    ids = O.router_topk(exact, 1)[0]
+    assert np.all(ids == 3)
+    gpu = make(W, E, T)
+    gpu.forward(x)
+    approx, is_approx, eps_rel, eps_abs = gpu.logits(T)
+    assert is_approx and np.all(np.abs(approx[:40] - exact[:, :NE]) <= eps_rel * np.linalg.norm(x[0].astype(np.float64)) + eps_abs)
+    assert np.array_equal(gpu.route(T)[0][:40], ids)
+    gpu.close()
