@@ -569,9 +569,12 @@ uint32_t few_rows_for(const moe_layer *l, uint64_t R, uint32_t nexp) {
 // instructions whatever the type (200 rows of IQ3_S: 1085 -> 491 us); with one or two it depends on how much work there is to
 // spread over its warps, of 16 weight rows, and on what it replaces. From 32 assignments on where the integer-dot kernel's decode is
 // long and runs once a row (32 rows, even routing: Q4_K 309 -> 168 us, IQ4_XS with IQ4_NL 315 -> 236) or where it finds a row's
-// units at run time (14 rows of 2,560 values: Q8_0 219 -> 152, IQ3_S 242 -> 160; 12 rows of 1,024 in IQ3_S 68 -> 57). Of the
-// rest from 200 on (Q8_0 9 rows 123 and 137, 20 rows 182 and 178, 50 rows 297 and 264; IQ2_S with Q2_0 32 rows 262 and 221), but not
-// IQ3_S, whose two kernels decode at the same rate (13 rows 141 and 160, 32 rows 246 and 248). Never
+// units at run time, in one of the products or both (Q8_0, IQ3_S, IQ3_XXS, IQ2_S and Q2_0, rows of 2,560 or of 768 values, 36 to 500
+// assignments: the layer takes 1.00 to 1.6 times as long by it, 2.7 times for Q2_0 at 500). Of the rest from 200 on (the layer's time by it
+// over that by the few-rows kernel at 200, 320 and 500 assignments over 512 experts: Q8_0 1.01, 1.06, 1.12; IQ3_XXS 1.00, 1.02, 1.04; IQ2_S with
+// Q2_0 1.14, 1.21, 1.24; Q2_0 1.72, 1.99, 2.15; below 200 from 0.89 on), but not IQ3_S, whose two kernels decode at the same rate
+// (0.98, 1.00, 1.01), nor Q8_0 with a codebook of four values in the down product, which gains less in the one than it loses in the
+// other (with IQ3_S 0.96, 0.97, 1.01; with IQ3_XXS 0.93, 0.94, 0.99; with any other type 0.98 to 1.29). Never
 // in a layer kept off the tensor cores (MOE_FLAG_NO_TENSOR), whose products are the integer-dot kernels' whatever the rows.
 bool groups_take_mma(const moe_layer *l, int M, uint64_t R) {
   if (!l->can_tensor || M < 2) return false;
@@ -581,7 +584,7 @@ bool groups_take_mma(const moe_layer *l, int M, uint64_t R) {
   auto specialised = [](uint32_t K) { return K == 2048 || K == 512 || K == 256; };  // launch_shape
   if (M > 2) return true;
   if ((heavy(g) && heavy(d)) || !specialised(l->E) || !specialised(l->F)) return R >= 32;
-  return R >= 200 && g != QT_IQ3_S;
+  return R >= 200 && g != QT_IQ3_S && !(g == QT_Q8_0 && (d == QT_IQ3_S || d == QT_IQ3_XXS));
 }
 
 // The exact fp32 router product of a step's rows, its x quantised by the same launch.
