@@ -102,10 +102,19 @@ def test_a_layer_kept_off_the_tensor_cores_keeps_its_integer_dots(t, n_embd, n_f
 
 @pytest.mark.parametrize("t", TYPES)
 def test_entries_whose_rows_leave_room_for_one_cta(t):
-    """Rows of which two CTAs' 32 do not fit an SM: one CTA of sixteen warps takes them; with entries of 1 to 32 rows, and a
-    down product of more items than CTAs, each of which then takes runs of several entries."""
-    layer = synth.make_layer(n_embd=2560, n_ff=512, n_experts=96, n_used=4, gate_type=t, seed=t + 7)
-    gpu = MoELayer(layer, max_tokens=350)
-    check(layer, gpu, synth.make_input(350, 2560, seed=5))
+    """The longest rows the kernel takes, of which two CTAs' 32 do not fit an SM in any type: one CTA of sixteen warps takes
+    gate and up, with entries of every count of row tiles; a down product of more items than CTAs, each of which then takes
+    runs of several entries."""
+    n_embd = 2560 if t == synth.Q6_K else 2816
+    layer = synth.make_layer(n_embd=n_embd, n_ff=256, n_experts=288, n_used=4, gate_type=t, seed=t + 7)
+    repeats = list(range(9, 33))
+    x = synth.make_input(300 + len(repeats), n_embd, seed=5)
+    x = np.concatenate([x[len(repeats):], np.repeat(x[:len(repeats)], repeats, axis=0)])
+    gpu = MoELayer(layer, max_tokens=len(x))
+    check(layer, gpu, x)
+    cnt = np.bincount(gpu.route(len(x))[0].reshape(-1), minlength=288)
+    assert np.count_nonzero(cnt) >= 256 and 1280 <= cnt.sum() <= 24 * 288  # below 256 hit no entry passes 16 rows
+    for lo, hi in ((1, 8), (9, 16), (17, 24), (25, 32)):
+        assert np.count_nonzero((cnt >= lo) & (cnt <= hi)) >= 4, (lo, hi)
     assert len(gpu.groups()) == 0
     gpu.close()
