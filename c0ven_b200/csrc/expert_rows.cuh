@@ -114,6 +114,13 @@ __device__ __forceinline__ int dot4x4(const uint4 &w, const int4 &a) {
 // Bytes of one activation row in shared memory: codes, then the scales (padded to 16), then q8_K's sums.
 __host__ __device__ constexpr uint32_t act_d_bytes(bool q8k, uint32_t K) { return q8k ? ((K / 64 + 15) & ~15u) : K / 8; }
 constexpr uint32_t kRowsMaxK = 16384;  // the longest activation row the integer-dot kernels stage (8 rows of it fit an SM's shared memory)
+// Row lengths that the integer-dot kernels have forms of their own for (launch_shape): the benchmark's, and a row of one block.
+constexpr uint32_t kRowsLengths[] = {2048, 512, 256};
+constexpr bool rows_specialised(uint32_t K) {
+  for (uint32_t n : kRowsLengths)
+    if (n == K) return true;
+  return false;
+}
 __host__ __device__ constexpr uint32_t act_row_stride(bool q8k, uint32_t K) { return K + act_d_bytes(q8k, K) + (q8k ? K / 8 : 0) + 16; }
 
 // SwiGLU as the CPU path states it (core/cpu/experts.cpp:21-27).

@@ -45,16 +45,15 @@ static cudaError_t launch_one(ExpertRowsArgs a, uint32_t max_groups, const uint3
 
 template <int QT, int NMAT, int M, int FORM>
 static cudaError_t launch_shape(const ExpertRowsArgs &a, uint32_t max_groups, const uint32_t *grid_global, const LaunchCtx &ctx, cudaStream_t st) {
-  const uint32_t upr = a.K / Unit<QT>::kValues;
-  // The three row lengths the kernels are specialised for are 2048, 512 and 256 values; any other takes the general
-  // instantiation, which finds a row's units at run time.
-  constexpr uint32_t U2048 = 2048 / Unit<QT>::kValues, U512 = 512 / Unit<QT>::kValues, U256 = 256 / Unit<QT>::kValues;
-  if (upr == U2048) return launch_one<QT, NMAT, M, 32, U2048 / 32, FORM>(a, max_groups, grid_global, ctx, st);
+  // Lengths that the kernels are not specialised for take the general instantiation, which finds a row's units at run time.
+  if (!rows_specialised(a.K)) return launch_one<QT, NMAT, M, 32, 0, FORM>(a, max_groups, grid_global, ctx, st);
+  constexpr uint32_t kLong = kRowsLengths[0] / Unit<QT>::kValues, kMid = kRowsLengths[1] / Unit<QT>::kValues, kShort = kRowsLengths[2] / Unit<QT>::kValues;
+  static_assert(sizeof(kRowsLengths) / sizeof(kRowsLengths[0]) == 3, "a form for each");
+  if (a.K == kRowsLengths[0]) return launch_one<QT, NMAT, M, 32, kLong / 32, FORM>(a, max_groups, grid_global, ctx, st);
   // A row of 32 units (Q8_0's 512 values): 16 lanes with two units each, two rows a warp pass, so that a reduction and a
   // store serve twice the bytes.
-  if (upr == U512) return launch_one<QT, NMAT, M, (U512 < 32 ? U512 : 16), (U512 < 32 ? 1 : U512 / 16), FORM>(a, max_groups, grid_global, ctx, st);
-  if (upr == U256) return launch_one<QT, NMAT, M, (U256 < 32 ? U256 : 32), 1, FORM>(a, max_groups, grid_global, ctx, st);
-  return launch_one<QT, NMAT, M, 32, 0, FORM>(a, max_groups, grid_global, ctx, st);
+  if (a.K == kRowsLengths[1]) return launch_one<QT, NMAT, M, (kMid < 32 ? kMid : 16), (kMid < 32 ? 1 : kMid / 16), FORM>(a, max_groups, grid_global, ctx, st);
+  return launch_one<QT, NMAT, M, (kShort < 32 ? kShort : 32), 1, FORM>(a, max_groups, grid_global, ctx, st);
 }
 
 template <int QT, int NMAT>

@@ -581,9 +581,8 @@ bool groups_take_mma(const moe_layer *l, int M, uint64_t R) {
   const uint32_t g = l->cfg.gate_type, d = l->cfg.down_type;
   if (!mma_takes(g, l->E, kGroupMax) || !mma_takes(d, l->F, kGroupMax)) return false;
   auto heavy = [](uint32_t t) { return t == QT_Q4_K || t == QT_Q6_K || t == QT_IQ4_XS || t == QT_IQ4_NL; };
-  auto specialised = [](uint32_t K) { return K == 2048 || K == 512 || K == 256; };  // launch_shape
   if (M > 2) return true;
-  if ((heavy(g) && heavy(d)) || !specialised(l->E) || !specialised(l->F)) return R >= 32;
+  if ((heavy(g) && heavy(d)) || !rows_specialised(l->E) || !rows_specialised(l->F)) return R >= 32;
   return R >= 200 && g != QT_IQ3_S && !(g == QT_Q8_0 && (d == QT_IQ3_S || d == QT_IQ3_XXS));
 }
 
