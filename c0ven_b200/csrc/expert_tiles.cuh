@@ -868,8 +868,7 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
   const uint32_t unit = PAIR ? blockIdx.x / 2 : blockIdx.x, nunits = PAIR ? gridDim.x / 2 : gridDim.x;
   const uint32_t RTU = PAIR ? RT / 2 : RT;  // a big tile's items
   const uint32_t nitems = ntiles * RTU;
-  // Item / RTU without a division: exact while item * RTU stays below 2^32.
-  const uint32_t magic = RTU > 1 ? 0xFFFFFFFFu / RTU + 1 : 0;
+  const uint32_t magic = item_magic(RTU);  // a big tile's number without a division (the launch bounds the tiles)
   auto tile_of_item = [&](uint32_t item) { return RTU > 1 ? __umulhi(item, magic) : item; };
   if (unit >= nitems) return;  // both CTAs of a pair alike
   const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;

@@ -35,6 +35,7 @@ cudaError_t launch_expert_tiles(const ExpertTilesArgs &a, const CUtensorMap &act
                                 const LaunchCtx &ctx, cudaStream_t st) {
   if (a.K % kTileK || a.R % kTileM || max_tiles == 0) return cudaErrorInvalidValue;
   const uint32_t RT = a.R / kTileM;
+  if (!items_divide(max_tiles, RT % 2 == 0 ? RT / 2 : RT)) return cudaErrorInvalidValue;
   if (RT % 2 == 0) {
     // Pairs of CTAs on 256 weight rows an item: half the rows' bytes through each CTA's shared memory.
     auto kernel = k_expert_tiles<QT, NMAT, true>;

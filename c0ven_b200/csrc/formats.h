@@ -71,6 +71,13 @@ FMT_HD constexpr uint64_t run_offset(uint32_t t, uint32_t f, uint64_t n) {
   return off * n;
 }
 
+// The tile kernels number their items tile by tile, n of them a tile, and divide by n with a multiply: item / n is the high word of
+// item * item_magic(n) (the item itself for n = 1), exactly while item * n stays below 2^32, since magic exceeds 2^32 / n by less
+// than 1. The launch admits no more tiles than that holds for (items_divide). A layer that fits a GPU stays far below: n is 64 at
+// most, and tiles * 256 rows of n * 256 results of four bytes each are 256 KB an item, 256 GB at a million of them.
+FMT_HD constexpr uint32_t item_magic(uint32_t n) { return n > 1 ? 0xFFFFFFFFu / n + 1 : 0u; }
+FMT_HD constexpr bool items_divide(uint64_t tiles, uint32_t n) { return tiles <= 0xFFFFFFFFull / n / n; }
+
 // Host repack, threaded (runs.cpp). Both are permutations of the slice's bytes.
 void to_runs(uint32_t type, const uint8_t *file_blocks, uint64_t nblocks, uint8_t *dst);
 void from_runs(uint32_t type, const uint8_t *runs, uint64_t nblocks, uint8_t *dst);

@@ -2,6 +2,7 @@
 and on the host functions themselves in a program of their own."""
 import pathlib
 import re
+import subprocess
 
 CSRC = pathlib.Path(__file__).resolve().parent.parent / "c0ven_b200" / "csrc"
 
@@ -25,3 +26,33 @@ def test_the_specialised_row_lengths_are_listed_once():
     assert "rows_specialised(" in rule and "rows_specialised(" in dispatch
     for text in (rule, dispatch):
         assert not re.search(r"\b(2048|512|256)\b", text)
+
+
+def test_items_are_divided_exactly_up_to_what_the_host_admits(tmp_path):
+    """The tile kernels divide an item's number by the items a tile has with a multiply: for every layer size at the largest
+    count of tiles that the launch admits, around every multiple; and one tile more is refused, in the launch."""
+    program = r"""
+#include <cstdio>
+#include "formats.h"
+using namespace moe;
+int main() {
+  for (uint32_t n = 1; n <= 64; n++) {
+    uint64_t tiles = ((1ull << 32) - 1) / n / n;
+    while (items_divide(tiles + 1, n)) tiles++;
+    while (tiles && !items_divide(tiles, n)) tiles--;
+    if (!tiles || items_divide(tiles + 1, n) || items_divide(1ull << 32, n)) return 1;
+    const uint64_t items = tiles * n;
+    const uint32_t magic = item_magic(n);
+    auto quotient = [&](uint64_t i) { return n > 1 ? (i * magic) >> 32 : i; };
+    for (uint64_t t = 0; t < tiles; t += t < 4096 || t + 4096 > tiles ? 1 : 997)
+      for (uint64_t i : {t * n, t * n + n / 2, t * n + n - 1})
+        if (i >= items || quotient(i) != t) return 2;
+  }
+  puts("exact");
+}
+"""
+    (tmp_path / "divide.cpp").write_text(program)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-I" + str(CSRC), str(tmp_path / "divide.cpp"), "-o", str(tmp_path / "divide")], check=True)
+    assert subprocess.run([str(tmp_path / "divide")], capture_output=True, text=True).stdout == "exact\n"
+    assert "!items_divide(max_tiles," in function("expert_tiles_inst.cuh", "launch_expert_tiles")
+    assert "item_magic(" in (CSRC / "expert_tiles.cuh").read_text()
