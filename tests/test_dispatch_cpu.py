@@ -33,6 +33,7 @@ def test_items_are_divided_exactly_up_to_what_the_host_admits(tmp_path):
     count of tiles that the launch admits, around every multiple; and one tile more is refused, in the launch."""
     program = r"""
 #include <cstdio>
+#include <initializer_list>
 #include "formats.h"
 using namespace moe;
 int main() {
