@@ -9,9 +9,11 @@
 
 namespace moe {
 
-// Pairs of CTAs the GPU runs at once for kernel (one CTA an SM, so at most one pair a TPC), asked once per device.
-template <class Kernel>
-static cudaError_t max_pairs(Kernel kernel, uint32_t threads, size_t smem, int device, uint32_t &pairs) {
+// Pairs of CTAs the GPU runs at once for kernel (one CTA an SM, so at most one pair a TPC), asked once per device. The kernel is
+// the template's own argument, for the answer is kept beside it: gate's and up's kernel and the down product's have one type,
+// but blocks of 736 and 864 threads.
+template <auto kernel>
+static cudaError_t max_pairs(uint32_t threads, size_t smem, int device, uint32_t &pairs) {
   static std::atomic<uint32_t> known[64];
   if (device < 0 || device >= 64) return cudaErrorInvalidValue;
   pairs = known[device].load(std::memory_order_acquire);
@@ -38,13 +40,13 @@ cudaError_t launch_expert_tiles(const ExpertTilesArgs &a, const CUtensorMap &act
   if (!items_divide(max_tiles, RT % 2 == 0 ? RT / 2 : RT)) return cudaErrorInvalidValue;
   if (RT % 2 == 0) {
     // Pairs of CTAs on 256 weight rows an item: half the rows' bytes through each CTA's shared memory.
-    auto kernel = k_expert_tiles<QT, NMAT, true>;
+    constexpr auto kernel = k_expert_tiles<QT, NMAT, true>;
     const size_t smem = TileSmem<QT, NMAT, true>::kBytes;
     static std::atomic<uint32_t> attr_done{0};
     cudaError_t e = ensure_dynamic_smem(kernel, smem, attr_done, ctx.device);
     if (e != cudaSuccess) return e;
     uint32_t pairs = 0;
-    e = max_pairs(kernel, tile_threads(NMAT), smem, ctx.device, pairs);
+    e = max_pairs<kernel>(tile_threads(NMAT), smem, ctx.device, pairs);
     if (e != cudaSuccess) return e;
     const uint64_t items = (uint64_t)max_tiles * (RT / 2);
     cudaLaunchConfig_t cfg{};

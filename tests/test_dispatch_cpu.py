@@ -57,3 +57,18 @@ int main() {
     assert subprocess.run([str(tmp_path / "divide")], capture_output=True, text=True).stdout == "exact\n"
     assert "!items_divide(max_tiles," in function("expert_tiles_inst.cuh", "launch_expert_tiles")
     assert "item_magic(" in (CSRC / "expert_tiles.cuh").read_text()
+
+
+def test_what_a_launch_keeps_is_kept_for_one_kernel():
+    """What a launch asks the device once and keeps (an attribute set, clusters that fit) lies in a static word, which has to be one
+    a kernel: a helper that is a template on the kernel's type alone has one for all kernels of that signature."""
+    statics = 0
+    for path in sorted(CSRC.glob("*.cu*")) + sorted(CSRC.glob("*.h")):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for m in re.finditer(r"static std::atomic<[^;]*;", text):
+            statics += 1
+            templates = [t for t in re.finditer(r"^template <([^\n]*)>$", text[:m.start()], re.M)]
+            start = [f for f in re.finditer(r"^(?!template|namespace|//)[\w:]+ [^;\n]*\([^;]*?\{$", text[:m.start()], re.M)][-1]
+            own = [t.group(1) for t in templates if text[t.end():start.start()].strip() == ""]
+            assert not own or not re.fullmatch(r"(class|typename) \w+", own[0]), (path.name, start.group(0))
+    assert statics >= 7  # the pattern still finds them
