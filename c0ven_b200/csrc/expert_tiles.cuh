@@ -142,14 +142,8 @@ __device__ __forceinline__ void tma_load_rows(uint32_t dst_smem, const CUtensorM
 }
 // Four rows y0 .. y3 of the map's tensor (its box one row of 64 values), values x .. x + 63 of each, into four
 // consecutive 128-byte rows of shared memory at dst (512-byte aligned inside a 1024-byte aligned tile), swizzled as the
-// tile's other rows are. The rows need not be neighbours: this is how a tile's rows are gathered by index.
-__device__ __forceinline__ void tma_gather4_rows(uint32_t dst_smem, const CUtensorMap *map, uint32_t x, uint32_t y0, uint32_t y1, uint32_t y2,
-                                                 uint32_t y3, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-               ::"r"(dst_smem), "l"((uint64_t)map), "r"(x), "r"(y0), "r"(y1), "r"(y2), "r"(y3), "r"(bar)
-               : "memory");
-}
-// The same by a CTA of a pair, the bytes counted on a barrier that may be the other CTA's.
+// tile's other rows are. The rows need not be neighbours: this is how a tile's rows are gathered by index. By a CTA of a pair,
+// the bytes counted on a barrier that may be the other CTA's.
 __device__ __forceinline__ void tma_gather4_rows_pair(uint32_t dst_smem, const CUtensorMap *map, uint32_t x, uint32_t y0, uint32_t y1,
                                                       uint32_t y2, uint32_t y3, uint32_t bar) {
   asm volatile(
@@ -777,15 +771,14 @@ struct StageMap {
   }
 };
 
-// Shared memory of a CTA: the stages (NMAT weight tiles of 16 KB and a row tile of 32 KB each), then (for types whose
+// Shared memory of a CTA: the stages (NMAT weight tiles of 16 KB and half a row tile, 16 KB, each), then (for types whose
 // quants come by copy) a ring of two quant slots, then the barriers, then a codebook type's codebook.
 // A quant slot holds, for every weight row of the item, the quants of one stage per decode group: 32 bytes a stage for
 // Q4_K, so 64 bytes a row with two groups (64-byte swizzle) and 128 with four (128-byte swizzle).
-template <int QT, int NMAT, bool PAIR = false>
+template <int QT, int NMAT>
 struct TileSmem {
-  // A CTA of a pair holds half the rows' tile, which leaves room for more stages.
-  static constexpr uint32_t kStages = PAIR ? (NMAT == 2 ? 4 : 6) : (NMAT == 2 ? 3 : 4);
-  static constexpr uint32_t kXRows = PAIR ? kTileN / 2 : kTileN;
+  static constexpr uint32_t kStages = NMAT == 2 ? 4 : 6;
+  static constexpr uint32_t kXRows = kTileN / 2;                                      // a CTA of a pair holds half the rows' tile
   static constexpr uint32_t kWBytes = kTileM * kTileK * 2, kXBytes = kXRows * kTileK * 2;
   static constexpr uint32_t kStageBytes = NMAT * kWBytes + kXBytes;
   static constexpr uint32_t kGroups = kTileDecoders / (NMAT * kTileM);                // decode groups: 2 or 4
@@ -825,25 +818,25 @@ __device__ __forceinline__ ItemTile item_tile(const ExpertTilesArgs &a, uint32_t
 }
 
 // NMAT 2: out = swiglu(gate x, up x); NMAT 1: out = down h. Persistent: the grid is one CTA per SM (fewer when there is
-// less work), single or in pairs (PAIR, below); a unit (a CTA or a pair) takes the work items dealt to it round by
-// round; item i is weight-row tile (or pair of tiles) i % RTU of big tile i / RTU, so neighbouring units share a tile's
+// less work), in clusters of two on the two SMs of a TPC. Such a pair is one unit of work: it takes the items dealt to it round by
+// round; item i is pair of weight-row tiles i % RTU of big tile i / RTU, so neighbouring pairs share a tile's
 // activations in L2. Five roles: 16 decode warps (quants to f16 weights in shared memory), 4 or 8 epilogue warps
 // (accumulators to the result), a warp whose first lane issues the bulk-tensor copies of the rows' activations (the
-// whole warp when the rows are gathered by index), the warp that owns tensor memory and whose first lane issues the
-// MMAs, and a warp whose first lane issues the copies of the quants for types that take them through the ring. A warp
-// arrives on a barrier once, by one lane.
+// whole warp when the rows are gathered by index), the warp that owns tensor memory and runs the MMAs in step, one elected
+// lane of it issuing them, and a warp whose first lane issues the copies of the quants for types that take them through the
+// ring. A warp arrives on a barrier once, by one lane.
 //
 // Tensor memory is two buffers of 256 columns. An item of at most 128 rows (any item, for NMAT 1) takes one buffer,
 // alternately, so the epilogue warps drain item i while the MMAs of item i + 1 run and the decode warps never stop. A
 // gate/up item of more than 128 rows needs both buffers (gate in one, up in the other): the MMAs of the next item
 // wait for its epilogue, and to keep that short the decode warps join the epilogue warps for it.
 // Dynamic shared memory TileSmem::kBytes.
-template <int QT, int NMAT, bool PAIR>
+template <int QT, int NMAT>
 __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __grid_constant__ ExpertTilesArgs a,
                                                                   const __grid_constant__ CUtensorMap act_map,
                                                                   const uint32_t *__restrict__ grid_global) {
   using namespace tc;
-  using SM = TileSmem<QT, NMAT, PAIR>;
+  using SM = TileSmem<QT, NMAT>;
   using Dec = Decoder<QT>;
   using Raw = typename Dec::Raw;
   constexpr uint32_t S = SM::kStages, kCols = 512;
@@ -857,16 +850,15 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
 
-  const uint32_t K = a.K, KT = K / kTileK, RT = a.R / kTileM;
+  const uint32_t K = a.K, KT = K / kTileK;
   const uint32_t ntiles = a.tiles ? *a.ntiles : (a.dense_rows + kTileN - 1) / kTileN;
-  // PAIR: the CTAs come in clusters of two, on the two SMs of a TPC. A pair is one unit of work: its item is 256 weight
-  // rows (128 decoded by each CTA) times the tile's rows, of which each CTA brings half into its own shared memory;
-  // the first CTA's MMA thread issues one tcgen05.mma.cta_group::2 for both, which reads both halves and writes each
+  // A pair's item is 256 weight rows (128 decoded by each CTA) times the tile's rows, of which each CTA brings half into its own
+  // shared memory; the first CTA's MMA warp issues one tcgen05.mma.cta_group::2 for both, which reads both halves and writes each
   // CTA's 128 weight rows of the product into that CTA's tensor memory. What a CTA's shared memory carries per flop
-  // is the weights as before but only half the rows, and shared-memory bandwidth is what bounds the single-CTA form.
-  const uint32_t rank = PAIR ? cluster_ctarank() : 0;
-  const uint32_t unit = PAIR ? blockIdx.x / 2 : blockIdx.x, nunits = PAIR ? gridDim.x / 2 : gridDim.x;
-  const uint32_t RTU = PAIR ? RT / 2 : RT;  // a big tile's items
+  // is a single CTA's weights but only half its rows, and shared-memory bandwidth is what bounded the kernel by single CTAs.
+  const uint32_t rank = cluster_ctarank();
+  const uint32_t unit = blockIdx.x / 2, nunits = gridDim.x / 2;
+  const uint32_t RTU = a.R / (2 * kTileM);  // a big tile's items
   const uint32_t nitems = ntiles * RTU;
   const uint32_t magic = item_magic(RTU);  // a big tile's number without a division (the launch bounds the tiles)
   auto tile_of_item = [&](uint32_t item) { return RTU > 1 ? __umulhi(item, magic) : item; };
@@ -890,7 +882,7 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
   // when the epilogue warps have read it; after an item that took both buffers, also when the decode warps have.
   if (tid == 0) {
     // In a pair the first CTA's full, accumulator-empty barriers take both CTAs' arrivals.
-    constexpr uint32_t kCtas = PAIR ? 2 : 1;
+    constexpr uint32_t kCtas = 2;
     for (uint32_t s = 0; s < S; s++) mbar_init(full_bar(s), kCtas * (kDW / kDecGroups + 1)), mbar_init(empty_bar(s), 1);
     for (uint32_t b = 0; b < 2; b++) mbar_init(acc_full(b), 1), mbar_init(acc_empty(b), kCtas * kEW);
     mbar_init(acc_empty_wide, kCtas * kDW);
@@ -900,32 +892,20 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
   }
   if constexpr (grid_words(QT) > 0)
     for (uint32_t i = tid; i < grid_words(QT); i += blockDim.x) grid[i] = grid_global[grid_offset(QT) + i];
-  if (warp == kMmaWarp) {
-    if constexpr (PAIR)
-      tmem_alloc_pair(smem_u32(tmem_slot), kCols);  // the same warp of both CTAs, the same place for the address
-    else
-      tmem_alloc(smem_u32(tmem_slot), kCols);
-  }
+  if (warp == kMmaWarp) tmem_alloc_pair(smem_u32(tmem_slot), kCols);  // the same warp of both CTAs, the same place for the address
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync();  // the other CTA's barriers exist before anything arrives on them
+  cluster_sync();  // the other CTA's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   bool ok = true;
   // The first CTA's barriers, as the pair's other CTA names them (for the first CTA itself: its own).
-  const uint32_t bar0_lead = PAIR ? map_to_cta(bar0, 0) : bar0;
+  const uint32_t bar0_lead = map_to_cta(bar0, 0);
   auto full_lead = [&](uint32_t s) { return bar0_lead + 8 * s; };
   auto acc_empty_lead = [&](uint32_t b) { return bar0_lead + 8 * (2 * S + 2 + b); };
   const uint32_t acc_empty_wide_lead = bar0_lead + 8 * (2 * S + 4);
-  // Arrivals that in a pair go to the first CTA's barrier.
-  auto arrive_lead = [&](uint32_t lead_bar, uint32_t own_bar) {
-    if constexpr (PAIR)
-      mbar_arrive_cluster(lead_bar);
-    else
-      mbar_arrive(own_bar);
-  };
   // The weight rows of an item that this CTA decodes and drains.
-  auto item_rows0 = [&](uint32_t item) { return ((item - tile_of_item(item) * RTU) * (PAIR ? 2u : 1u) + rank) * kTileM; };
+  auto item_rows0 = [&](uint32_t item) { return ((item - tile_of_item(item) * RTU) * 2u + rank) * kTileM; };
 
   // CTA b's item of round r: the items come expert by expert for the experts with full tiles, then the short tiles of
   // the others by falling row count, and the rounds deal them boustrophedon (b, then G - 1 - b, ...), so that every CTA
@@ -1054,7 +1034,7 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
       auto stage_end = [&](uint32_t s) {
         fence_async_smem();
         __syncwarp();
-        if (lane == 0) arrive_lead(full_lead(s), full_bar(s));
+        if (lane == 0) mbar_arrive_cluster(full_lead(s));
       };
       auto tile_of = [&](uint32_t s) { return smem + s * SM::kStageBytes + mat * SM::kWBytes; };
       if constexpr (quants_by_copy(QT)) {
@@ -1155,7 +1135,7 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
           drain(t, r0, 0, kTileN, warp / 4, kDW / 4 + 1);
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) arrive_lead(acc_empty_wide_lead, acc_empty_wide);
+          if (lane == 0) mbar_arrive_cluster(acc_empty_wide_lead);
         }
         use0++, use1++, wides++;
       } else {
@@ -1176,7 +1156,7 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
         drain(t, r0, 0, kTileN, kDW / 4, kDW / 4 + 1);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_lead(acc_empty_lead(0), acc_empty(0)), arrive_lead(acc_empty_lead(1), acc_empty(1));
+        if (lane == 0) mbar_arrive_cluster(acc_empty_lead(0)), mbar_arrive_cluster(acc_empty_lead(1));
         use0++, use1++, wides++;
       } else {
         const uint32_t b = next_buf;
@@ -1186,54 +1166,32 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
         drain(t, r0, b * kTileN, b * kTileN + kTileN / 2, (warp - kDW) / 4, kEW / 4);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_lead(acc_empty_lead(b), acc_empty(b));
+        if (lane == 0) mbar_arrive_cluster(acc_empty_lead(b));
         use_inc(b), next_buf ^= 1;
       }
     }
   } else if (warp == kCopyWarp) {
     if (a.gather_rows) {
       // The copy warp, gathering: the tile's rows are scattered over the activations (row r of the expert order is row
-      // gather_rows[r] of the map's tensor) and a copy brings four of them: up to 32 copies a stage for a pair's CTA (one
-      // a lane), 64 for a single CTA (two a lane). A lane keeps its row indices for the whole item. Rows past the
-      // tile's count repeat its last row; their columns of the result are dropped.
-      constexpr uint32_t kPerLane = PAIR ? 1 : 2;
+      // gather_rows[r] of the map's tensor) and a copy brings four of them: up to 32 copies a stage, one a lane. A lane keeps its
+      // row indices for the whole item. Rows past the tile's count repeat its last row; their columns of the result are dropped.
       uint32_t li = 0;
       for (uint32_t rnd = 0, item; (item = item_at(rnd)) != kNoItem && ok; rnd++, li++) {
         const ItemTile t = item_tile(a, tile_of_item(item));
-        const uint32_t half = ((t.count + 15) & ~15u) / 2;
-        const uint32_t mine = PAIR ? half : t.count, first_row = PAIR ? rank * half : 0;
-        const uint32_t ncopies = (mine + 3) / 4;
-        uint32_t idx[4 * kPerLane];
+        const uint32_t half = ((t.count + 15) & ~15u) / 2, ncopies = (half + 3) / 4;
+        uint32_t idx[4];
 #pragma unroll
-        for (uint32_t j = 0; j < 4 * kPerLane; j++) {
-          const uint32_t r = first_row + 4 * (lane + 32 * (j / 4)) + j % 4;
-          idx[j] = a.gather_rows[t.start + min(r, t.count - 1)];
-        }
+        for (uint32_t j = 0; j < 4; j++) idx[j] = a.gather_rows[t.start + min(rank * half + 4 * lane + j, t.count - 1)];
         for (uint32_t it = 0; it < KT && ok; it++) {
           const uint32_t g = li * KT + it, s = g % S, use_s = g / S;
-          const uint32_t bar = PAIR ? full_lead(s) : full_bar(s);
           if (lane == 0) {
             if (use_s > 0) ok = mbar_wait(empty_bar(s), (use_s - 1) & 1, abort, a.error);
-            if (ok) {
-              if constexpr (PAIR)
-                mbar_arrive_expect_cluster(bar, ncopies * 4 * kTileK * 2);
-              else
-                mbar_arrive_expect(bar, ncopies * 4 * kTileK * 2);
-            }
+            if (ok) mbar_arrive_expect_cluster(full_lead(s), ncopies * 4 * kTileK * 2);
           }
           ok = __shfl_sync(0xffffffffu, ok, 0);
           if (!ok) break;
           const uint32_t xt = smem_u32(smem + s * SM::kStageBytes) + NMAT * SM::kWBytes, x0 = StageMap<QT, kDecGroups>::first_value(it, KT);
-#pragma unroll
-          for (uint32_t c = 0; c < kPerLane; c++) {
-            const uint32_t copy = lane + 32 * c;
-            if (copy < ncopies) {
-              if constexpr (PAIR)
-                tma_gather4_rows_pair(xt + copy * 4 * kTileK * 2, &act_map, x0, idx[4 * c], idx[4 * c + 1], idx[4 * c + 2], idx[4 * c + 3], bar);
-              else
-                tma_gather4_rows(xt + copy * 4 * kTileK * 2, &act_map, x0, idx[4 * c], idx[4 * c + 1], idx[4 * c + 2], idx[4 * c + 3], bar);
-            }
-          }
+          if (lane < ncopies) tma_gather4_rows_pair(xt + lane * 4 * kTileK * 2, &act_map, x0, idx[0], idx[1], idx[2], idx[3], full_lead(s));
         }
       }
       if (!ok && lane == 0) {
@@ -1251,22 +1209,15 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
         // A CTA of a pair brings its half of the rows the instruction takes (the rows rounded up to 16): the first
         // CTA the first half.
         const uint32_t half = ((t.count + 15) & ~15u) / 2;
-        const uint32_t mine = PAIR ? half : t.count, row0 = t.start + (PAIR ? rank * half : 0);
-        const uint32_t nbox = (mine + kTileBoxRows - 1) / kTileBoxRows;
+        const uint32_t row0 = t.start + rank * half, nbox = (half + kTileBoxRows - 1) / kTileBoxRows;
         for (uint32_t it = 0; it < KT && ok; it++) {
           const uint32_t g = li * KT + it, s = g % S, use_s = g / S;
           if (use_s > 0) ok = mbar_wait(empty_bar(s), (use_s - 1) & 1, abort, a.error);
           if (!ok) break;
           const uint32_t xt = smem_u32(smem + s * SM::kStageBytes) + NMAT * SM::kWBytes, x0 = StageMap<QT, kDecGroups>::first_value(it, KT);
-          if constexpr (PAIR) {
-            mbar_arrive_expect_cluster(full_lead(s), nbox * kTileBoxRows * kTileK * 2);
-            for (uint32_t i = 0; i < nbox; i++)
-              tma_load_rows_pair(xt + i * kTileBoxRows * kTileK * 2, &act_map, x0, row0 + i * kTileBoxRows, full_lead(s));
-          } else {
-            mbar_arrive_expect(full_bar(s), nbox * kTileBoxRows * kTileK * 2);
-            for (uint32_t i = 0; i < nbox; i++)
-              tma_load_rows(xt + i * kTileBoxRows * kTileK * 2, &act_map, x0, row0 + i * kTileBoxRows, full_bar(s));
-          }
+          mbar_arrive_expect_cluster(full_lead(s), nbox * kTileBoxRows * kTileK * 2);
+          for (uint32_t i = 0; i < nbox; i++)
+            tma_load_rows_pair(xt + i * kTileBoxRows * kTileK * 2, &act_map, x0, row0 + i * kTileBoxRows, full_lead(s));
         }
       }
       if (!ok) {
@@ -1304,24 +1255,14 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
     // commit frees the stage when they are done, in both CTAs of a pair.
     const uint32_t leader = elect_leader();
     auto wait_lead = [&](uint32_t bar, uint32_t parity) { return mbar_wait_warp(bar, parity, abort, a.error); };
-    auto mma = [&](uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
-      if constexpr (PAIR)
-        mma_f16_pair(leader, d, da, db, idesc, acc);
-      else
-        mma_f16(leader, d, da, db, idesc, acc);
-    };
-    auto commit = [&](uint32_t bar) {
-      if constexpr (PAIR)
-        mma_commit_pair(leader, bar, 3);
-      else
-        mma_commit(leader, bar);
-    };
+    auto mma = [&](uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) { mma_f16_pair(leader, d, da, db, idesc, acc); };
+    auto commit = [&](uint32_t bar) { mma_commit_pair(leader, bar, 3); };
     const uint32_t stages = smem_u32(smem);
     uint32_t s = 0, phase = 0;
     bool after_wide = false;
     for (uint32_t rnd = 0, item; (item = item_at(rnd)) != kNoItem && ok; rnd++) {
       const ItemTile t = item_tile(a, tile_of_item(item));
-      const uint32_t idesc = instr_desc((t.count + 15) & ~15u, PAIR ? 2 * kTileM : kTileM);
+      const uint32_t idesc = instr_desc((t.count + 15) & ~15u, 2 * kTileM);
       const bool wide = is_wide(t.count);
       const uint32_t b = next_buf, colg = tmem_base + (wide ? 0 : b * kTileN), colu = colg + (wide ? kTileN : kTileN / 2);
       // The buffers this item writes must have been read: by the epilogue warps, and after a two-buffer item by the
@@ -1358,14 +1299,11 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
   __syncthreads();
   // Neither CTA of a pair may leave (or free tensor memory) while the other may still read its shared memory or write
   // its tensor memory.
-  if constexpr (PAIR) cluster_sync();
+  cluster_sync();
   if (warp == kMmaWarp) {
     __syncwarp();
     tc_fence_after();
-    if constexpr (PAIR)
-      tmem_free_pair(tmem_base, kCols);
-    else
-      tmem_free(tmem_base, kCols);
+    tmem_free_pair(tmem_base, kCols);
   }
 }
 

@@ -35,36 +35,26 @@ static cudaError_t max_pairs(uint32_t threads, size_t smem, int device, uint32_t
 template <int QT, int NMAT>
 cudaError_t launch_expert_tiles(const ExpertTilesArgs &a, const CUtensorMap &act_map, uint32_t max_tiles, const uint32_t *grid_global,
                                 const LaunchCtx &ctx, cudaStream_t st) {
-  if (a.K % kTileK || a.R % kTileM || max_tiles == 0) return cudaErrorInvalidValue;
-  const uint32_t RT = a.R / kTileM;
-  if (!items_divide(max_tiles, RT % 2 == 0 ? RT / 2 : RT)) return cudaErrorInvalidValue;
-  if (RT % 2 == 0) {
-    // Pairs of CTAs on 256 weight rows an item: half the rows' bytes through each CTA's shared memory.
-    constexpr auto kernel = k_expert_tiles<QT, NMAT, true>;
-    const size_t smem = TileSmem<QT, NMAT, true>::kBytes;
-    static std::atomic<uint32_t> attr_done{0};
-    cudaError_t e = ensure_dynamic_smem(kernel, smem, attr_done, ctx.device);
-    if (e != cudaSuccess) return e;
-    uint32_t pairs = 0;
-    e = max_pairs<kernel>(tile_threads(NMAT), smem, ctx.device, pairs);
-    if (e != cudaSuccess) return e;
-    const uint64_t items = (uint64_t)max_tiles * (RT / 2);
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = 2, at.val.clusterDim.y = 1, at.val.clusterDim.z = 1;
-    cfg.gridDim = dim3(2 * (unsigned)std::min<uint64_t>(items, pairs)), cfg.blockDim = dim3(tile_threads(NMAT));
-    cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = &at, cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, a, act_map, grid_global);
-  }
-  auto kernel = k_expert_tiles<QT, NMAT, false>;
-  const size_t smem = TileSmem<QT, NMAT, false>::kBytes;
+  // An item is 256 weight rows, a pair's; check_config admits layers of no others.
+  if (a.K % kTileK || a.R % (2 * kTileM) || max_tiles == 0) return cudaErrorInvalidValue;
+  const uint32_t RTU = a.R / (2 * kTileM);
+  if (!items_divide(max_tiles, RTU)) return cudaErrorInvalidValue;
+  constexpr auto kernel = k_expert_tiles<QT, NMAT>;
+  const size_t smem = TileSmem<QT, NMAT>::kBytes;
   static std::atomic<uint32_t> attr_done{0};
-  const cudaError_t e = ensure_dynamic_smem(kernel, smem, attr_done, ctx.device);
+  cudaError_t e = ensure_dynamic_smem(kernel, smem, attr_done, ctx.device);
   if (e != cudaSuccess) return e;
-  const uint64_t items = (uint64_t)max_tiles * RT;
-  kernel<<<(unsigned)std::min<uint64_t>(items, (uint64_t)ctx.sms), tile_threads(NMAT), smem, st>>>(a, act_map, grid_global);
-  return cudaGetLastError();
+  uint32_t pairs = 0;
+  e = max_pairs<kernel>(tile_threads(NMAT), smem, ctx.device, pairs);
+  if (e != cudaSuccess) return e;
+  const uint64_t items = (uint64_t)max_tiles * RTU;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = 2, at.val.clusterDim.y = 1, at.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(2 * (unsigned)std::min<uint64_t>(items, pairs)), cfg.blockDim = dim3(tile_threads(NMAT));
+  cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = &at, cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, a, act_map, grid_global);
 }
 
 template cudaError_t launch_expert_tiles<EXPERT_TILES_QT, 1>(const ExpertTilesArgs &, const CUtensorMap &, uint32_t, const uint32_t *, const LaunchCtx &,

@@ -328,7 +328,7 @@ void create(moe_layer *l, const moe_layer_config &c, const moe_layer_weights &w)
     l->sms = n > 0 ? (uint32_t)n : 148;
     l->ctx = LaunchCtx{c.device, l->sms};
   }
-  l->can_tensor = !(c.flags & MOE_FLAG_NO_TENSOR) && c.n_embd % kTileK == 0 && c.n_ff % kTileM == 0;
+  l->can_tensor = !(c.flags & MOE_FLAG_NO_TENSOR);
   l->stream = std::make_unique<Stream>();
   l->aux = std::make_unique<Stream>();
   l->fork_ev = std::make_unique<Event>(), l->join_ev = std::make_unique<Event>();
