@@ -442,7 +442,7 @@ void create(moe_layer *l, const moe_layer_config &c, const moe_layer_weights &w)
 // below what is dropped gave an error of 2.6 times that bound, and another expert.)
 // sum |x_i w_i| <= |x| |w_e| (Cauchy-Schwarz), and a running sum over the first i values is at most |x| |w_e's first i values|,
 // whose norms are known here. So over runs of the row that are summed apart (a step's pieces; the chains) it adds up to |x| times
-// the root of the sum over the runs of (the sum of the run's prefix norms) squared, whatever way x's norm falls to them: prefix_sums.
+// the root of the sum over the runs of (the sum of the run's prefix norms) squared, whatever way x's norm falls to them.
 // eps = eps_rel |x|, with eps_rel the largest over the experts of 2^-23 (15 steps + chains / 2 + 16 |w_e|), a hundredth more
 // for the roundings of roundings, covers all three where every rounding falls the same way (of |w_e|, at E = 2048 and in one, two and four
 // pieces: 2^-12.6, 2^-13.5, 2^-14.5); a random row's error is some hundredth of it. eps_abs is the rest: 2^-25 of the largest sum of
@@ -456,24 +456,31 @@ void setup_router_tensor(moe_layer *l, const float *router, const float *bias, c
   for (uint32_t e = 0; e < NE; e++) {
     const float *w = router + (size_t)e * E;
     float m = 0.0f;
-    double n2 = 0.0, w_sum = 0.0;
-    for (uint32_t i = 0; i < E; i++) m = std::max(m, std::fabs(w[i])), n2 += (double)w[i] * w[i], w_sum += std::fabs(w[i]);
-    w_sum_max = std::max(w_sum_max, w_sum);
-    // The norms of each run's first values, every `step` of them, added up; of the runs' sums the norm.
-    auto prefix_sums = [&](uint32_t runs, uint32_t step) {
-      double all = 0.0;
-      for (uint32_t r = 0; r < runs; r++) {
-        double p2 = 0.0, sum = 0.0;
-        for (uint32_t i = r * (E / runs); i < (r + 1) * (E / runs); i++) {
-          p2 += (double)w[i] * w[i];
-          if (i % step == step - 1) sum += std::sqrt(p2);
+    double w_sum = 0.0, chains2 = 0.0;
+    double run2[3] = {}, run_sum[3] = {}, steps2[3] = {};  // of the row in one, two and four runs: the current one's, and all's so far
+    for (uint32_t p = 0; p < kRouterPieces; p++) {
+      double chain2 = 0.0, chain_sum = 0.0;
+      for (uint32_t i0 = p * (E / kRouterPieces); i0 < (p + 1) * (E / kRouterPieces); i0 += 16) {
+        double step2 = 0.0;
+        for (uint32_t i = i0; i < i0 + 16; i++) {
+          const double v2 = (double)w[i] * w[i];
+          m = std::max(m, std::fabs(w[i])), w_sum += std::fabs(w[i]), step2 += v2, chain2 += v2;
+          chain_sum += std::sqrt(chain2);
         }
-        all += sum * sum;
+        for (uint32_t j = 0; j < 3; j++) run2[j] += step2, run_sum[j] += std::sqrt(run2[j]);
       }
-      return std::sqrt(all);
-    };
-    const double chains = prefix_sums(kRouterPieces, 1);
-    for (uint32_t j = 0; j < 3; j++) eps[j] = std::max(eps[j], 1.01 * (15.0 * prefix_sums(1u << j, 16) + 0.5 * chains) + 16.0 * std::sqrt(n2));
+      chains2 += chain_sum * chain_sum;
+      for (uint32_t j = 0; j < 3; j++)
+        if ((p + 1) % (kRouterPieces >> j) == 0) {
+          steps2[j] += run_sum[j] * run_sum[j];
+          if (j > 0) run2[j] = 0.0;
+          run_sum[j] = 0.0;
+        }
+    }
+    w_sum_max = std::max(w_sum_max, w_sum);
+    // run2[0], the row in one run, is |w_e|^2 by now.
+    for (uint32_t j = 0; j < 3; j++)
+      eps[j] = std::max(eps[j], 1.01 * (15.0 * std::sqrt(steps2[j]) + 0.5 * std::sqrt(chains2)) + 16.0 * std::sqrt(run2[0]));
     int ex = 0;
     if (m > 0.0f && std::isfinite(m)) std::frexp(m, &ex);
     ex = std::min(std::max(ex, -100), 100);
