@@ -31,7 +31,7 @@ constexpr uint32_t kMmaRowsUnit = 256;          // weight rows come in multiples
 constexpr uint32_t kMmaMaxSmem = 100 * 1024;    // for the rows of an entry
 
 // The rows in shared memory: codes with a stride that spreads eight rows' words over the banks; the scales, sub-block or
-// block by block with the rows side by side; the sums of each 32 or 16 codes. After them a codebook type's codebook.
+// block by block with the rows side by side; the sums of each 32 or 16 codes. Before them a codebook type's codebook and the warps' rings.
 __host__ __device__ constexpr uint32_t mma_pad(uint32_t qt) { return qt == QT_Q6_K ? 16 : 32; }
 __host__ __device__ constexpr uint32_t mma_sum_len(uint32_t qt) { return qt == QT_Q4_K ? 32 : qt == QT_Q6_K ? 16 : 0; }
 __host__ __device__ constexpr uint32_t mma_smem(uint32_t qt, uint32_t rows, uint32_t K) {

@@ -1,9 +1,9 @@
-// The experts' products for many rows per expert: a grouped GEMM on the 5th-generation tensor cores. A work item is 128
-// weight rows of one expert and up to 256 of the rows routed to it; persistent CTAs, one per SM, take items in turn.
+// The experts' products for many rows per expert: a grouped GEMM on the 5th-generation tensor cores. A work item is 256
+// weight rows of one expert and up to 256 of the rows routed to it; persistent pairs of CTAs, one CTA an SM, take items in turn.
 // Decode warps turn the quantised blocks into f16 straight into shared memory in the tensor core's K-major
 // core-matrix layout; one thread brings the rows' activations beside them with bulk-tensor (TMA) copies, 64 rows a
-// copy, in the 128-byte-swizzled K-major layout; one thread issues tcgen05.mma with the weights as the M side and the rows as the N side (so a short
-// tile costs a short instruction), accumulating f32 in tensor memory; the workers read the accumulators back with
+// copy, in the 128-byte-swizzled K-major layout; one lane of a warp issues tcgen05.mma with the weights as the M side and the rows as the N side (so a
+// short tile costs a short instruction), accumulating f32 in tensor memory; epilogue warps read the accumulators back with
 // tcgen05.ld, apply SwiGLU and store. This replaces the reference's moe_gate_up_t / moe_down_t
 // (kernels/quant/qgemm.cl:88-239), whose tiles are 64 rows on Xe2's DPAS.
 //
@@ -32,7 +32,9 @@ constexpr uint32_t kTileN = 256;   // activation rows at most
 constexpr uint32_t kTileK = 64;    // values of the contraction a stage holds
 constexpr uint32_t kTileDecoders = 512;  // threads that decode weights: 16 warps, enough of them to hide their loads' latency
 // Threads that turn accumulators into results: a warp per quarter of the weight rows, two for the down product, whose items are
-// a quarter as long as gate's and up's for twice the results (32,768 rows, the layer: 3,715 us with one, 3,461 with two).
+// a quarter as long as gate's and up's for twice the results. That pays where tiles are full (the layer with one and with two:
+// 32,768 rows of Q4_K 4,143 and 4,058 us; 8,192, skewed, 1,206 and 1,225, within what its runs differ by; 4,352 of IQ4_XS, 85 rows
+// an expert, 892 and 897).
 __host__ __device__ constexpr uint32_t tile_epilogue(int nmat) { return nmat == 1 ? 256 : 128; }
 __host__ __device__ constexpr uint32_t tile_threads(int nmat) { return kTileDecoders + tile_epilogue(nmat) + 96; }  // and the rows' copy warp, the MMA warp, the quants' copy warp
 constexpr uint32_t kTileBoxRows = 64;    // rows one bulk-tensor copy brings (the tensor map's box: 64 values x 64 rows)
@@ -199,9 +201,9 @@ __device__ __forceinline__ void tmem_free_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 // MMAs and commits are issued by one lane, `leader`, in code that the whole warp runs together: the instruction takes its
-// descriptors from uniform registers, which the compiler can keep them in only where no lane goes its own way. (In a branch
-// for lane 0 each was worked out in that lane's registers and moved over, some twenty instructions an MMA at the ten clocks
-// each that a scheduler's six warps leave: 173 clocks an MMA of 96 rows and 200 of 256, for 48 and 128 of the tensor core's.)
+// descriptors from uniform registers, which the compiler can keep them in only where no lane goes its own way. (Issued in a branch
+// for lane 0 an MMA of 96 rows took 173 clocks of that thread and one of 256 rows 200, by its own clock counts, for 48 and 128 of
+// the tensor core's, and it waited for a tenth of them; so 152 and 182.)
 // The pair's commit: one arrival on the barrier at this place in each CTA of the mask.
 __device__ __forceinline__ void mma_commit_pair(uint32_t leader, uint32_t bar, uint32_t cta_mask) {
   asm volatile(
@@ -773,8 +775,8 @@ struct StageMap {
 
 // Shared memory of a CTA: the stages (NMAT weight tiles of 16 KB and half a row tile, 16 KB, each), then (for types whose
 // quants come by copy) a ring of two quant slots, then the barriers, then a codebook type's codebook.
-// A quant slot holds, for every weight row of the item, the quants of one stage per decode group: 32 bytes a stage for
-// Q4_K, so 64 bytes a row with two groups (64-byte swizzle) and 128 with four (128-byte swizzle).
+// A quant slot holds, for every weight row of the item, the quants of one stage per decode group: 32 bytes a stage in these
+// types of four bits a value, so 64 bytes a row with two groups (64-byte swizzle) and 128 with four (128-byte swizzle).
 template <int QT, int NMAT>
 struct TileSmem {
   static constexpr uint32_t kStages = NMAT == 2 ? 4 : 6;
@@ -926,11 +928,12 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
 
   // Columns q (this warp's quarter of the weight rows: TMEM lanes 32 q ..) of chunks slot, slot + nslots, ... of W rows
   // each, from the accumulators at column colg (and colu, the up product) to the result. A lane holds one weight row's
-  // values for the chunk's W rows; for each row the warp's 32 lanes store 32 consecutive values. The address of a
-  // chunk is worked out once and stepped by the row stride: what the loop costs per value is a conversion and a store.
+  // values for the chunk's W rows; for each row the warp's lanes store 32 consecutive values: in f32 one a lane, in f16 the even
+  // lanes one row's and the odd ones the next's, two a lane. The address of a chunk is worked out once and stepped by the row stride: what the loop costs
+  // per value is a conversion and a store, in f16 half a shuffle and half a store.
   // The loads of a warp's next chunk are in flight while it converts and stores the one before (two sets of
   // registers): what a chunk costs is then its instructions, not tensor memory's latency, which alone had the down
-  // product's four epilogue warps take longer over an item than its MMAs do.
+  // product's epilogue warps, four of them then, take longer over an item than its MMAs do.
   auto drain = [&](const ItemTile &t, uint32_t r0, uint32_t colg, uint32_t colu, uint32_t slot, uint32_t nslots) {
     constexpr int W = NMAT == 2 ? 8 : 16;
     const uint32_t q = warp % 4, r = r0 + 32 * q + lane, nch = ((t.count + 15) & ~15u) / W;
@@ -1229,7 +1232,7 @@ __global__ void __launch_bounds__(tile_threads(NMAT), 1) k_expert_tiles(const __
     }
   } else if (warp == kQuantWarp) {
     if (quants_by_copy(QT) && lane == 0) {
-    // The quants' copy thread (a warp of its own: sharing a warp with the MMA thread cost the tile kernels 8 %): a quant slot, one stage per decode group for every weight row of the item, as soon
+    // The quants' copy thread (a warp of its own: sharing a warp with the MMAs' issue cost the tile kernels 8 %): a quant slot, one stage per decode group for every weight row of the item, as soon
     // as the decode warps have read the slot's last contents; it runs ahead of the stages by the ring's two slots.
     uint32_t li = 0;
     for (uint32_t rnd = 0, item; (item = item_at(rnd)) != kNoItem && ok; rnd++, li++) {

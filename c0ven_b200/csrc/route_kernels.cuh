@@ -85,11 +85,12 @@ static __global__ void __launch_bounds__(256) k_quant(const float *x, uint64_t n
 // A CTA takes four of the router's rows and up to ROWS rows of x: a warp a piece, its lanes the pairs of a row of x and one of the
 // router's (8 rows: a chain a lane) or a row of x each (32 rows: four chains a lane). Both come through a ring in shared memory by
 // 16-byte asynchronous copies, 16 values of every piece a stage, so that each of the router's rows is read from HBM once. What bounds
-// it is the way of x out of L2, 256 KB a CTA at 32 rows of 2,048 values, and the chains, of E / 8 multiply-adds. (A lane walking its
+// it is the chain of its stages, sixteen at 2,048 values, each a wait for its copies and a barrier: no unit is near its limit (32
+// rows, ncu: issue slots 29 % and the L1 39 % busy while an SM has work). (A lane walking its
 // piece of a weight row itself for two rows of x a CTA, the router's 4 MB read out of L2 again for every two rows: 33 us at 32
-// rows by ncu, cold, 17.6 now; two layers of 32 rows of IQ3_S 493 us and 464, 64 rows of Q8_0 377 and 272 together with the groups'
+// rows by ncu, cold, 18 to 20 now; two layers of 32 rows of IQ3_S 6 % less, 64 rows of Q8_0 377 and 272 together with the groups'
 // other kernel, four rows of Q4_K with Q6_K 70 and 64.)
-// One row has a kernel of its own, k_router_logits_one: by the form for 8 rows, of a ring of 43 to 104 KB, which keeps the next
+// One row has a kernel of its own, k_router_logits_one: by the form for 8 rows, with rings of 42 to 104 KB, which keep the next
 // kernel's waiting CTAs off the SM, the layer in Q8_0 took 27.5 to 28.8 us, 26.7 so.
 // The step's quantisers ride along: the first sq.ctas CTAs of every grid row share out the blocks of x among their warps,
 // so that quantising x is neither a launch of its own in front of the router nor behind it. A warp takes as many blocks as

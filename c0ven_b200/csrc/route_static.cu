@@ -80,6 +80,8 @@ MOE_API moe_status moe_route_rows_static(const float *x_dev, uint32_t T, uint32_
   const uint32_t N = n_experts + 1;
   float *rl = scratch;
   uint32_t *hist = (uint32_t *)(scratch + kLogitFloats);
+  // One form for every step: 1 to 8 rows of 2,048 values over 512 experts take 21 us so, 32 rows 32, 64 rows 38 (by a warp that
+  // walked the router's rows itself 46 to 81, 128 and 189).
   // Both regions are written in full for the rows of this call before they are read (every logit of rows < T; every
   // expert's count of every chunk), so the last call's contents need no clearing.
   k_router_logits_rows<kRouterRows><<<dim3((N + kRouterExperts - 1) / kRouterExperts, (T + kRouterRows - 1) / kRouterRows), 32 * kRouterPieces, router_rows_smem(kRouterRows), st>>>(x_dev, T, n_embd, router_dev, N, bias_dev, n_experts, rl, StepQuant{});

@@ -11,7 +11,7 @@
 // still leaves SMs idle, a half or a quarter of the row: an item is a chain of stages at the pace of one SM's copies,
 // 32 of them and some 33 us at 2,048 values a row, however few items there are); persistent CTAs of six warps take items in turn: one thread issues the
 // bulk-tensor copies (x hi and lo: 64 values x 128 rows; the router's hi and lo: 64 values x 256 experts, all in the
-// 128-byte-swizzled K-major layout), one issues the MMAs (M 128, N 256, K 16; twelve a stage), four warps read the
+// 128-byte-swizzled K-major layout), a warp runs the MMAs in step, one lane of it issuing them (M 128, N 256, K 16; twelve a stage), four warps read the
 // accumulators back and store the logits. Tensor memory holds two accumulators of 256 columns, so the MMAs of item
 // i + 1 run while item i drains. No copy is multicast; every wait is bounded, as in the experts' tile kernel.
 #pragma once

@@ -27,7 +27,7 @@ __device__ __forceinline__ float key_value(uint32_t key) {
 constexpr int kMaxPerLane = 16;  // experts a lane holds at most: 512 / 32
 
 // Steps of many rows: the logits come from the tensor-core product (router_mma.cuh) and are approximate. For row t
-// every one is within eps_t of the logit the exact order gives, eps_t = eps_rel * |x_t| * (largest |w_e|) + eps_abs,
+// every one is within eps_t of the logit the exact order gives, eps_t = eps_rel * |x_t| + eps_abs (setup_router_tensor),
 // with |x_t|^2 summed from norm2_parts. The top-k below then recomputes, in the exact order, only what that bound
 // cannot decide.
 struct RouterApprox {

@@ -74,9 +74,9 @@ def test_without_a_shared_expert_and_equal_logits():
 
 
 @pytest.mark.parametrize("n_embd,no_tensor", [(8192, False), (8192, True), (16384, False), (16384, True)])
-def test_rows_too_long_for_eight_of_them_in_a_router_cta(n_embd, no_tensor):
-    """Eight rows of more than 7,232 values pass a CTA's shared memory: steps of one or two rows a CTA run all the same, and
-    the long steps of a layer kept off the tensor cores take two."""
+def test_the_router_on_the_longest_rows(n_embd, no_tensor):
+    """Rows of up to 16,384 values: the kernel of one row holds all of it in shared memory, the others a ring of stages whatever
+    the length; and the longer steps of a layer kept off the tensor cores, in several CTAs' worth of rows."""
     layer = synth.make_layer(n_embd=n_embd, n_ff=256, n_experts=32, n_used=2, gate_type=synth.Q4_K, down_type=synth.Q8_0, seed=n_embd)
     gpu = MoELayer(layer, max_tokens=70, no_tensor=no_tensor)
     for T in (1, 2, 9, 64, 70):
